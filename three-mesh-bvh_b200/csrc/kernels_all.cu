@@ -74,9 +74,7 @@ __global__ void __launch_bounds__(kBlock) raycast_all_kernel(MeshDev m, const fl
           for (;;) {
             Tri t = load_tri(m.tris, k);
             int ts = tri_side(t, side, sides);
-            float th, te;
-            if (ts >= 0 && tri_hit_t(t.a, t.b, t.c, r.o, r.d, r.d_l1, ts, th, te) &&
-                in_range(th, te, t, r, dlen, near_d, far_d)) {
+            if (ts >= 0 && hit_exact(m, t, k, r, dlen, ts, near_d, far_d)) {
               if (cnt < cap) store_pending_record(out + cnt, k, 0.0f);
               ++cnt;
             }
@@ -170,9 +168,7 @@ __global__ void __launch_bounds__(kBlock, kAllBlocksPerSm) raycast_all_persisten
             for (uint32_t k = link & ~kLeafBit;; ++k) {
               const Tri t = load_tri(m.tris, k);
               const int ts = tri_side(t, side, sides);
-              float th, te;
-              if (ts >= 0 && tri_hit_t(t.a, t.b, t.c, r.o, r.d, r.d_l1, ts, th, te) &&
-                  in_range(th, te, t, r, dlen, near_d, far_d)) {
+              if (ts >= 0 && hit_exact(m, t, k, r, dlen, ts, near_d, far_d)) {
                 if (cnt < cap) store_pending_record(out + cnt, k, 0.0f);
                 ++cnt;
               }
@@ -250,7 +246,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_all_packet_kernel(
     r.o = make_float3(0.f, 0.f, 0.f);
     r.d = make_float3(1.f, 0.f, 0.f);
     r.inv = make_float3(1.f, 1e30f, 1e30f);
-    r.d_l1 = 1.f;
+    r.dk = kFilterK;
   }
   const float dlen = sqrtf(r.d.x * r.d.x + r.d.y * r.d.y + r.d.z * r.d.z);
   uint32_t cnt = 0;
@@ -266,9 +262,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_all_packet_kernel(
           for (uint32_t k = link & ~kLeafBit;; ++k) {
             Tri t = load_tri(m.tris, k);
             int ts = tri_side(t, side, sides);
-            float th, te;
-            if (ts >= 0 && tri_hit_t(t.a, t.b, t.c, r.o, r.d, r.d_l1, ts, th, te) &&
-                in_range(th, te, t, r, dlen, near_d, far_d)) {
+            if (ts >= 0 && hit_exact(m, t, k, r, dlen, ts, near_d, far_d)) {
               if (cnt < cap) store_pending_record(out + cnt, k, 0.0f);
               ++cnt;
             }

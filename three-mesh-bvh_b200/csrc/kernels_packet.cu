@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) raycast_first_packet_kernel(MeshD
     r.o = make_float3(0.f, 0.f, 0.f);
     r.d = make_float3(1.f, 0.f, 0.f);
     r.inv = make_float3(1.f, 1e30f, 1e30f);
-    r.d_l1 = 1.f;
+    r.dk = kFilterK;
   }
   const unsigned valid_mask = __ballot_sync(full, valid);
   Best best{kInf, 0.0f, 0xFFFFFFFFu};
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
     r.o = make_float3(0.f, 0.f, 0.f);
     r.d = make_float3(1.f, 0.f, 0.f);
     r.inv = make_float3(1.f, 1e30f, 1e30f);
-    r.d_l1 = 1.f;
+    r.dk = kFilterK;
   }
   Best best{kInf, 0.0f, 0xFFFFFFFFu};
   float lane_t[kMaxStack];

@@ -29,7 +29,7 @@ __device__ __forceinline__ RayF ray_from(float3 o, float3 d) {
   const float dy = fabsf(d.y) < kTiny ? copysignf(kTiny, d.y) : d.y;
   const float dz = fabsf(d.z) < kTiny ? copysignf(kTiny, d.z) : d.z;
   r.inv = make_float3(__frcp_rn(dx), __frcp_rn(dy), __frcp_rn(dz));
-  r.d_l1 = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
+  r.dk = kFilterK * (fabsf(d.x) + fabsf(d.y) + fabsf(d.z));
   return r;
 }
 
@@ -388,7 +388,9 @@ __global__ void __launch_bounds__(kBlock, 14) scene_raycast_all_kernel(MeshDev m
               for (uint32_t k = bl & ~kLeafBit;; ++k) {
                 const Tri t = load_tri(m.tris, k);
                 const int ts = tri_side(t, side, no_sides);
-                if (ts >= 0 && tri_hit(t.a, t.b, t.c, L.r.o, L.r.d, L.r.d_l1, ts)) {
+                float th, te;
+                const int st = ts < 0 ? 0 : tri_filter(t.a, t.b, t.c, L.r.o, L.r.d, L.r.dk, ts, th, te);
+                if (st > 0 || (st < 0 && tri_hit_slow(t.a, t.b, t.c, L.r.o, L.r.d, ts))) {
                   const ff tt = tri_t_ff(tri_eval_ff(t.a, t.b, t.c, L.r.o, L.r.d));
                   const ff dist = ff_mul(tt, dlen);
                   if (!ff_lt(dist, ff_from(L.near_d)) && !ff_lt(ff_from(L.far_d), dist)) {

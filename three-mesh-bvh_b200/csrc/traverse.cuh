@@ -39,9 +39,16 @@ __device__ __forceinline__ void ld8(const void* p, float4& a, float4& b) {
       : "l"(p));
 }
 
+// Reciprocal within one unit in the last place; the slab margins absorb it.
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 struct RayF {
   float3 o, d, inv;
-  float d_l1;
+  float dk;  // kFilterK |d|_1 (tri_filter)
 };
 
 __device__ __forceinline__ RayF make_ray(const float* __restrict__ rays, uint64_t i) {
@@ -57,13 +64,13 @@ __device__ __forceinline__ RayF make_ray(const float* __restrict__ rays, uint64_
   float dx = fabsf(r.d.x) < kTiny ? copysignf(kTiny, r.d.x) : r.d.x;
   float dy = fabsf(r.d.y) < kTiny ? copysignf(kTiny, r.d.y) : r.d.y;
   float dz = fabsf(r.d.z) < kTiny ? copysignf(kTiny, r.d.z) : r.d.z;
-  r.inv = make_float3(__frcp_rn(dx), __frcp_rn(dy), __frcp_rn(dz));
-  r.d_l1 = fabsf(r.d.x) + fabsf(r.d.y) + fabsf(r.d.z);
+  r.inv = make_float3(rcp_fast(dx), rcp_fast(dy), rcp_fast(dz));
+  r.dk = kFilterK * (fabsf(r.d.x) + fabsf(r.d.y) + fabsf(r.d.z));
   return r;
 }
 
 // Conservative slab test (intersectUtils.js:2-78).  Accepts whenever the reference's float64
-// test could accept: the entry/exit distances carry at most ~3 roundings, and are widened by
+// test could accept: the entry/exit distances carry at most ~4 roundings, and are widened by
 // 2^-20 relative before the comparisons.  `entry` returns the widened entry distance.
 __device__ __forceinline__ bool box_hit(float x0, float y0, float z0, float x1, float y1, float z1, const RayF& r,
                                         float near_d, float far_d, float& entry) {
@@ -172,19 +179,40 @@ __device__ __forceinline__ void store_miss(bvhc_hit* p) {
 // ---------------------------------------------------------------------------------------------
 // raycastFirst leaf step shared by both kernel forms.  Candidate hits are ordered with float32 t
 // values and their error bounds; float-float only settles candidates the bounds cannot separate
-// (the reference keeps the strictly closer one; exact ties keep the candidate found first).
+// (the reference keeps the strictly closer one; of exact ties, here, the smaller record, which is the
+// one it finds first in left-to-right order).
 // ---------------------------------------------------------------------------------------------
 constexpr float kTwoU = 1.1920928955078125e-07f;  // 2u
 
-// near <= dist <= far for dist = t |d|, decided with the float32 bounds, else in float-float.
-__device__ __forceinline__ bool in_range(float t, float t_err, const Tri& tr, const RayF& r, float dlen, float near_d,
-                                         float far_d) {
-  float dist = t * dlen;
-  float derr = t_err * dlen + fabsf(dist) * kTwoU + 1e-30f;
-  if (dist - derr >= near_d && dist + derr <= far_d) return true;
-  if (dist + derr < near_d || dist - derr > far_d) return false;
-  ff dl = ff_mul(tri_t_ff(tri_eval_ff(tr.a, tr.b, tr.c, r.o, r.d)), dir_length(r.d));
+// near <= t |d| <= far from the float32 t and its bound: 1 inside, 0 outside, -1 undecided.
+__device__ __forceinline__ int range_filter(float t, float t_err, float dlen, float near_d, float far_d) {
+  const float dist = t * dlen;
+  const float derr = t_err * dlen + fabsf(dist) * kTwoU + 1e-30f;
+  if (dist - derr >= near_d && dist + derr <= far_d) return 1;
+  return dist + derr < near_d || dist - derr > far_d ? 0 : -1;
+}
+
+// The same and the hit itself in float-float; on a hit, *t is its float-float t.  Out of line, with
+// the float-float code in one place: the filters settle nearly every test, and code inlined for the
+// rest costs registers in every loop that holds it.
+static __device__ __noinline__ bool hit_slow(const TriRecord* __restrict__ tris, uint32_t k, float3 o, float3 d,
+                                             int side, float near_d, float far_d, ff* t) {
+  const Tri tr = load_tri(tris, k);
+  const TriFF e = tri_eval_ff(tr.a, tr.b, tr.c, o, d);
+  if (!tri_decide_ff(e, side)) return false;
+  *t = tri_t_ff(e);
+  const ff dl = ff_mul(*t, dir_length(d));
   return !ff_lt(dl, ff_from(near_d)) && !ff_lt(ff_from(far_d), dl);
+}
+
+// Whether the ray hits triangle record k (loaded as `tr`) within [near, far], exactly.
+__device__ __forceinline__ bool hit_exact(const MeshDev& m, const Tri& tr, uint32_t k, const RayF& r, float dlen,
+                                          int side, float near_d, float far_d) {
+  float t, t_err;
+  int st = tri_filter(tr.a, tr.b, tr.c, r.o, r.d, r.dk, side, t, t_err);
+  if (st > 0) st = range_filter(t, t_err, dlen, near_d, far_d);
+  ff tt;
+  return st < 0 ? hit_slow(m.tris, k, r.o, r.d, side, near_d, far_d, &tt) : st > 0;
 }
 
 struct Best {
@@ -192,35 +220,39 @@ struct Best {
   uint32_t rec;
 };
 
+// Offers triangle record k to `best` in float-float: an exact tie goes to the smaller record.
+static __device__ __noinline__ Best offer_slow(const TriRecord* __restrict__ tris, uint32_t k, float3 o, float3 d,
+                                               int side, float near_d, float far_d, Best best) {
+  ff tn;
+  if (!hit_slow(tris, k, o, d, side, near_d, far_d, &tn)) return best;
+  const float err = fabsf(tn.hi) * kTinyRel + 1e-30f;
+  bool take = best.rec == 0xFFFFFFFFu || tn.hi + err < best.t - best.err;
+  if (!take && !(tn.hi - err > best.t + best.err)) {
+    const Tri bt = load_tri(tris, best.rec);
+    const ff tb = tri_t_ff(tri_eval_ff(bt.a, bt.b, bt.c, o, d));
+    take = ff_lt(tn, tb) || (!ff_lt(tb, tn) && k < best.rec);
+  }
+  return take ? Best{tn.hi, err, k} : best;
+}
+
+// Offers triangle record k (loaded as `tr`): the float32 values and bounds decide, else offer_slow.
+__device__ __forceinline__ void offer_first(const MeshDev& m, const Tri& tr, uint32_t k, const RayF& r, float dlen,
+                                            int side, float near_d, float far_d, Best& best) {
+  float t, t_err;
+  int st = tri_filter(tr.a, tr.b, tr.c, r.o, r.d, r.dk, side, t, t_err);
+  if (st > 0) st = range_filter(t, t_err, dlen, near_d, far_d);
+  // none yet: best.t is infinite and its bound 0, so every hit is nearer
+  if (st > 0) st = t + t_err < best.t - best.err ? 1 : (t - t_err > best.t + best.err ? 0 : -1);
+  if (st > 0) best = Best{t, t_err, k};
+  else if (st < 0) best = offer_slow(m.tris, k, r.o, r.d, side, near_d, far_d, best);
+}
+
 __device__ __forceinline__ void leaf_first(const MeshDev& m, uint32_t k, const RayF& r, float dlen, int side,
                                            const SideTable& sides, float near_d, float far_d, Best& best) {
   for (;;) {
-    Tri t = load_tri(m.tris, k);
-    int ts = tri_side(t, side, sides);
-    float th, te;
-    if (ts >= 0 && tri_hit_t(t.a, t.b, t.c, r.o, r.d, r.d_l1, ts, th, te) &&
-        in_range(th, te, t, r, dlen, near_d, far_d)) {
-      bool take;
-      if (best.rec == 0xFFFFFFFFu || th + te < best.t - best.err) {
-        take = true;
-      } else if (th - te > best.t + best.err) {
-        take = false;
-      } else {
-        Tri bt = load_tri(m.tris, best.rec);
-        ff tn = tri_t_ff(tri_eval_ff(t.a, t.b, t.c, r.o, r.d));
-        ff tb = tri_t_ff(tri_eval_ff(bt.a, bt.b, bt.c, r.o, r.d));
-        take = ff_lt(tn, tb);
-        if (take) {
-          th = tn.hi;
-          te = fabsf(tn.hi) * kTinyRel + 1e-30f;
-        }
-      }
-      if (take) {
-        best.t = th;
-        best.err = te;
-        best.rec = k;
-      }
-    }
+    const Tri t = load_tri(m.tris, k);
+    const int ts = tri_side(t, side, sides);
+    if (ts >= 0) offer_first(m, t, k, r, dlen, ts, near_d, far_d, best);
     if (t.flags & kTriLast) break;
     ++k;
   }
