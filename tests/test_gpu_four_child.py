@@ -1,0 +1,83 @@
+"""raycastFirst over the four-child records, one and four lanes per ray, against the per-ray child-pair
+kernel byte for byte: one candidate order decides in every kernel (the nearest hit, exact ties to the
+smaller record), so neither the records' shape nor the batch size may change a bit."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(pkg, name):
+    """(geometry, build options): a root that is a leaf within one run; one of 40 triangles (halved into
+    runs under its unbounded root); leaves of 40; one root per group, with gaps; a plain tree."""
+    if name == "triangle":
+        return pkg.Geometry(np.array([[0, 0, 0], [4, 0, 0], [0, 4, 0]], np.float32), np.array([0, 1, 2], np.uint16)), {}
+    if name == "leaf40":
+        g = pkg.torus_knot(10, 3, 10, 4)
+        g.index = g.index[:120]
+        return g, {"maxLeafSize": 64}
+    g = pkg.torus_knot(10, 3, 60, 12, noise_sigma=0.05, noise_seed=3)
+    if name == "leaves40":
+        return g, {"maxLeafSize": 40}
+    if name == "groups":
+        g.add_group(0, 900, 0)
+        g.add_group(1200, 1500, 1)
+        g.add_group(3000, 600, 2)
+    return g, {}
+
+
+def _rays(pkg, n):
+    r = np.concatenate([pkg.rays_sphere_to_box(n, seed=n), pkg.rays_incoherent(n, seed=n + 1)])[:n]
+    r[::5, 3:] *= np.float32(3.5)          # directions need not be unit vectors
+    r[1::7, 3] = 0.0                       # a zero component
+    return r
+
+
+@pytest.mark.parametrize("mesh", ["triangle", "leaf40", "leaves40", "groups", "plain"])
+@pytest.mark.parametrize("n", [1, 7, 9, 33, 4097, 131072, 131073])
+def test_matches_the_per_ray_kernel(pkg, cuda, mesh, n):
+    import torch
+
+    g, opts = _mesh(pkg, mesh)
+    bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH, **opts})
+    rays = torch.from_numpy(_rays(pkg, n)).to(cuda)
+    cases = [(0, 0.0, math.inf), (2, 0.0, math.inf), (1, 20.0, 45.0), (2, -5.0, 38.0)]
+    for leaf in (0, 3):
+        bvh.set_leaf_size(leaf)
+        for compact, wide, sort in ((0, 0, 0), (1, 1, 0), (1, 0, 3)):
+            for side, near, far in cases:
+                bvh.set_traversal(0, 1)
+                want = bvh.raycast_first_batch(rays, side, near, far)
+                bvh.set_traversal(1, 1, 16, 0, compact, sort, 0, wide)
+                got = bvh.raycast_first_batch(rays, side, near, far)
+                bvh.synchronize()
+                assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (leaf, compact, sort, side)
+    if mesh == "groups":
+        host = _rays(pkg, n)
+        bvh.set_traversal(0, 1)
+        want = bvh.raycast_first_batch(host, [0, 2, 1])
+        bvh.set_traversal(1, 1)
+        assert np.array_equal(bvh.raycast_first_batch(host, [0, 2, 1]).view(np.uint8), want.view(np.uint8))
+    if mesh != "triangle":
+        assert n < 33 or (want["face_index"] if mesh == "groups" else want.cpu().numpy().view(np.uint32)[:, 0]).min() < 2000
+
+
+@pytest.mark.parametrize("leaf", [0, 4])
+def test_parts_of_leaves_follow_a_refit(pkg, cuda, leaf):
+    """Boxes of runs and of halves of leaves come from their triangles, so a refit recomputes them."""
+    import torch
+
+    g = pkg.torus_knot(10, 3, 80, 12, noise_sigma=0.05, noise_seed=4)
+    bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH, "maxLeafSize": 40})
+    bvh.set_leaf_size(leaf)
+    bvh.raycast_first_batch(pkg.rays_incoherent(8))
+    rng = np.random.default_rng(5)
+    bvh.refit((g.position * 1.3 + rng.normal(0, 0.4, g.position.shape)).astype(np.float32))
+    for n in (3000, 140_000):
+        rays = torch.from_numpy(_rays(pkg, n)).to(cuda)
+        bvh.set_traversal(0, 1)
+        want = bvh.raycast_first_batch(rays, 2)
+        bvh.set_traversal(1, 1)
+        assert torch.equal(bvh.raycast_first_batch(rays, 2).view(torch.int32), want.view(torch.int32))

@@ -2,10 +2,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <exception>
+#include <limits>
 #include <new>
 #include <stdexcept>
 #include <thread>
@@ -104,12 +106,14 @@ struct bvhc_mesh {
   uint32_t* d_quad_roots = nullptr;
   uint32_t* d_quad_src = nullptr;
   uint64_t n_quads = 0;
+  int quad_stack = 0;
 
   // the records raycastFirst traverses
   MeshDev view_first() const {
     MeshDev v = leaf_size ? MeshDev{d_nodes_f, d_tris_f, d_roots_f, n_roots, d_err} : view();
     v.quads = d_quads;
     v.quad_roots = d_quad_roots;
+    v.quad_stack = quad_stack;
     v.depth = leaf_size ? max_depth_f : max_depth;
     return v;
   }
@@ -446,66 +450,209 @@ struct LeafSplitter {
   }
 };
 
-// Four-child records from a child-pair tree: starting from a pair's two children, the internal
-// child with the largest box surface area is replaced by its own two children until there are
-// four children or only leaves.  `src` keeps, per quad child, the child-pair slot its box comes
-// from (2 * pair + side; kEmptyLeaf for an unused child), so refits can copy boxes over.
+// Four-child records from a child-pair tree: starting from a pair's two children, the internal child
+// with the largest box surface area is replaced in place by its own two children until there are four
+// children or only leaves.  A leaf of more than kMaxRun triangles has a record of its own, made the
+// same way from its halves; the leaf's own box stays in its parent's record, because the reference
+// tests it against near and far.  `src` keeps, per quad child, where its box comes from, for refits: the child-pair slot
+// (2 * pair + side), or kLeafBit | the first of its `count` triangle records; kEmptyLeaf: unused, or a
+// root leaf's unbounded box.
 struct QuadBuilder {
   const std::vector<PairNode>& pairs;
+  const std::vector<TriRecord>& tris;
   std::vector<QuadNode> quads;
   std::vector<uint32_t> src;
+  int stack = 0;  // entries a traversal can stack: at most the siblings along one path
+
+  struct Child {
+    uint32_t pair;   // internal: its pair record; else kEmptyLeaf
+    uint32_t slot;   // the child-pair slot holding its box, or kEmptyLeaf
+    uint32_t first, count;  // not internal: its triangle records
+    float box[6];
+    bool part;       // of a leaf: its box is not one of the tree's
+    bool internal() const { return pair != kEmptyLeaf; }
+    bool splits() const { return internal() || count > (uint32_t)kMaxRun; }
+  };
 
   static float area(const float* b) {
     float dx = std::max(b[3] - b[0], 0.0f), dy = std::max(b[4] - b[1], 0.0f), dz = std::max(b[5] - b[2], 0.0f);
     return dx * dy + dy * dz + dz * dx;
   }
 
-  uint32_t build(uint32_t pair) {
-    struct Child {
-      uint32_t link, slot;
-      const float* box;
+  // Subtrees below the records of `defer` levels are put off, to be built by several threads.
+  struct Later {
+    Child child;
+    uint32_t quad;
+    int k, below;
+  };
+  int defer = -1;
+  std::vector<Later> later;
+
+  uint32_t add() {
+    if (quads.size() >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
+    const uint32_t idx = (uint32_t)quads.size();
+    const float nan = std::numeric_limits<float>::quiet_NaN();
+    const QuadChild unused{{nan, nan}, {nan, nan}, nan, nan, kEmptyLeaf, 0};  // until a child is put in
+    quads.push_back(QuadNode{{unused, unused, unused, unused}});
+    src.insert(src.end(), 4, kEmptyLeaf);
+    return idx;
+  }
+
+  // Builds what was put off: each subtree by one of the host's threads into records of its own, which
+  // are then appended.
+  void finish() {
+    if (later.empty()) return;
+    std::vector<QuadBuilder> part(later.size(), QuadBuilder{pairs, tris});
+    std::atomic<size_t> next{0};
+    std::atomic<int> failed{0};
+    auto work = [&]() {
+      for (size_t t; (t = next++) < later.size();) {
+        try {
+          part[t].build(later[t].child, later[t].below);
+        } catch (const Status&) {
+          failed = 1;
+        } catch (...) {
+          failed = 2;
+        }
+      }
     };
+    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> pool;
+    for (unsigned t = 1; t < hw; ++t) {
+      try {
+        pool.emplace_back(work);
+      } catch (...) {  // the threads that did start do the rest
+        break;
+      }
+    }
+    work();
+    for (auto& th : pool) th.join();
+    if (failed == 1) throw Status{BVHC_ERR_UNSUPPORTED};
+    if (failed) throw std::bad_alloc();
+    size_t total = quads.size();
+    for (const QuadBuilder& p : part) total += p.quads.size();
+    if (total >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
+    quads.reserve(total);
+    src.reserve(4 * total);
+    for (size_t t = 0; t < part.size(); ++t) {
+      const uint32_t base = (uint32_t)quads.size();
+      quads[later[t].quad].c[later[t].k].link = base;
+      for (QuadNode q : part[t].quads) {
+        for (QuadChild& c : q.c)
+          if (!(c.link & kLeafBit)) c.link += base;
+        quads.push_back(q);
+      }
+      src.insert(src.end(), part[t].src.begin(), part[t].src.end());
+      stack = std::max(stack, part[t].stack);
+      part[t].quads = {};
+    }
+    later.clear();
+  }
+
+  uint32_t leaf_count(uint32_t first) const {
+    uint32_t k = first;
+    while (!(tris[k].flags & kTriLast)) ++k;
+    return k - first + 1;
+  }
+
+  Child side(uint32_t pair, int s) const {
+    Child c{};
+    const uint32_t link = pairs[pair].link[s];
+    c.slot = 2 * pair + (uint32_t)s;
+    std::memcpy(c.box, pairs[pair].f + 6 * s, sizeof c.box);
+    c.pair = link & kLeafBit ? kEmptyLeaf : link;
+    if (link & kLeafBit && link != kEmptyLeaf) {
+      c.first = link & ~kLeafBit;
+      c.count = leaf_count(c.first);
+    }
+    return c;
+  }
+
+  Child run(uint32_t first, uint32_t count) const {
+    Child c{};
+    c.pair = c.slot = kEmptyLeaf;
+    c.first = first;
+    c.count = count;
+    c.part = true;
+    LeafSplitter::bounds(&tris[first], count, c.box);
+    return c;
+  }
+
+  void halves(const Child& c, Child& a, Child& b) const {
+    if (c.pair != kEmptyLeaf) {
+      a = side(c.pair, 0);
+      b = side(c.pair, 1);
+    } else {
+      const uint32_t half = (c.count + 1) / 2;
+      a = run(c.first, half);
+      b = run(c.first + half, c.count - half);
+    }
+  }
+
+  // A root: its pair's record, or for a root that is a leaf (never box-tested by the reference) one
+  // child with an unbounded box, or the record of the leaf's halves likewise.
+  uint32_t root(uint32_t link) {
+    if (!(link & kLeafBit)) {
+      Child c{};
+      c.pair = link;
+      return build(c, 0);
+    }
+    const uint32_t idx = add();
+    if (link == kEmptyLeaf) return idx;
+    Child c{};
+    c.pair = c.slot = kEmptyLeaf;
+    c.first = link & ~kLeafBit;
+    c.count = leaf_count(c.first);
+    const uint32_t l = c.splits() ? build(c, 0) : run_link(c.first, (int)c.count);
+    QuadChild& q = quads[idx].c[0];
+    q.c[0] = q.c[1] = q.cz = 0.0f;
+    q.h[0] = q.h[1] = q.hz = kBoxUnbounded;
+    q.link = l;
+    return idx;
+  }
+
+  uint32_t build(const Child& parent, int below, int level = 0) {
     Child ch[4];
     int n = 2;
-    ch[0] = {pairs[pair].link[0], 2 * pair, pairs[pair].f};
-    ch[1] = {pairs[pair].link[1], 2 * pair + 1, pairs[pair].f + 6};
+    halves(parent, ch[0], ch[1]);
     while (n < 4) {
       int pick = -1;
       float best = -1.0f;
       for (int k = 0; k < n; ++k) {
-        if (ch[k].link & kLeafBit) continue;
+        if (!(ch[k].internal() || (ch[k].part && ch[k].splits()))) continue;
         float a = area(ch[k].box);
-        if (a > best) {
+        if (!(a <= best)) {
           best = a;
           pick = k;
         }
       }
       if (pick < 0) break;
-      const uint32_t p = ch[pick].link;
-      ch[pick] = {pairs[p].link[0], 2 * p, pairs[p].f};
-      ch[n++] = {pairs[p].link[1], 2 * p + 1, pairs[p].f + 6};
+      const Child c = ch[pick];
+      for (int k = n; k > pick + 1; --k) ch[k] = ch[k - 1];
+      halves(c, ch[pick], ch[pick + 1]);
+      ++n;
     }
-    if (quads.size() >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
-    const uint32_t idx = (uint32_t)quads.size();
-    quads.push_back(QuadNode{});
-    src.resize(4 * (size_t)(idx + 1), kEmptyLeaf);
-    for (int k = 0; k < 4; ++k) {
-      QuadNode& q = quads[idx];
-      if (k < n) {
-        for (int a = 0; a < 3; ++a) {
-          q.lo[a][k] = ch[k].box[a];
-          q.hi[a][k] = ch[k].box[3 + a];
-        }
-        q.link[k] = ch[k].link;
-        src[4 * (size_t)idx + k] = ch[k].slot;
-      } else {
-        q.link[k] = kEmptyLeaf;
-      }
+    const uint32_t idx = add();
+    for (int k = 0; k < n; ++k) {
+      if (ch[k].pair == kEmptyLeaf && ch[k].count == 0) continue;  // an empty leaf
+      QuadChild& q = quads[idx].c[k];
+      const float* b = ch[k].box;
+      box_centre_half(b[0], b[3], q.c[0], q.h[0]);
+      box_centre_half(b[1], b[4], q.c[1], q.h[1]);
+      box_centre_half(b[2], b[5], q.cz, q.hz);
+      if (!ch[k].splits()) q.link = run_link(ch[k].first, (int)ch[k].count);
+      src[4 * (size_t)idx + k] = ch[k].part ? kLeafBit | ch[k].first : ch[k].slot;
+      if (ch[k].part) q.count = ch[k].count;
     }
+    stack = std::max(stack, below + n - 1);
     for (int k = 0; k < n; ++k)
-      if (!(ch[k].link & kLeafBit)) {
-        uint32_t q = build(ch[k].link);
-        quads[idx].link[k] = q;
+      if (ch[k].splits()) {
+        if (level == defer) {
+          later.push_back({ch[k], idx, k, below + n - 1});
+          continue;
+        }
+        uint32_t q = build(ch[k], below + n - 1, level + 1);
+        quads[idx].c[k].link = q;
       }
     return idx;
   }
@@ -582,11 +729,23 @@ static void keep_serialized(bvhc_mesh* m, std::vector<std::vector<uint8_t>> root
 }
 
 // Four-child records over raycastFirst's child-pair layout (pairs + roots), replacing any before.
-static cudaError_t install_quads(bvhc_mesh* m, const std::vector<PairNode>& pairs, const std::vector<uint32_t>& roots) {
-  QuadBuilder qb{pairs};
+static cudaError_t install_quads(bvhc_mesh* m, const std::vector<PairNode>& pairs, const std::vector<TriRecord>& tris,
+                                 const std::vector<uint32_t>& roots) {
+  if (tris.size() >= kRunFirst) {  // more records than a run link can name: the child-pair kernels run
+    cudaFree(m->d_quads);
+    cudaFree(m->d_quad_roots);
+    cudaFree(m->d_quad_src);
+    m->d_quads = nullptr;
+    m->d_quad_roots = m->d_quad_src = nullptr;
+    m->n_quads = 0;
+    return cudaSuccess;
+  }
+  QuadBuilder qb{pairs, tris};
   std::vector<uint32_t> qroots(roots.size());
   try {
-    for (size_t r = 0; r < roots.size(); ++r) qroots[r] = (roots[r] & kLeafBit) ? roots[r] : qb.build(roots[r]);
+    if (tris.size() > 50000) qb.defer = roots.size() > 64 ? 0 : 3;  // 1 or 64 subtrees a root and up
+    for (size_t r = 0; r < roots.size(); ++r) qroots[r] = qb.root(roots[r]);
+    qb.finish();
   } catch (const Status&) {
     return cudaErrorInvalidValue;
   } catch (const std::bad_alloc&) {
@@ -610,6 +769,7 @@ static cudaError_t install_quads(bvhc_mesh* m, const std::vector<PairNode>& pair
   m->d_quad_roots = qr;
   m->d_quad_src = qs;
   m->n_quads = qb.quads.size();
+  m->quad_stack = qb.stack;
   return cudaSuccess;
 }
 
@@ -856,7 +1016,7 @@ bvhc_status bvhc_mesh_create(int device, int version, const void* const* roots, 
   bvhc_status st = finish_mesh(device, pairs, tris, root_links, max_depth, {}, out);
   if (st == BVHC_OK) {
     keep_serialized(*out, std::move(copies), std::move(slot_nodes), index, index_elem_bytes, index_count, n_verts);
-    cudaError_t e = install_quads(*out, (*out)->h_pairs, (*out)->h_roots);
+    cudaError_t e = install_quads(*out, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
     if (e != cudaSuccess) {
       bvhc_mesh_destroy(*out);
       *out = nullptr;
@@ -921,7 +1081,7 @@ bvhc_status bvhc_batch_create(int device, int n_meshes, const int32_t* roots_per
   bvhc_status st = finish_mesh(device, pairs, tris, root_links, max_depth, mesh_root_off, out);
   if (st == BVHC_OK) {
     keep_serialized(*out, std::move(copies), std::move(slot_nodes), index, index_elem_bytes, index_count, n_verts);
-    cudaError_t e = install_quads(*out, (*out)->h_pairs, (*out)->h_roots);
+    cudaError_t e = install_quads(*out, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
     if (e != cudaSuccess) {
       bvhc_mesh_destroy(*out);
       *out = nullptr;
@@ -1171,8 +1331,8 @@ bvhc_status bvhc_mesh_set_leaf_size(bvhc_mesh* m, int max_leaf) {
   free_refit_plan(m->refit[1]);
   if (max_leaf > 0 && !m->h_root_bytes.empty())  // so that a refit keeps this copy in step
     BVHC_CUDA_TRY(build_refit_plan(pairs, tris, roots, serialized_root_boxes(m), m->refit[1]));
-  if (max_leaf > 0) BVHC_CUDA_TRY(install_quads(m, pairs, roots));
-  else BVHC_CUDA_TRY(install_quads(m, m->h_pairs, m->h_roots));
+  if (max_leaf > 0) BVHC_CUDA_TRY(install_quads(m, pairs, tris, roots));
+  else BVHC_CUDA_TRY(install_quads(m, m->h_pairs, m->h_tris, m->h_roots));
   return BVHC_OK;
 }
 
@@ -1202,7 +1362,7 @@ bvhc_status bvhc_mesh_refit(bvhc_mesh* m, const float* positions, uint64_t n_ver
     BVHC_CUDA_TRY(launch_refit(m->refit[1], m->d_nodes_f, m->d_tris_f, m->d_tri_vid, pos, stride_floats, true, s));
   if (m->d_quads)  // the four-child records take their boxes from raycastFirst's child pairs
     BVHC_CUDA_TRY(launch_quad_boxes(m->d_quads, m->n_quads, m->d_quad_src, m->leaf_size > 0 ? m->d_nodes_f : m->d_nodes,
-                                    s));
+                                    m->leaf_size > 0 ? m->d_tris_f : m->d_tris, s));
   if (m->d_pos && m->grad_verts <= n_verts) {  // the adjoint's vertex copy follows the geometry
     BVHC_CUDA_TRY(cudaMemcpy2DAsync(m->d_pos, 3 * sizeof(float), pos, stride_floats * sizeof(float),
                                     3 * sizeof(float), m->grad_verts, cudaMemcpyDeviceToDevice, s));

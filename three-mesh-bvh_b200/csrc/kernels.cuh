@@ -24,6 +24,7 @@ struct MeshDev {
   unsigned int* err;
   const QuadNode* quads = nullptr;     // four-child copy of `nodes` (same triangle records), if any
   const uint32_t* quad_roots = nullptr;
+  int quad_stack = 0;                  // entries a traversal of the four-child records can stack
   int depth = kMaxStack - 2;           // deepest node level of these records (bounds the stack use)
 };
 
@@ -99,6 +100,16 @@ cudaError_t launch_raycast_first_persistent(const MeshDev& m, const BatchDev* ba
                                             bvhc_hit* out, unsigned long long* work, const TraversalConfig& cfg,
                                             cudaStream_t stream, uint32_t* queue = nullptr,
                                             unsigned int* qcount = nullptr, const RaySort* sort = nullptr);
+// Its traversals over the four-child records (no finalize): four lanes per ray (group_stack(m) > 0) and
+// one (phased_stack(m), n < 2^32).  `work` is reset here when it is used.
+cudaError_t launch_raycast_first_group(const MeshDev& m, const BatchDev* batch, const float* rays, uint64_t n, int side,
+                                       const SideTable& sides, float near_d, float far_d, bvhc_hit* out,
+                                       unsigned long long* work, cudaStream_t stream, const uint32_t* queue,
+                                       const unsigned int* qcount);
+cudaError_t launch_raycast_first_phased(const MeshDev& m, const BatchDev* batch, const float* rays, uint64_t n,
+                                        int side, const SideTable& sides, float near_d, float far_d, bvhc_hit* out,
+                                        unsigned long long* work, cudaStream_t stream, const uint32_t* queue,
+                                        const unsigned int* qcount);
 // Completes the pending records a traversal left in `out` (record index in face_index), for the
 // queued rays (queue / qcount) or all n.
 cudaError_t launch_finalize_first(const MeshDev& m, const float* rays, uint64_t n, bvhc_hit* out,
@@ -232,10 +243,10 @@ struct RefitPlan {
 // changed; force = true recomputes every box.  tri_vid: 3 vertex ids per triangle (faceIndex).
 cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris, const uint32_t* tri_vid,
                          const float* pos, int stride, bool force, cudaStream_t stream);
-// Copies every four-child record's child boxes from the child-pair slots they were collapsed from
-// (src: 4 per record, kEmptyLeaf for an unused child).
+// Every four-child record's child boxes, from the child-pair slots they were collapsed from (src: 4
+// per record) or, for parts of a leaf (src kLeafBit | first), from their triangle records.
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
-                              cudaStream_t stream);
+                              const TriRecord* tris, cudaStream_t stream);
 
 // What another translation unit needs to launch on a mesh: its device view, traversal variant and
 // device ordinal (defined in api.cu).  Returns false for a null mesh.

@@ -73,37 +73,23 @@ __global__ void __launch_bounds__(kBlock) raycast_first_kernel(MeshDev m, const 
 }
 
 // ---------------------------------------------------------------------------------------------
-// raycastFirst, persistent form.  A fixed grid of warps pulls rays from a global work counter in
-// chunks of 32..kChunk rays per warp (one atomicAdd per chunk); a lane whose ray is finished sits idle
-// until `refill` lanes of its warp are idle, and then those lanes take the next rays of the warp's
-// chunk together, so warps stay full while rays of very different cost (early misses, deep
-// traversals) are mixed.  Each outer iteration runs the "while-while" phases: every lane walks
-// child pairs until it reaches a leaf or finishes, then the lanes holding a leaf test it together.
-// A finished hit is written as a pending (record, t) pair; finalize_first_kernel then computes the
-// reported records one ray per thread, so the float-float work runs with full warps.
+// raycastFirst, persistent form over child pairs: what runs where the four-child records do not serve
+// (trees too deep for their stacks, more than 2^29 triangle records, 2^32 rays or more; otherwise
+// kernels_phased.cu and kernels_group.cu).  A fixed grid of warps pulls rays from a global work counter
+// in chunks of 32..kChunk rays per warp (one atomicAdd per chunk); a lane whose ray is finished sits
+// idle until `refill` lanes of its warp are idle, and then those lanes take the next rays of the warp's
+// chunk together.  Each outer iteration runs the "while-while" phases: every lane walks child pairs
+// until it reaches a leaf or finishes, then the lanes holding a leaf test it together.  A finished hit
+// is written as a pending (record, t) pair; finalize_first_kernel then computes the reported records
+// one ray per thread, so the float-float work runs with full warps.
 // ---------------------------------------------------------------------------------------------
 constexpr unsigned kChunk = 256;
-
-// Mesh of ray `rid` in a batch: the last mesh whose first ray is <= rid (ray_off is CSR).
-__device__ __forceinline__ int mesh_of_ray(const BatchDev& bd, uint64_t rid) {
-  int lo = 0, hi = bd.n_meshes - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (__ldg(bd.ray_off + mid) <= rid) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
 
 // BATCHED: every ray belongs to one of many meshes packed into one node/triangle pool (the
 // meshes of a BatchedMesh, ExtensionUtilities.js:87-161); a lane looks up its ray's mesh when it
 // takes the ray and traverses that mesh's roots.  Otherwise the mesh's roots are m.roots[0..n).
-// MINB: minimum resident blocks per SM requested from the register allocator (1 = no limit).
-// WIDE: walk the four-child records (m.quads, m.quad_roots; same leaves and triangle records):
-// half the levels, so half as many dependent node loads per ray; at a record the children the ray
-// enters are taken nearest first (ORDER does not apply) and the others stacked farthest first.
-template <int ORDER, bool BATCHED, int MINB, int STACK, bool WIDE = false>
-__global__ void __launch_bounds__(kBlock, MINB) raycast_first_persistent_kernel(
+template <bool BATCHED>
+__global__ void __launch_bounds__(kBlock) raycast_first_persistent_kernel(
     MeshDev m, const BatchDev bd, const float* __restrict__ rays, uint64_t n, int side, const SideTable sides,
     float near_d, float far_d, bvhc_hit* __restrict__ out, unsigned long long* __restrict__ work, int refill,
     const uint32_t* __restrict__ queue, const unsigned int* __restrict__ qcount) {
@@ -123,8 +109,8 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_persistent_kernel(
   Best best{kInf, 0.0f, 0xFFFFFFFFu};
   uint32_t link = 0;
   int sp = 0, root = 0, root_end = m.n_roots;
-  uint32_t stack_link[STACK];
-  float stack_t[STACK];
+  uint32_t stack_link[kMaxStack];
+  float stack_t[kMaxStack];
   uint64_t pool = 0, pool_end = 0;  // warp-uniform: this warp's untaken rays [pool, pool_end)
   bool drained = false;             // warp-uniform: the work counter is exhausted
 
@@ -140,7 +126,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_persistent_kernel(
       }
     }
     if (++root < root_end) {
-      link = WIDE ? m.quad_roots[root] : m.roots[root];
+      link = m.roots[root];
       return;
     }
     store_first_pending(out + rid, best);  // finalize_first_kernel completes a hit
@@ -185,7 +171,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_persistent_kernel(
             root_end = m.n_roots;
           }
           sp = 0;
-          link = WIDE ? m.quad_roots[root] : m.roots[root];
+          link = m.roots[root];
         }
       }
       if (need <= avail) {
@@ -198,78 +184,18 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_persistent_kernel(
       if (idle == 0xFFFFFFFFu && __ballot_sync(0xFFFFFFFFu, active) == 0u) break;
     }
     if (!active) continue;
-    // phase 1: child pairs (or four-child records), until this lane holds a leaf or has finished
-    // its ray
-    while (WIDE && active && !(link & kLeafBit)) {
-      const QuadNode* qn = m.quads + link;
-      float4 lx, ly, lz, hx, hy, hz;
-      ld8(qn->lo[0], lx, ly);
-      ld8(qn->lo[2], lz, hx);
-      ld8(qn->hi[1], hy, hz);
-      const float4 lk = ld4(qn->link);
-      const uint32_t ck[4] = {__float_as_uint(lk.x), __float_as_uint(lk.y), __float_as_uint(lk.z),
-                              __float_as_uint(lk.w)};
-      const float blo[3][4] = {{lx.x, lx.y, lx.z, lx.w}, {ly.x, ly.y, ly.z, ly.w}, {lz.x, lz.y, lz.z, lz.w}};
-      const float bhi[3][4] = {{hx.x, hx.y, hx.z, hx.w}, {hy.x, hy.y, hy.z, hy.w}, {hz.x, hz.y, hz.z, hz.w}};
-      const float lim = fminf(far_d, (best.t + best.err) * (1.0f + kSlabMargin));
-      float key[4];
-      uint32_t cl[4];
-      int nh = 0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float e;
-        const bool h = ck[c] != kEmptyLeaf &&
-                       box_hit(blo[0][c], blo[1][c], blo[2][c], bhi[0][c], bhi[1][c], bhi[2][c], r, near_d, lim, e);
-        key[c] = h ? e : kInf;
-        cl[c] = ck[c];
-        nh += h ? 1 : 0;
-      }
-      // the four (entry, child) pairs nearest first; children the ray misses sort last
-      auto cas = [&](int a, int c) {
-        if (key[c] < key[a]) {
-          const float tk = key[a];
-          key[a] = key[c];
-          key[c] = tk;
-          const uint32_t tl = cl[a];
-          cl[a] = cl[c];
-          cl[c] = tl;
-        }
-      };
-      cas(0, 1);
-      cas(2, 3);
-      cas(0, 2);
-      cas(1, 3);
-      cas(1, 2);
-      if (nh == 0) {
-        pop_next();
-      } else if (sp + nh - 1 > STACK) {
-        atomicOr(m.err, kErrStackOverflow);
-        best.rec = 0xFFFFFFFFu;
-        sp = 0;
-        root = root_end;
-        pop_next();
-      } else {
-#pragma unroll
-        for (int j = 3; j >= 1; --j)
-          if (j < nh) {
-            stack_link[sp] = cl[j];
-            stack_t[sp] = key[j];
-            ++sp;
-          }
-        link = cl[0];
-      }
-    }
-    while (!WIDE && active && !(link & kLeafBit)) {
+    // phase 1: child pairs, until this lane holds a leaf or has finished its ray
+    while (active && !(link & kLeafBit)) {
       Pair p = load_pair(m.nodes, link);
       float lim = fminf(far_d, (best.t + best.err) * (1.0f + kSlabMargin));
       float e0, e1;
       bool h0 = box_hit(p.l[0], p.l[1], p.l[2], p.l[3], p.l[4], p.l[5], r, near_d, lim, e0);
       bool h1 = box_hit(p.r[0], p.r[1], p.r[2], p.r[3], p.r[4], p.r[5], r, near_d, lim, e1);
-      bool lf = left_first<ORDER>(p, r, e0, e1);
+      bool lf = left_first<1>(p, r, e0, e1);
       uint32_t c1 = lf ? p.ll : p.lr, c2 = lf ? p.lr : p.ll;
       bool h1st = lf ? h0 : h1, h2nd = lf ? h1 : h0;
       if (h1st && h2nd) {
-        if (sp >= STACK) {
+        if (sp >= kMaxStack) {
           atomicOr(m.err, kErrStackOverflow);
           best.rec = 0xFFFFFFFFu;
           sp = 0;
@@ -396,75 +322,6 @@ __global__ void __launch_bounds__(kClsThreads) classify_kernel(
 
 }  // namespace dev
 
-// Resident blocks per SM x SM count for a persistent kernel on the current device, cached per
-// (device, kernel variant).
-template <class K>
-static unsigned int persistent_grid(K kernel, int variant) {
-  constexpr int kDevs = 64, kVariants = 30;
-  static unsigned int cache[kDevs][kVariants] = {};
-  int dev_id = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev_id);
-  if (dev_id >= 0 && dev_id < kDevs && cache[dev_id][variant]) return cache[dev_id][variant];
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, dev::kBlock, 0);
-  unsigned int g = (unsigned int)(std::max(1, sms) * std::max(1, per_sm));
-  if (dev_id >= 0 && dev_id < kDevs) cache[dev_id][variant] = g;
-  return g;
-}
-
-struct PersistentArgs {
-  MeshDev m;
-  BatchDev bd;
-  const float* rays;
-  uint64_t n;
-  int side;
-  SideTable sides;
-  float near_d, far_d;
-  bvhc_hit* out;
-  unsigned long long* work;
-  int refill;
-  const uint32_t* queue;
-  const unsigned int* qcount;
-};
-
-template <int ORDER, bool BATCHED, int MINB, int STACK, bool WIDE = false>
-static void launch_persistent(const PersistentArgs& a, cudaStream_t stream) {
-  auto kernel = dev::raycast_first_persistent_kernel<ORDER, BATCHED, MINB, STACK, WIDE>;
-  const int occ_id = MINB == 1 ? 0 : (MINB == 6 ? 1 : 2);
-  int variant = WIDE ? 24 + (BATCHED ? 3 : 0) + occ_id : (STACK == 32 ? 12 : 0) + ORDER * 6 + (BATCHED ? 3 : 0) + occ_id;
-  unsigned int g = persistent_grid(kernel, variant);
-  g = (unsigned int)std::min<uint64_t>(g, (a.n + dev::kBlock - 1) / dev::kBlock);
-  kernel<<<g, dev::kBlock, 0, stream>>>(a.m, a.bd, a.rays, a.n, a.side, a.sides, a.near_d, a.far_d, a.out, a.work,
-                                        a.refill, a.queue, a.qcount);
-}
-
-template <int ORDER, bool BATCHED, int STACK>
-static void launch_persistent_occ(const PersistentArgs& a, int occupancy, cudaStream_t stream) {
-  if (occupancy == 0) launch_persistent<ORDER, BATCHED, 1, STACK>(a, stream);
-  else if (occupancy == 1) launch_persistent<ORDER, BATCHED, 6, STACK>(a, stream);
-  else launch_persistent<ORDER, BATCHED, 8, STACK>(a, stream);
-}
-
-template <bool BATCHED>
-static void launch_persistent_cfg(const PersistentArgs& a, const TraversalConfig& cfg, cudaStream_t stream) {
-  if (cfg.wide && a.m.quads && a.m.quad_roots) {
-    // four-child records: nearest child first, the 64-entry stack (a record stacks up to three);
-    // a batch's meshes index their quad roots as their child-pair roots
-    if (cfg.occupancy == 0) launch_persistent<1, BATCHED, 1, 64, true>(a, stream);
-    else if (cfg.occupancy == 1) launch_persistent<1, BATCHED, 6, 64, true>(a, stream);
-    else launch_persistent<1, BATCHED, 8, 64, true>(a, stream);
-    return;
-  }
-  const bool s32 = stack_entries(a.m, cfg.stack) == 32;
-  if (cfg.order == 0) {
-    if (s32) launch_persistent_occ<0, BATCHED, 32>(a, cfg.occupancy, stream);
-    else launch_persistent_occ<0, BATCHED, 64>(a, cfg.occupancy, stream);
-  } else {
-    if (s32) launch_persistent_occ<1, BATCHED, 32>(a, cfg.occupancy, stream);
-    else launch_persistent_occ<1, BATCHED, 64>(a, cfg.occupancy, stream);
-  }
-}
-
 // Root-box pre-pass into `queue`, then (single mesh, sort requested) the ray-ordering sort.
 cudaError_t prepare_queue(const MeshDev& m, const BatchDev* batch, const float* rays, uint64_t n, float near_d,
                                  float far_d, bvhc_hit* out, uint32_t* queue, unsigned int* qcount,
@@ -503,21 +360,31 @@ cudaError_t launch_raycast_first_persistent(const MeshDev& m, const BatchDev* ba
                                             cudaStream_t stream, uint32_t* queue, unsigned int* qcount,
                                             const RaySort* sort) {
   if (n == 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(work, 0, sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   const bool compact = queue != nullptr && qcount != nullptr && n < (1ull << 32);
-  BatchDev bd = batch ? *batch : BatchDev{nullptr, nullptr, 0};
   if (compact) {
     e = prepare_queue(m, batch, rays, n, near_d, far_d, out, queue, qcount, sort, stream);
     if (e != cudaSuccess) return e;
+  } else {
+    queue = nullptr;
+    qcount = nullptr;
   }
-  PersistentArgs a{m, bd, rays, n, side, sides, near_d, far_d, out, work, cfg.refill,
-                   compact ? queue : nullptr, compact ? qcount : nullptr};
-  if (batch) launch_persistent_cfg<true>(a, cfg, stream);
-  else launch_persistent_cfg<false>(a, cfg, stream);
-  e = cudaGetLastError();
+  if (n <= kGroupMaxRays && group_stack(m)) {
+    e = launch_raycast_first_group(m, batch, rays, n, side, sides, near_d, far_d, out, work, stream, queue, qcount);
+  } else if (n < (1ull << 32) && phased_stack(m)) {
+    e = launch_raycast_first_phased(m, batch, rays, n, side, sides, near_d, far_d, out, work, stream, queue, qcount);
+  } else {
+    e = cudaMemsetAsync(work, 0, sizeof(unsigned long long), stream);
+    if (e != cudaSuccess) return e;
+    const BatchDev bd = batch ? *batch : BatchDev{nullptr, nullptr, 0};
+    auto kernel = batch ? dev::raycast_first_persistent_kernel<true> : dev::raycast_first_persistent_kernel<false>;
+    const unsigned int grid = (unsigned int)std::min<uint64_t>((uint64_t)sm_count() * 4, (n + dev::kBlock - 1) / dev::kBlock);
+    kernel<<<grid, dev::kBlock, 0, stream>>>(m, bd, rays, n, side, sides, near_d, far_d, out, work, cfg.refill, queue,
+                                             qcount);
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess) return e;
-  return launch_finalize_first(m, rays, n, out, a.queue, a.qcount, stream);
+  return launch_finalize_first(m, rays, n, out, queue, qcount, stream);
 }
 
 cudaError_t launch_finalize_first(const MeshDev& m, const float* rays, uint64_t n, bvhc_hit* out,

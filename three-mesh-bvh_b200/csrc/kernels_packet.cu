@@ -113,16 +113,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) raycast_first_packet_kernel(MeshD
 
 // ---------------------------------------------------------------------------------------------
 // raycastFirst, warp-cooperative over the four-child records (m.quads): the same shared traversal
-// as above with half as many node visits.  At a record each lane tests the four child boxes (one
-// 16-byte load per bound plane serves all four); the children any lane enters are ordered by the
-// entry distances of the first lane that enters one (the warp's rays are coherent), the nearest is
+// as above with half as many node visits.  At a record each lane tests the four child boxes; the
+// children any lane enters are ordered by the entry distances of the first lane that enters one (the warp's rays are coherent), the nearest is
 // visited and the others are stacked farthest first, each with every lane's own entry distance.
 // ---------------------------------------------------------------------------------------------
 template <int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
     MeshDev m, const float* __restrict__ rays, uint64_t n, int side, const SideTable sides, float near_d,
     float far_d, bvhc_hit* __restrict__ out, const uint32_t* __restrict__ queue,
-    const unsigned int* __restrict__ qcount, uint64_t pitch, int rows_log2) {
+    const unsigned int* __restrict__ qcount, uint64_t pitch, int rows_log2, bool ranged_call) {
   __shared__ uint32_t s_link[kWarps][kMaxStack];
   const unsigned full = 0xFFFFFFFFu;
   const int w = threadIdx.x >> 5;
@@ -144,6 +143,9 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
     r.inv = make_float3(1.f, 1e30f, 1e30f);
     r.dk = kFilterK;
   }
+  const RaySlab rs = ray_slab(r);
+  const float near_s = slab_near(near_d);
+  const bool odd = ranged_call && odd_length(r.d);  // parts of leaves are not held against near and far
   Best best{kInf, 0.0f, 0xFFFFFFFFu};
   float lane_t[kMaxStack];
   for (int root = 0; root < m.n_roots; ++root) {
@@ -152,30 +154,27 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
     for (;;) {
       bool pop = false;
       if (link & kLeafBit) {
-        if (link != kEmptyLeaf && valid) leaf_first(m, link & ~kLeafBit, r, dlen, side, sides, near_d, far_d, best);
+        if (valid) run_first(m, link, r, dlen, side, sides, near_d, far_d, best);
         pop = true;
       } else {
-        // 112 of the record's 128 bytes: three 256-bit loads and one 128-bit load (the quad array is
-        // one allocation of 128-byte records)
-        const QuadNode* qn = m.quads + link;
-        float4 lx, ly, lz, hx, hy, hz;
-        ld8(qn->lo[0], lx, ly);
-        ld8(qn->lo[2], lz, hx);
-        ld8(qn->hi[1], hy, hz);
-        const float4 lk = ld4(qn->link);
-        const uint32_t ck[4] = {__float_as_uint(lk.x), __float_as_uint(lk.y), __float_as_uint(lk.z),
-                                __float_as_uint(lk.w)};
-        const float blo[3][4] = {{lx.x, lx.y, lx.z, lx.w}, {ly.x, ly.y, ly.z, ly.w}, {lz.x, lz.y, lz.z, lz.w}};
-        const float bhi[3][4] = {{hx.x, hx.y, hx.z, hx.w}, {hy.x, hy.y, hy.z, hy.w}, {hz.x, hz.y, hz.z, hz.w}};
-        const float lim = fminf(far_d, (best.t + best.err) * (1.0f + kSlabMargin));
+        // the record's four children: one 256-bit load each
+        ChildBox ch[4];
+        uint32_t ck[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          ch[c] = load_child(m.quads[link].c + c);
+          ck[c] = ch[c].link;
+        }
+        const float lim_hit = slab_limit((best.t + best.err) * (1.0f + kSlabMargin));
+        const float lim = fminf(slab_limit(far_d), lim_hit);
         float e[4];
         bool h[4];
         unsigned b[4];
         unsigned any = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          h[c] = valid && ck[c] != kEmptyLeaf &&
-                 box_hit(blo[0][c], blo[1][c], blo[2][c], bhi[0][c], bhi[1][c], bhi[2][c], r, near_d, lim, e[c]);
+          const bool free_box = odd && ch[c].part;
+          h[c] = child_hit(ch[c], rs, free_box ? 0.0f : near_s, free_box ? lim_hit : lim, e[c]) && valid;
           b[c] = __ballot_sync(full, h[c]);
           any |= b[c];
         }
@@ -233,7 +232,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
         bool found = false;
         while (sp > 0) {
           --sp;
-          float plim = (best.t + best.err) * (1.0f + kSlabMargin);
+          float plim = slab_limit((best.t + best.err) * (1.0f + kSlabMargin));
           if (__ballot_sync(full, valid && lane_t[sp] <= plim)) {
             link = s_link[w][sp];
             found = true;
@@ -287,7 +286,7 @@ cudaError_t launch_raycast_first_packet(const MeshDev& m, const float* rays, uin
               : cfg.occupancy == 1 ? dev::raycast_first_packet4_kernel<6>
                                    : dev::raycast_first_packet4_kernel<8>;
     k4<<<grid_for(n), dev::kBlock, 0, stream>>>(m, rays, n, side, sides, near_d, far_d, out, queue, qcount, pitch,
-                                                rl);
+                                                rl, dev::ranged(near_d, far_d));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_finalize_first(m, rays, n, out, queue, qcount, stream);

@@ -32,17 +32,58 @@ struct alignas(64) PairNode {
 };
 static_assert(sizeof(PairNode) == 64, "PairNode must be 64 bytes");
 
-// Four-child record for raycastFirst's warp-cooperative traversal, collapsed from the child-pair
-// tree (each internal child replaced by its own two children, largest surface area first, until
-// four children or only leaves remain).  Planes are stored per axis for the four children, so one
-// 16-byte load gives one bound of all four boxes.  Unused children have link kEmptyLeaf.
-struct alignas(64) QuadNode {
-  float lo[3][4];     // lo[axis][child]
-  float hi[3][4];     // hi[axis][child]
-  uint32_t link[4];   // internal child -> quad record index; leaf -> kLeafBit | first triangle record
-  uint32_t pad[4];
+// Four-child record of the ray queries, collapsed from the child-pair tree (each internal child
+// replaced in place by its own two children, largest surface area first, until there are four
+// children or only leaves; the children stay in the tree's left-to-right order).  A child is one
+// 32-byte sector (one 256-bit load): its box as centre and half extent, x and y side by side as the
+// operands of packed float instructions.  With centre and half extent a slab's entry and exit are
+// t_c -+ r, additions on the FMA pipe, where lo / hi planes need a minimum and a maximum per axis on
+// the half-rate ALU pipe.  The half extents are rounded up (box_centre_half), so the box holds the
+// reference's.  Unused children have link kEmptyLeaf and a NaN box, which no ray enters.  Every root is
+// a record: a root that is a leaf is one child with an unbounded box.
+struct alignas(32) QuadChild {
+  float c[2], h[2];   // x, y
+  float cz, hz;
+  uint32_t link;      // internal child -> quad record index; else a run of triangle records (run_link)
+  uint32_t count;     // a part of a leaf: its triangle records; 0 for a node or a whole leaf of the tree
+};
+struct alignas(128) QuadNode {
+  QuadChild c[4];
 };
 static_assert(sizeof(QuadNode) == 128, "QuadNode must be 128 bytes");
+
+constexpr float kBoxUnbounded = 3e38f;
+
+// A leaf of a four-child record: a run of at most kMaxRun consecutive triangle records of one of the
+// tree's leaves (a larger leaf has a record, or several, of parts with their own exact bounds), as
+// kLeafBit, the run's length less one in two bits, its first record in the rest.
+constexpr int kMaxRun = 4;
+constexpr int kRunShift = 29;
+constexpr uint32_t kRunFirst = (1u << kRunShift) - 1u;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+    inline uint32_t run_link(uint32_t first, int count) {
+  return kLeafBit | ((uint32_t)(count - 1) << kRunShift) | first;
+}
+
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+    // One axis of a box as centre and half extent.  The half extent carries 2^-20 (|c| + h) of slack:
+    // its own two roundings and the ray test's error in c (kernels' slab test) are under 8u (|c| + h),
+    // u = 2^-24.  Swapped bounds count as the box between them, as in the slab test with minimum and
+    // maximum; bounds that are not numbers, or too large, give an unbounded axis.
+    inline void box_centre_half(float lo, float hi, float& c, float& h) {
+  c = 0.5f * lo + 0.5f * hi;
+  const float a = hi - c, b = c - lo;
+  const float aa = a < 0.0f ? -a : a, ab = b < 0.0f ? -b : b, ac = c < 0.0f ? -c : c;
+  h = (aa > ab ? aa : ab) * (1.0f + 9.5367431640625e-07f) + ac * 9.5367431640625e-07f;
+  if (!(aa < kBoxUnbounded && ab < kBoxUnbounded && h < kBoxUnbounded)) {
+    c = 0.0f;
+    h = kBoxUnbounded;
+  }
+}
 
 struct alignas(16) TriRecord {
   // v[0..8] = a.xyz, b.xyz, c.xyz ; face = reference faceIndex ; flags bit 0 = last in leaf ;

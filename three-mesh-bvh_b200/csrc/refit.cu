@@ -82,30 +82,43 @@ __global__ void __launch_bounds__(kRefitBlock) refit_kernel(RefitPlan plan, Pair
   }
 }
 
-// Four-child records: each child box is copied from the child-pair slot it was collapsed from.
+// Four-child records: a child's box is that of the child-pair slot it was collapsed from, or for a part
+// of a leaf (src kLeafBit | first record) the bounds of its triangles.  The unbounded child of a root
+// that is a leaf (src kEmptyLeaf) keeps its box.
 __global__ void __launch_bounds__(kRefitBlock) quad_boxes_kernel(QuadNode* __restrict__ quads, uint64_t n_quads,
                                                                  const uint32_t* __restrict__ src,
-                                                                 const PairNode* __restrict__ pairs) {
+                                                                 const PairNode* __restrict__ pairs,
+                                                                 const TriRecord* __restrict__ tris) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= 4 * n_quads) return;
   const uint32_t slot = __ldg(src + k);
+  QuadChild& c = quads[k >> 2].c[k & 3u];
+  float b[6];
   if (slot == kEmptyLeaf) return;
-  const float* b = pairs[slot >> 1].f + 6 * (slot & 1u);
-  QuadNode& q = quads[k >> 2];
-  const int c = (int)(k & 3u);
-  for (int a = 0; a < 3; ++a) {
-    q.lo[a][c] = b[a];
-    q.hi[a][c] = b[3 + a];
+  if (!(slot & kLeafBit)) {
+    const float* f = pairs[slot >> 1].f + 6 * (slot & 1u);
+    for (int a = 0; a < 6; ++a) b[a] = f[a];
+  } else {
+    const TriRecord* t = tris + (slot & ~kLeafBit);
+    for (int a = 0; a < 3; ++a) b[a] = b[3 + a] = t->v[a];
+    for (uint32_t q = 0; q < c.count; ++q)
+      for (int a = 0; a < 9; ++a) {
+        b[a % 3] = fminf(b[a % 3], t[q].v[a]);
+        b[3 + a % 3] = fmaxf(b[3 + a % 3], t[q].v[a]);
+      }
   }
+  box_centre_half(b[0], b[3], c.c[0], c.h[0]);
+  box_centre_half(b[1], b[4], c.c[1], c.h[1]);
+  box_centre_half(b[2], b[5], c.cz, c.hz);
 }
 
 }  // namespace dev
 
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
-                              cudaStream_t stream) {
+                              const TriRecord* tris, cudaStream_t stream) {
   if (n_quads == 0) return cudaSuccess;
   const unsigned int grid = (unsigned int)((4 * n_quads + dev::kRefitBlock - 1) / dev::kRefitBlock);
-  dev::quad_boxes_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(quads, n_quads, src, pairs);
+  dev::quad_boxes_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(quads, n_quads, src, pairs, tris);
   return cudaGetLastError();
 }
 

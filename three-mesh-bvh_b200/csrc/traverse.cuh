@@ -85,6 +85,99 @@ __device__ __forceinline__ bool box_hit(float x0, float y0, float z0, float x1, 
   return en <= ex && en <= far_d && ex >= near_d;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Four-child records: the slab test on centre and half extent.
+// ---------------------------------------------------------------------------------------------
+// Two float operations in one instruction (sm_100's packed float32 forms; each half rounds as the
+// scalar operation does).
+struct f2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f2 f2_make(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_split(f2 a, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {  // a - b as one fused multiply-add by -1
+  f2 r;
+  const f2 m = f2_make(-1.0f, -1.0f);
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(m.v), "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// A ray as the slab test reads it: reciprocal direction, -origin / direction, |reciprocal| and the
+// slack of the origin's part.  An exact slab bound (p - o) / d of a box with centre c and half extent
+// h (before box_centre_half's slack) is within 4u (|c| + |o|) |inv| (centre: the reciprocal's ulp, the
+// rounding of o inv and of the sum) plus 5u (|o| + |c| + h) |inv| (radius and final sum) of t_c -+ r;
+// the half extent's slack of 16u (|c| + h) and s = 16u |o| |inv| cover that, so entry and exit here
+// lie outside the exact ones.
+struct RaySlab {
+  f2 inv, noi, ainv, s;          // x, y
+  float invz, noiz, ainvz, sz;
+};
+__device__ __forceinline__ RaySlab ray_slab(const RayF& r) {
+  RaySlab q;
+  const float ax = fabsf(r.inv.x), ay = fabsf(r.inv.y);
+  q.inv = f2_make(r.inv.x, r.inv.y);
+  q.noi = f2_make(-r.o.x * r.inv.x, -r.o.y * r.inv.y);
+  q.ainv = f2_make(ax, ay);
+  q.s = f2_make(0x1p-20f * fabsf(r.o.x) * ax, 0x1p-20f * fabsf(r.o.y) * ay);
+  q.invz = r.inv.z;
+  q.noiz = -r.o.z * r.inv.z;
+  q.ainvz = fabsf(r.inv.z);
+  q.sz = 0x1p-20f * fabsf(r.o.z) * q.ainvz;
+  return q;
+}
+
+// The limits of the slab test, widened: a box is entered when entry <= exit, entry <= lim and exit >=
+// near.  Every hit has t >= 0, so a negative near acts as 0; with a NaN near nothing is entered.
+__device__ __forceinline__ float slab_near(float near_d) { return near_d <= 0.0f ? 0.0f : near_d * (1.0f - 0x1p-19f); }
+__device__ __forceinline__ float slab_limit(float lim) { return lim * (1.0f + 0x1p-19f); }
+
+// near and far are distances, and the reference holds them against the ray parameter of its nodes'
+// boxes: for a direction that is not of unit length that drops hits by the extent of their leaf's box.
+// Parts of leaves, whose boxes the reference does not have, must then not be held against them: a
+// direction counts as of unit length while the difference is within the slack of the widened limits.
+// Calls with near <= 0 and no far have nothing to hold (RANGED false).
+static inline bool ranged(float near_d, float far_d) { return !(near_d <= 0.0f && far_d >= kInf); }
+__device__ __forceinline__ bool odd_length(float3 d) {
+  return !(fabsf(d.x * d.x + d.y * d.y + d.z * d.z - 1.0f) <= 0x1p-20f);
+}
+
+struct ChildBox {
+  f2 c, h;
+  float cz, hz;
+  uint32_t link, part;
+};
+__device__ __forceinline__ ChildBox load_child(const QuadChild* __restrict__ p) {
+  float4 a, b;
+  ld8(p, a, b);
+  return {f2_make(a.x, a.y), f2_make(a.z, a.w), b.x, b.y, __float_as_uint(b.z), __float_as_uint(b.w)};
+}
+__device__ __forceinline__ bool child_hit(const ChildBox& c, const RaySlab& r, float near_s, float lim, float& entry) {
+  const f2 t = f2_fma(c.c, r.inv, r.noi), q = f2_fma(c.h, r.ainv, r.s);
+  const float tz = fmaf(c.cz, r.invz, r.noiz), qz = fmaf(c.hz, r.ainvz, r.sz);
+  float nx, ny, fx, fy;
+  f2_split(f2_sub(t, q), nx, ny);
+  f2_split(f2_add(t, q), fx, fy);
+  const float en = max3(nx, ny, tz - qz), ex = min3(fx, fy, tz + qz);
+  entry = en;
+  return en <= ex && en <= lim && ex >= near_s;
+}
+
 struct Tri {
   float3 a, b, c;
   uint32_t face, flags, material;
@@ -258,6 +351,17 @@ __device__ __forceinline__ void leaf_first(const MeshDev& m, uint32_t k, const R
   }
 }
 
+// The same over a run of a four-child record.
+__device__ __forceinline__ void run_first(const MeshDev& m, uint32_t link, const RayF& r, float dlen, int side,
+                                          const SideTable& sides, float near_d, float far_d, Best& best) {
+  const uint32_t first = link & kRunFirst, end = first + ((link >> kRunShift) & 3u) + 1u;
+  for (uint32_t k = first; k < end; ++k) {
+    const Tri t = load_tri(m.tris, k);
+    const int ts = tri_side(t, side, sides);
+    if (ts >= 0) offer_first(m, t, k, r, dlen, ts, near_d, far_d, best);
+  }
+}
+
 // A pending record: the triangle record index in face_index, `t` in distance.  All 32 bytes are
 // written, so that the record's DRAM sector is written whole (a half-sector store makes L2 fetch
 // the other half first).
@@ -318,6 +422,17 @@ __device__ __forceinline__ uint64_t tiled_index(uint64_t i, uint64_t pitch, int 
   return b * band + ((r & 31u) >> cl) * pitch + ((r >> 5) << cl) + (r & ((1u << cl) - 1u));
 }
 
+// Mesh of ray `rid` in a batch: the last mesh whose first ray is <= rid (ray_off is CSR).
+__device__ __forceinline__ int mesh_of_ray(const BatchDev& bd, uint64_t rid) {
+  int lo = 0, hi = bd.n_meshes - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (__ldg(bd.ray_off + mid) <= rid) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
 // Pre-pass tiles (classify_kernel, kernels_first.cu).
 constexpr int kClsThreads = 256;
 constexpr int kClsItems = 8;
@@ -333,6 +448,31 @@ static inline unsigned int grid_for(uint64_t n) { return (unsigned int)((n + dev
 static inline int stack_entries(const MeshDev& m, int requested) {
   return requested == 32 && m.depth <= 30 ? 32 : 64;
 }
+
+// Streaming multiprocessors of the current device.
+static inline int sm_count() {
+  int dev_id = 0, sms = 0;
+  cudaGetDevice(&dev_id);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id);
+  return sms > 0 ? sms : 1;
+}
+
+// Whether a view has four-child records, and ones that the phased kernels' stack serves; the entries
+// of a group's stack (at most kMaxGroupStack), 0 when the group kernels cannot serve it.  Nothing ever
+// overflows either: what a traversal stacks is siblings along one path, and quad_stack counts the most
+// siblings of any path.
+constexpr int kMaxGroupStack = 96;
+static inline bool phased_stack(const MeshDev& m) { return m.quads && m.quad_roots && m.quad_stack <= kMaxStack; }
+static inline int group_stack(const MeshDev& m) {
+  return m.quads && m.quad_roots && m.quad_stack <= kMaxGroupStack ? (m.quad_stack < 1 ? 1 : m.quad_stack) : 0;
+}
+
+// Calls of up to this many rays take four lanes per ray, larger ones one lane.  With few rays the
+// longest ray's chain of dependent steps is the time, and four lanes make each step shorter; with many,
+// the chip is full and the lanes' own work counts.  Measured (box / sphere rays on the 10,000-,
+// 80,000- and 2M-triangle knots): 4,097 rays 50 / 64 / 87 us against 110 / 157 / 190 in one lane, 100,000
+// rays about even, 250,000 rays 246 / 294 / 403 against 195 / 254 / 458; between them the two cross.
+constexpr uint64_t kGroupMaxRays = 131072;
 
 // Root-box pre-pass into `queue`, then (single mesh, sort requested) the ray-ordering sort
 // (kernels_first.cu).
