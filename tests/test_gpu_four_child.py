@@ -81,3 +81,29 @@ def test_parts_of_leaves_follow_a_refit(pkg, cuda, leaf):
         want = bvh.raycast_first_batch(rays, 2)
         bvh.set_traversal(1, 1)
         assert torch.equal(bvh.raycast_first_batch(rays, 2).view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("mesh", ["triangle", "leaf40", "leaves40", "groups", "plain"])
+@pytest.mark.parametrize("n", [1, 7, 9, 33, 4097, 40_000])
+def test_closest_matches_the_per_query_kernel(pkg, cuda, mesh, n):
+    """closestPointToPoint in groups and by warps, in each query order, against the per-query kernel
+    (which a minThreshold above 0 selects; 1e-30 stops at nothing else than a point on the mesh)."""
+    import torch
+
+    g, opts = _mesh(pkg, mesh)
+    bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH, **opts})
+    rng = np.random.default_rng(n)
+    lo, hi = g.position.min(0) - 2, g.position.max(0) + 2
+    pts = (lo + rng.random((n, 3)) * (hi - lo)).astype(np.float32)
+    pts[::4] = g.position[rng.integers(0, g.position.shape[0], pts[::4].shape[0])] * np.float32(1.01) + np.float32(0.01)
+    if n > 30:
+        pts[3:6] = [[np.nan, 0, 0], [0, np.inf, 0], [3e38, 0, 0]]
+    d = torch.from_numpy(pts).to(cuda)
+    for far in (math.inf, 1.5, 0.0):
+        bvh.set_traversal(closest=0)
+        want = bvh.closest_point_batch(d, 1e-30, far).view(torch.int32)
+        for kw in (dict(closest=0), dict(closest=1), dict(closest=1, tile=32, tile_rows=4), dict(closest=2)):
+            bvh.set_traversal(**kw)
+            got = bvh.closest_point_batch(d, 0.0, far)
+            bvh.synchronize()
+            assert torch.equal(got.view(torch.int32), want), (far, kw)

@@ -100,28 +100,40 @@ struct bvhc_mesh {
   void* d_refit_pos = nullptr;
   size_t refit_pos_cap = 0;
 
-  // four-child records over raycastFirst's child-pair records (same triangle records), with the
-  // child-pair slot each quad child's box comes from
-  QuadNode* d_quads = nullptr;
-  uint32_t* d_quad_roots = nullptr;
-  uint32_t* d_quad_src = nullptr;
-  uint64_t n_quads = 0;
-  int quad_stack = 0;
+  // four-child records: [0] over the reference's leaves, with the lo / hi form closestPointToPoint
+  // reads; [1] over raycastFirst's split-leaf copy
+  struct QuadSet {
+    QuadNode* quads = nullptr;
+    BoxNode* boxes = nullptr;
+    uint32_t* roots = nullptr;
+    uint32_t* src = nullptr;  // where each child's box comes from (QuadBuilder::src)
+    uint64_t n = 0;
+    int stack = 0;
+  };
+  QuadSet quad_set[2];
 
   // the records raycastFirst traverses
   MeshDev view_first() const {
-    MeshDev v = leaf_size ? MeshDev{d_nodes_f, d_tris_f, d_roots_f, n_roots, d_err} : view();
-    v.quads = d_quads;
-    v.quad_roots = d_quad_roots;
-    v.quad_stack = quad_stack;
-    v.depth = leaf_size ? max_depth_f : max_depth;
+    if (!leaf_size) return view();
+    MeshDev v{d_nodes_f, d_tris_f, d_roots_f, n_roots, d_err};
+    set_quads(v, quad_set[1]);
+    v.depth = max_depth_f;
     return v;
   }
 
   MeshDev view() const {
     MeshDev v{d_nodes, d_tris, d_roots, n_roots, d_err};
+    set_quads(v, quad_set[0]);
     v.depth = max_depth;
     return v;
+  }
+
+ private:
+  static void set_quads(MeshDev& v, const QuadSet& q) {
+    v.quads = q.quads;
+    v.boxes = q.boxes;
+    v.quad_roots = q.roots;
+    v.quad_stack = q.stack;
   }
 };
 
@@ -608,6 +620,7 @@ struct QuadBuilder {
     q.c[0] = q.c[1] = q.cz = 0.0f;
     q.h[0] = q.h[1] = q.hz = kBoxUnbounded;
     q.link = l;
+    q.count = c.count;
     return idx;
   }
 
@@ -728,18 +741,20 @@ static void keep_serialized(bvhc_mesh* m, std::vector<std::vector<uint8_t>> root
   }
 }
 
-// Four-child records over raycastFirst's child-pair layout (pairs + roots), replacing any before.
-static cudaError_t install_quads(bvhc_mesh* m, const std::vector<PairNode>& pairs, const std::vector<TriRecord>& tris,
-                                 const std::vector<uint32_t>& roots) {
-  if (tris.size() >= kRunFirst) {  // more records than a run link can name: the child-pair kernels run
-    cudaFree(m->d_quads);
-    cudaFree(m->d_quad_roots);
-    cudaFree(m->d_quad_src);
-    m->d_quads = nullptr;
-    m->d_quad_roots = m->d_quad_src = nullptr;
-    m->n_quads = 0;
-    return cudaSuccess;
-  }
+static void free_quads(bvhc_mesh::QuadSet& q) {
+  cudaFree(q.quads);
+  cudaFree(q.boxes);
+  cudaFree(q.roots);
+  cudaFree(q.src);
+  q = bvhc_mesh::QuadSet{};
+}
+
+// Four-child records over a child-pair layout, into set `k`, replacing any before.  A mesh with more
+// triangle records than a run link can name has none: the child-pair kernels run.
+static cudaError_t install_quads(bvhc_mesh* m, int k, const std::vector<PairNode>& pairs,
+                                 const std::vector<TriRecord>& tris, const std::vector<uint32_t>& roots) {
+  free_quads(m->quad_set[k]);
+  if (tris.size() >= kRunFirst) return cudaSuccess;
   QuadBuilder qb{pairs, tris};
   std::vector<uint32_t> qroots(roots.size());
   try {
@@ -751,25 +766,22 @@ static cudaError_t install_quads(bvhc_mesh* m, const std::vector<PairNode>& pair
   } catch (const std::bad_alloc&) {
     return cudaErrorMemoryAllocation;
   }
-  QuadNode* q = nullptr;
-  uint32_t *qr = nullptr, *qs = nullptr;
-  cudaError_t e = upload(&q, qb.quads);
-  if (e == cudaSuccess) e = upload(&qr, qroots);
-  if (e == cudaSuccess) e = upload(&qs, qb.src);
+  bvhc_mesh::QuadSet q;
+  cudaError_t e = upload(&q.quads, qb.quads);
+  if (e == cudaSuccess) e = upload(&q.roots, qroots);
+  if (e == cudaSuccess) e = upload(&q.src, qb.src);
+  q.n = qb.quads.size();
+  q.stack = qb.stack;
+  if (k == 0) {
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&q.boxes), q.n * sizeof(BoxNode));
+    if (e == cudaSuccess) e = launch_quad_boxes(q.quads, q.n, q.src, m->d_nodes, m->d_tris, q.boxes, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  }
   if (e != cudaSuccess) {
-    cudaFree(q);
-    cudaFree(qr);
-    cudaFree(qs);
+    free_quads(q);
     return e;
   }
-  cudaFree(m->d_quads);
-  cudaFree(m->d_quad_roots);
-  cudaFree(m->d_quad_src);
-  m->d_quads = q;
-  m->d_quad_roots = qr;
-  m->d_quad_src = qs;
-  m->n_quads = qb.quads.size();
-  m->quad_stack = qb.stack;
+  m->quad_set[k] = q;
   return cudaSuccess;
 }
 
@@ -1016,7 +1028,7 @@ bvhc_status bvhc_mesh_create(int device, int version, const void* const* roots, 
   bvhc_status st = finish_mesh(device, pairs, tris, root_links, max_depth, {}, out);
   if (st == BVHC_OK) {
     keep_serialized(*out, std::move(copies), std::move(slot_nodes), index, index_elem_bytes, index_count, n_verts);
-    cudaError_t e = install_quads(*out, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
+    cudaError_t e = install_quads(*out, 0, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
     if (e != cudaSuccess) {
       bvhc_mesh_destroy(*out);
       *out = nullptr;
@@ -1081,7 +1093,7 @@ bvhc_status bvhc_batch_create(int device, int n_meshes, const int32_t* roots_per
   bvhc_status st = finish_mesh(device, pairs, tris, root_links, max_depth, mesh_root_off, out);
   if (st == BVHC_OK) {
     keep_serialized(*out, std::move(copies), std::move(slot_nodes), index, index_elem_bytes, index_count, n_verts);
-    cudaError_t e = install_quads(*out, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
+    cudaError_t e = install_quads(*out, 0, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
     if (e != cudaSuccess) {
       bvhc_mesh_destroy(*out);
       *out = nullptr;
@@ -1102,9 +1114,7 @@ void bvhc_mesh_destroy(bvhc_mesh* m) {
   cudaFree(m->d_roots_f);
   free_refit_plan(m->refit[0]);
   free_refit_plan(m->refit[1]);
-  cudaFree(m->d_quads);
-  cudaFree(m->d_quad_roots);
-  cudaFree(m->d_quad_src);
+  for (auto& q : m->quad_set) free_quads(q);
   cudaFree(m->d_tri_vid);
   cudaFree(m->d_refit_pos);
   cudaFree(m->d_err);
@@ -1331,8 +1341,8 @@ bvhc_status bvhc_mesh_set_leaf_size(bvhc_mesh* m, int max_leaf) {
   free_refit_plan(m->refit[1]);
   if (max_leaf > 0 && !m->h_root_bytes.empty())  // so that a refit keeps this copy in step
     BVHC_CUDA_TRY(build_refit_plan(pairs, tris, roots, serialized_root_boxes(m), m->refit[1]));
-  if (max_leaf > 0) BVHC_CUDA_TRY(install_quads(m, pairs, tris, roots));
-  else BVHC_CUDA_TRY(install_quads(m, m->h_pairs, m->h_tris, m->h_roots));
+  if (max_leaf > 0) BVHC_CUDA_TRY(install_quads(m, 1, pairs, tris, roots));
+  else free_quads(m->quad_set[1]);
   return BVHC_OK;
 }
 
@@ -1360,9 +1370,12 @@ bvhc_status bvhc_mesh_refit(bvhc_mesh* m, const float* positions, uint64_t n_ver
   BVHC_CUDA_TRY(launch_refit(m->refit[0], m->d_nodes, m->d_tris, m->d_tri_vid, pos, stride_floats, false, s));
   if (m->leaf_size > 0 && m->refit[1].leaves)  // raycastFirst's copy: every box recomputed
     BVHC_CUDA_TRY(launch_refit(m->refit[1], m->d_nodes_f, m->d_tris_f, m->d_tri_vid, pos, stride_floats, true, s));
-  if (m->d_quads)  // the four-child records take their boxes from raycastFirst's child pairs
-    BVHC_CUDA_TRY(launch_quad_boxes(m->d_quads, m->n_quads, m->d_quad_src, m->leaf_size > 0 ? m->d_nodes_f : m->d_nodes,
-                                    m->leaf_size > 0 ? m->d_tris_f : m->d_tris, s));
+  for (int k = 0; k < 2; ++k) {  // the four-child records follow their child pairs
+    const bvhc_mesh::QuadSet& q = m->quad_set[k];
+    if (q.quads)
+      BVHC_CUDA_TRY(launch_quad_boxes(q.quads, q.n, q.src, k ? m->d_nodes_f : m->d_nodes, k ? m->d_tris_f : m->d_tris,
+                                      q.boxes, s));
+  }
   if (m->d_pos && m->grad_verts <= n_verts) {  // the adjoint's vertex copy follows the geometry
     BVHC_CUDA_TRY(cudaMemcpy2DAsync(m->d_pos, 3 * sizeof(float), pos, stride_floats * sizeof(float),
                                     3 * sizeof(float), m->grad_verts, cudaMemcpyDeviceToDevice, s));
@@ -1828,15 +1841,13 @@ bvhc_status bvhc_closest_point_to_point(bvhc_mesh* m, const float* points, uint6
     // one launch; the sorted variant uses queue slot 3
     BVHC_CUDA_TRY(closest_sort(m, 3, n, min_threshold, &q, &qc, &sort));
     if (mem == BVHC_MEM_DEVICE)
-      return from_cuda(launch_closest_point(v, points, n, min_threshold, max_threshold, out, s, variant,
-                                            m->cfg.occupancy, q, qc, q ? &sort : nullptr, (uint32_t)m->cfg.tile,
+      return from_cuda(launch_closest_point(v, points, n, min_threshold, max_threshold, out, s, variant, q, qc, q ? &sort : nullptr, (uint32_t)m->cfg.tile,
                                             m->cfg.tile_rows));
     BVHC_CUDA_TRY(ensure(&m->d_in, &m->in_cap, n * 12));
     BVHC_CUDA_TRY(ensure(&m->d_out, &m->out_cap, n * sizeof(bvhc_closest)));
     BVHC_CUDA_TRY(cudaMemcpyAsync(m->d_in, points, n * 12, cudaMemcpyHostToDevice, s));
     BVHC_CUDA_TRY(launch_closest_point(v, static_cast<const float*>(m->d_in), n, min_threshold,
-                                       max_threshold, static_cast<bvhc_closest*>(m->d_out), s, variant,
-                                       m->cfg.occupancy, q, qc, q ? &sort : nullptr, (uint32_t)m->cfg.tile,
+                                       max_threshold, static_cast<bvhc_closest*>(m->d_out), s, variant, q, qc, q ? &sort : nullptr, (uint32_t)m->cfg.tile,
                                        m->cfg.tile_rows));
     BVHC_CUDA_TRY(cudaMemcpyAsync(out, m->d_out, n * sizeof(bvhc_closest), cudaMemcpyDeviceToHost, s));
     return read_and_clear_error(m, s);
@@ -1863,8 +1874,7 @@ bvhc_status bvhc_closest_point_to_point(bvhc_mesh* m, const float* points, uint6
     cudaStream_t st = m->pipe[k];
     BVHC_CUDA_TRY(cudaMemcpyAsync(m->slot_in[k], points + 3 * off, cnt * 12, cudaMemcpyHostToDevice, st));
     BVHC_CUDA_TRY(launch_closest_point(v, static_cast<const float*>(m->slot_in[k]), cnt, min_threshold,
-                                       max_threshold, static_cast<bvhc_closest*>(m->slot_out[k]), st, variant,
-                                       m->cfg.occupancy, qs[k], qcs[k], qs[k] ? &sorts[k] : nullptr,
+                                       max_threshold, static_cast<bvhc_closest*>(m->slot_out[k]), st, variant, qs[k], qcs[k], qs[k] ? &sorts[k] : nullptr,
                                        (uint32_t)m->cfg.tile, m->cfg.tile_rows));
     BVHC_CUDA_TRY(
         cudaMemcpyAsync(out + off, m->slot_out[k], cnt * sizeof(bvhc_closest), cudaMemcpyDeviceToHost, st));

@@ -24,6 +24,7 @@ struct MeshDev {
   unsigned int* err;
   const QuadNode* quads = nullptr;     // four-child copy of `nodes` (same triangle records), if any
   const uint32_t* quad_roots = nullptr;
+  const BoxNode* boxes = nullptr;      // the same records with lo / hi bounds (the reference's leaves only)
   int quad_stack = 0;                  // entries a traversal of the four-child records can stack
   int depth = kMaxStack - 2;           // deepest node level of these records (bounds the stack use)
 };
@@ -121,13 +122,12 @@ cudaError_t launch_raycast_first_packet(const MeshDev& m, const float* rays, uin
                                         const SideTable& sides, float near_d, float far_d, bvhc_hit* out,
                                         const TraversalConfig& cfg, cudaStream_t stream, uint32_t* queue = nullptr,
                                         unsigned int* qcount = nullptr, const RaySort* sort = nullptr);
-// closestPointToPoint.  variant 0: one query per thread; 1: warp-cooperative in input order; 2:
-// warp-cooperative over the queries sorted by a Morton key of the point (queue, qcount and sort
-// scratch for n queries required).  Variants 1 and 2 apply only with min_t <= 0 (else variant 0).
-// Variant 1 reads the queries in tiled order when `tile` is a row length (see tiled_index).
+// closestPointToPoint.  variant 0: the queries in input order; odd: in tiled order when `tile` is a row
+// length (see tiled_index), else in input order; even: sorted by a Morton key of the point (queue,
+// qcount and sort scratch for n queries required).  With min_t > 0 the per-query kernel over child
+// pairs runs, in input order.
 cudaError_t launch_closest_point(const MeshDev& m, const float* pts, uint64_t n, float min_t, float max_t,
-                                 bvhc_closest* out, cudaStream_t stream, int variant = 0, int occupancy = 0,
-                                 uint32_t* queue = nullptr, unsigned int* qcount = nullptr,
+                                 bvhc_closest* out, cudaStream_t stream, int variant = 0, uint32_t* queue = nullptr, unsigned int* qcount = nullptr,
                                  const RaySort* sort = nullptr, uint32_t tile = 0, int tile_rows = 0);
 
 // raycast (all hits).  variant 0: one ray per thread; 1: warp-cooperative in input order; 2:
@@ -244,9 +244,10 @@ struct RefitPlan {
 cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris, const uint32_t* tri_vid,
                          const float* pos, int stride, bool force, cudaStream_t stream);
 // Every four-child record's child boxes, from the child-pair slots they were collapsed from (src: 4
-// per record) or, for parts of a leaf (src kLeafBit | first), from their triangle records.
+// per record) or, for parts of a leaf (src kLeafBit | first), from their triangle records; `boxes`
+// (nullable) gets the same records with lo / hi bounds.
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
-                              const TriRecord* tris, cudaStream_t stream);
+                              const TriRecord* tris, BoxNode* boxes, cudaStream_t stream);
 
 // What another translation unit needs to launch on a mesh: its device view, traversal variant and
 // device ordinal (defined in api.cu).  Returns false for a null mesh.

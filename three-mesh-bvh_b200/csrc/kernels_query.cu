@@ -3,7 +3,7 @@
 // launches.
 #include <algorithm>
 
-#include "traverse.cuh"
+#include "closest.cuh"
 
 namespace bvhc {
 namespace dev {
@@ -17,46 +17,6 @@ namespace dev {
 // reference.  Candidate distances are compared in float32 with an error bound and re-compared
 // in float-float when the bound does not separate them.
 // ---------------------------------------------------------------------------------------------
-constexpr float kU = 5.9604644775390625e-08f;  // 2^-24
-
-__device__ __forceinline__ float box_score(const float* b, float3 p) {
-  float dx = fmaxf(b[0], fminf(b[3], p.x)) - p.x;
-  float dy = fmaxf(b[1], fminf(b[4], p.y)) - p.y;
-  float dz = fmaxf(b[2], fminf(b[5], p.z)) - p.z;
-  return dx * dx + dy * dy + dz * dz;
-}
-
-// Squared distance from p to the box's centre: the visiting order's tie-break when both child
-// boxes hold p (both scores 0), which the scores alone cannot order.
-__device__ __forceinline__ float centre_d2(const float* b, float3 p) {
-  const float dx = 0.5f * (b[0] + b[3]) - p.x, dy = 0.5f * (b[1] + b[4]) - p.y, dz = 0.5f * (b[2] + b[5]) - p.z;
-  return dx * dx + dy * dy + dz * dz;
-}
-
-// Whether the right child should be visited first: the smaller score, equal scores by the nearer
-// centre (the warp-cooperative forms; the per-query kernel keeps the reference's order).  The
-// centre distances are computed only on equal scores (written as a branch: as one expression they
-// were evaluated on every node, 4% of the grid's time).
-__device__ __forceinline__ bool right_nearer(const Pair& pr, float s0, float s1, float3 p) {
-  if (s1 != s0) return s1 < s0;
-  return centre_d2(pr.r, p) < centre_d2(pr.l, p);
-}
-
-__device__ __noinline__ ff box_score_ff(const float* b, float3 p) {
-  ff dx = two_diff(fmaxf(b[0], fminf(b[3], p.x)), p.x);
-  ff dy = two_diff(fmaxf(b[1], fminf(b[4], p.y)), p.y);
-  ff dz = two_diff(fmaxf(b[2], fminf(b[5], p.z)), p.z);
-  return ff_add(ff_add(ff_mul(dx, dx), ff_mul(dy, dy)), ff_mul(dz, dz));
-}
-
-// score < maxThreshold^2, decided exactly (the box score carries at most 5 roundings, all terms
-// positive, so 2^-20 relative slack separates every case the float32 value can settle).
-__device__ __forceinline__ bool under_max(float s, const float* b, float3 p, ff max2) {
-  if (s * (1.0f + kSlabMargin) < max2.hi * (1.0f - kSlabMargin)) return true;
-  if (s * (1.0f - kSlabMargin) > max2.hi * (1.0f + kSlabMargin)) return false;
-  return ff_lt(box_score_ff(b, p), max2);
-}
-
 // The best candidate of one query so far.
 struct CPBest {
   float d2, err;     // float32 squared distance and its error bound
@@ -87,25 +47,8 @@ __device__ __forceinline__ CPBest cp_none() {
 // itself keeps the answer independent of how queries are grouped and of how the triangles of a
 // leaf are laid out).  Every record holds a distinct faceIndex.  Returns the candidate's float32
 // squared distance and bound, and its float-float value when one was needed.
-// With `cull`, a triangle whose bounding box is already farther than the best candidate is
-// passed over without its closest point: its distance exceeds the best one, so it cannot win
-// (callers that test minThreshold on every triangle pass false).
 __device__ __forceinline__ void cp_offer(const MeshDev& m, float3 p, const Tri& t, uint32_t k, CPBest& b, float& d2,
-                                         float& err, bool& have_ff, ff& cand_ff, bool cull = false) {
-  if (cull && b.rec != 0xFFFFFFFFu) {
-    // squared distance to the triangle's box: at most 4 roundings above the exact value's
-    // relative 2^-22, so the 2^-20 shrink keeps it a lower bound
-    const float dx = fmaxf(fmaxf(fminf(t.a.x, fminf(t.b.x, t.c.x)) - p.x, p.x - fmaxf(t.a.x, fmaxf(t.b.x, t.c.x))), 0.0f);
-    const float dy = fmaxf(fmaxf(fminf(t.a.y, fminf(t.b.y, t.c.y)) - p.y, p.y - fmaxf(t.a.y, fmaxf(t.b.y, t.c.y))), 0.0f);
-    const float dz = fmaxf(fmaxf(fminf(t.a.z, fminf(t.b.z, t.c.z)) - p.z, p.z - fmaxf(t.a.z, fmaxf(t.b.z, t.c.z))), 0.0f);
-    const float lb = dx * dx + dy * dy + dz * dz;
-    if (lb * (1.0f - 0x1p-20f) > b.d2 + b.err) {
-      d2 = lb;
-      err = 0.0f;
-      have_ff = false;
-      return;
-    }
-  }
+                                         float& err, bool& have_ff, ff& cand_ff) {
   float3 q;
   float sc;
   d2 = closest_sq_f(p, t.a, t.b, t.c, q, sc);
@@ -152,24 +95,6 @@ __device__ __forceinline__ void cp_offer(const MeshDev& m, float3 p, const Tri& 
   }
 }
 
-// The reported record of triangle record `rec` (0xFFFFFFFF: none): distance and closest point in
-// float-float, rounded once.
-__device__ __forceinline__ void cp_store(const MeshDev& m, float3 p, uint32_t rec, bvhc_closest* o) {
-  if (rec == 0xFFFFFFFFu) {
-    o->face_index = BVHC_NO_HIT;
-    o->distance = kInf;
-    o->point[0] = o->point[1] = o->point[2] = 0.0f;
-    return;
-  }
-  Tri t = load_tri(m.tris, rec);
-  CPFF c = closest_ff(p, t.a, t.b, t.c);
-  o->face_index = t.face;
-  o->distance = ff_to_f(ff_sqrt(c.d2));
-  o->point[0] = ff_to_f(c.q.x);
-  o->point[1] = ff_to_f(c.q.y);
-  o->point[2] = ff_to_f(c.q.z);
-}
-
 __global__ void __launch_bounds__(kBlock) closest_point_kernel(MeshDev m, const float* __restrict__ pts, uint64_t n,
                                                                float min_t, float max_t,
                                                                bvhc_closest* __restrict__ out) {
@@ -194,7 +119,7 @@ __global__ void __launch_bounds__(kBlock) closest_point_kernel(MeshDev m, const 
             float d2, err;
             bool have_ff;
             ff cand_ff;
-            cp_offer(m, p, t, k, b, d2, err, have_ff, cand_ff, !(min2.hi > 0.0f));
+            cp_offer(m, p, t, k, b, d2, err, have_ff, cand_ff);
             // early out below minThreshold (closestPointToPoint.js:55-57)
             if (min2.hi > 0.0f) {
               bool below;
@@ -244,131 +169,57 @@ __global__ void __launch_bounds__(kBlock) closest_point_kernel(MeshDev m, const 
       if (!found) break;
     }
   }
-  out[i].face_index = b.rec;  // pending, as in the warp-cooperative kernel
+  out[i].face_index = b.rec;  // pending: closest_point_finalize_kernel completes the record
 }
 
-// ---------------------------------------------------------------------------------------------
-// closestPointToPoint, warp-cooperative form for spatially coherent queries (grids, SDF samples)
-// with minThreshold 0.  The 32 queries of a warp walk the tree together with one shared stack of
-// links: a child is entered when any lane wants it (its score under maxThreshold^2, decided
-// exactly, and not certainly above that lane's best), and each lane keeps, for the current node
-// and for every stacked child, whether it wants it (its own score, or NaN for "no").  A lane only
-// tests the triangles of leaves it wants, so every lane reaches exactly the leaves its own
-// traversal would and its result is the minimum over the same candidates: which leaves a query
-// reaches, and so the "null iff no leaf is reached" rule, does not depend on the visiting order,
-// and leaves skipped because of the best distance cannot hold a strictly closer triangle.  (With
-// minThreshold > 0 the reference stops at the first triangle below it in its own order, which a
-// shared order would not reproduce; those calls use the per-query kernel.)
-// ---------------------------------------------------------------------------------------------
-//
-// GROUP = 32 walks the tree with the whole warp; 16 and 8 split the warp into groups of that many
-// lanes (consecutive queries), each with its own shared stack: a group's node set is the union over
-// fewer, closer queries, and groups at different nodes on the same code path still issue together.
-template <int MINB, int GROUP>
-__global__ void __launch_bounds__(kBlock, MINB) closest_point_packet_kernel(
-    MeshDev m, const float* __restrict__ pts, uint64_t n, float max_t, bvhc_closest* __restrict__ out,
-    const uint32_t* __restrict__ queue, const unsigned int* __restrict__ qcount, uint64_t pitch, int rows_log2) {
-  static_assert(GROUP == 32 || GROUP == 16 || GROUP == 8, "group of 8, 16 or 32 lanes");
-  __shared__ uint32_t s_link[kBlock / GROUP][kMaxStack];
-  const int w = threadIdx.x / GROUP;                      // group within the block
-  const unsigned lane = threadIdx.x & (GROUP - 1u);       // lane within the group
-  const unsigned full = GROUP == 32 ? 0xFFFFFFFFu : ((1u << GROUP) - 1u) << ((threadIdx.x & 31u) & ~(GROUP - 1u));
-  const uint64_t n_work = queue ? (uint64_t)__ldg(qcount) : n;
-  if ((uint64_t)blockIdx.x * blockDim.x >= n_work) return;  // block-uniform
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < n_work;
-  if (valid && queue) i = __ldg(queue + i);
-  else if (valid && pitch) i = tiled_index(i, pitch, rows_log2, n);  // tiles of grid points
-  float3 p = make_float3(0.f, 0.f, 0.f);
-  if (valid) p = make_float3(__ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2));
-  const ff max2 = two_prod(max_t, max_t);
-  const float kNo = __int_as_float(0x7FFFFFFF);  // NaN: "this lane does not want the entry"
-  CPBest b = cp_none();
-  float lane_s[kMaxStack];
-  bool overflow = false;
-  for (int root = 0; root < m.n_roots && !overflow; ++root) {
-    uint32_t link = m.roots[root];
-    bool act = valid;  // this lane wants the current node (a root leaf has no bounds test)
-    int sp = 0;
-    for (;;) {
-      bool pop = false;
-      if (link & kLeafBit) {
-        if (link != kEmptyLeaf && act) {
-          uint32_t k = link & ~kLeafBit;
-          for (;;) {
-            Tri t = load_tri(m.tris, k);
-            float d2, err;
-            bool have_ff;
-            ff cand_ff;
-            cp_offer(m, p, t, k, b, d2, err, have_ff, cand_ff, true);
-            if (t.flags & kTriLast) break;
-            ++k;
-          }
-        }
-        pop = true;
-      } else {
-        Pair pr = load_pair(m.nodes, link);
-        float s0 = box_score(pr.l, p), s1 = box_score(pr.r, p);
-        float best_hi = b.d2 + b.err;
-        bool w0 = act && s0 * (1.0f - kSlabMargin) <= best_hi && under_max(s0, pr.l, p, max2);
-        bool w1 = act && s1 * (1.0f - kSlabMargin) <= best_hi && under_max(s1, pr.r, p, max2);
-        unsigned b0 = __ballot_sync(full, w0) & full, b1 = __ballot_sync(full, w1) & full;
-        if (b0 && b1) {
-          // nearer child first by majority of the lanes that want both (a lane wanting one prefers it)
-          bool pref_right = (w0 && w1) ? right_nearer(pr, s0, s1, p) : w1;
-          unsigned voters = __ballot_sync(full, w0 || w1) & full;
-          bool right_first = 2 * __popc(__ballot_sync(full, (w0 || w1) && pref_right) & full) > __popc(voters);
-          if (sp >= kMaxStack) {
-            if (lane == 0) atomicOr(m.err, kErrStackOverflow);
-            b = cp_none();
-            overflow = true;
-            break;
-          }
-          if (lane == 0) s_link[w][sp] = right_first ? pr.ll : pr.lr;
-          lane_s[sp] = right_first ? (w0 ? s0 : kNo) : (w1 ? s1 : kNo);
-          ++sp;
-          link = right_first ? pr.lr : pr.ll;
-          act = right_first ? w1 : w0;
-          __syncwarp(full);
-        } else if (b0) {
-          link = pr.ll;
-          act = w0;
-        } else if (b1) {
-          link = pr.lr;
-          act = w1;
-        } else {
-          pop = true;
-        }
-      }
-      if (pop) {
-        bool found = false;
-        while (sp > 0) {
-          --sp;
-          bool ok = lane_s[sp] * (1.0f - kSlabMargin) <= b.d2 + b.err;  // false for NaN
-          if (__ballot_sync(full, ok) & full) {
-            link = s_link[w][sp];
-            act = ok;
-            found = true;
-            break;
-          }
-        }
-        if (!found) break;
-      }
-    }
-  }
-  // pending: the record index in face_index; closest_point_finalize_kernel completes the record,
-  // which keeps the float-float code out of this kernel
-  if (valid) out[i].face_index = b.rec;
-}
-
-// Completes the records closest_point_kernel / closest_point_packet_kernel left pending, one query
-// per thread in input order.
+// Completes the records the traversals left pending, one query per thread in input order; `packed`:
+// five words as launch_closest_phased leaves them, else the triangle record alone.
 __global__ void __launch_bounds__(kBlock) closest_point_finalize_kernel(MeshDev m, const float* __restrict__ pts,
-                                                                        uint64_t n, bvhc_closest* __restrict__ out) {
+                                                                        uint64_t n, bvhc_closest* __restrict__ out,
+                                                                        bool packed) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float3 p = make_float3(__ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2));
-  cp_store(m, p, out[i].face_index, out + i);
+  const uint32_t* o = reinterpret_cast<const uint32_t*>(out + i);
+  const uint32_t pending = o[0];
+  bvhc_closest r;
+  if (pending == 0xFFFFFFFFu) {
+    r.face_index = BVHC_NO_HIT;
+    r.distance = kInf;
+    r.point[0] = r.point[1] = r.point[2] = 0.0f;
+    out[i] = r;
+    return;
+  }
+  uint32_t vertex = packed ? pending >> kRunShift : 3u;
+  Tri t = load_tri(m.tris, packed ? pending & kRunFirst : pending);
+  CPFF c = closest_ff(p, t.a, t.b, t.c);
+  // what the traversal could not settle: the same vertex is an exact tie, else the float-float distances
+  // decide; an exact tie goes to the smaller faceIndex
+  const uint32_t ties = packed ? o[1] : 0u;
+  for (uint32_t k = 0; k < ties; ++k) {
+    const uint32_t cand = o[2 + k], cv = cand >> kRunShift;
+    const Tri u = load_tri(m.tris, cand & kRunFirst);
+    if (cv != 3u && vertex != 3u && same_vertex(t, vertex, u, cv)) {
+      if (u.face < t.face) {
+        t = u;
+        vertex = cv;
+        c = closest_ff(p, t.a, t.b, t.c);
+      }
+      continue;
+    }
+    const CPFF d = closest_ff(p, u.a, u.b, u.c);
+    if (ff_lt(d.d2, c.d2) || (!ff_lt(c.d2, d.d2) && u.face < t.face)) {
+      t = u;
+      vertex = cv;
+      c = d;
+    }
+  }
+  r.face_index = t.face;
+  r.distance = ff_to_f(ff_sqrt(c.d2));
+  r.point[0] = ff_to_f(c.q.x);
+  r.point[1] = ff_to_f(c.q.y);
+  r.point[2] = ff_to_f(c.q.z);
+  out[i] = r;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1220,18 +1071,16 @@ __global__ void __launch_bounds__(kBlock) shape_key_kernel(const float* __restri
 }  // namespace dev
 
 cudaError_t launch_closest_point(const MeshDev& m, const float* pts, uint64_t n, float min_t, float max_t,
-                                 bvhc_closest* out, cudaStream_t stream, int variant, int occupancy, uint32_t* queue,
+                                 bvhc_closest* out, cudaStream_t stream, int variant, uint32_t* queue,
                                  unsigned int* qcount, const RaySort* sort, uint32_t tile, int tile_rows) {
   if (n == 0) return cudaSuccess;
-  // the warp-cooperative forms need minThreshold 0 (see closest_point_packet_kernel): 1 / 2 with
-  // whole warps, 3 / 4 with 16-lane groups, 5 / 6 with 8-lane groups; the even ones run over
-  // Morton-sorted queries
-  const bool sorted = variant > 0 && variant % 2 == 0;
+  const bool sorted = variant > 0 && variant % 2 == 0 && queue && qcount && sort && n < (1ull << 32);
   cudaError_t e;
-  if (variant == 0 || !(min_t <= 0.0f) || (sorted && (!queue || !qcount || !sort || n >= (1ull << 32)))) {
+  // minThreshold > 0 stops at the first triangle below it in the reference's order
+  if (!(min_t <= 0.0f) || n >= (1ull << 32) || !group_stack(m) || !m.boxes) {
     dev::closest_point_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, min_t, max_t, out);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    dev::closest_point_finalize_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, out);
+    dev::closest_point_finalize_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, out, false);
     return cudaGetLastError();
   }
   if (sorted) {
@@ -1250,24 +1099,12 @@ cudaError_t launch_closest_point(const MeshDev& m, const float* pts, uint64_t n,
     if ((e = launch_ray_sort(2, n, qcount, sort->scratch, queue, stream)) != cudaSuccess) return e;
   } else {
     queue = nullptr;
-    qcount = nullptr;
   }
-  using K = void (*)(MeshDev, const float*, uint64_t, float, bvhc_closest*, const uint32_t*, const unsigned int*,
-                     uint64_t, int);
-  static const K kernels[3][3] = {
-      {dev::closest_point_packet_kernel<1, 32>, dev::closest_point_packet_kernel<6, 32>,
-       dev::closest_point_packet_kernel<8, 32>},
-      {dev::closest_point_packet_kernel<1, 16>, dev::closest_point_packet_kernel<6, 16>,
-       dev::closest_point_packet_kernel<8, 16>},
-      {dev::closest_point_packet_kernel<1, 8>, dev::closest_point_packet_kernel<6, 8>,
-       dev::closest_point_packet_kernel<8, 8>}};
-  const K kernel = kernels[std::min((variant - 1) / 2, 2)][occupancy < 0 ? 0 : occupancy > 2 ? 2 : occupancy];
   // input order (odd variants) may be read in tiles: rows of `tile` points (a grid's row), 2-D blocks
   const int rl = tile_rows_log2(tile_rows);
-  const uint64_t pitch = (!queue && tile >= 8 && tile % (32u >> rl) == 0) ? (uint64_t)tile : 0;
-  kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, max_t, out, queue, qcount, pitch, rl);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  dev::closest_point_finalize_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, out);
+  const uint32_t pitch = (variant % 2 == 1 && tile >= 8 && tile % (32u >> rl) == 0) ? tile : 0;
+  if ((e = launch_closest_phased(m, pts, (uint32_t)n, max_t, out, queue, pitch, rl, stream)) != cudaSuccess) return e;
+  dev::closest_point_finalize_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, out, true);
   return cudaGetLastError();
 }
 

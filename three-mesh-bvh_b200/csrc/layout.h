@@ -45,12 +45,23 @@ struct alignas(32) QuadChild {
   float c[2], h[2];   // x, y
   float cz, hz;
   uint32_t link;      // internal child -> quad record index; else a run of triangle records (run_link)
-  uint32_t count;     // a part of a leaf: its triangle records; 0 for a node or a whole leaf of the tree
+  uint32_t count;     // a part of a leaf (or a root that is one): its triangle records, else 0
 };
 struct alignas(128) QuadNode {
   QuadChild c[4];
 };
 static_assert(sizeof(QuadNode) == 128, "QuadNode must be 128 bytes");
+
+// The same record for closestPointToPoint, whose maxThreshold is decided on the reference's exact
+// boxes: lo / hi bounds, an unused child at infinity.
+struct alignas(32) BoxChild {
+  float lo[3], hi[3];
+  uint32_t link, part;  // as QuadChild's link and count
+};
+struct alignas(128) BoxNode {
+  BoxChild c[4];
+};
+static_assert(sizeof(BoxNode) == 128, "BoxNode must be 128 bytes");
 
 constexpr float kBoxUnbounded = 3e38f;
 

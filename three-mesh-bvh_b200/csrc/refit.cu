@@ -84,17 +84,25 @@ __global__ void __launch_bounds__(kRefitBlock) refit_kernel(RefitPlan plan, Pair
 
 // Four-child records: a child's box is that of the child-pair slot it was collapsed from, or for a part
 // of a leaf (src kLeafBit | first record) the bounds of its triangles.  The unbounded child of a root
-// that is a leaf (src kEmptyLeaf) keeps its box.
+// that is a leaf (src kEmptyLeaf, link not) keeps its box.  `boxes` (nullable): the lo / hi form of the
+// same records, written whole.
 __global__ void __launch_bounds__(kRefitBlock) quad_boxes_kernel(QuadNode* __restrict__ quads, uint64_t n_quads,
                                                                  const uint32_t* __restrict__ src,
                                                                  const PairNode* __restrict__ pairs,
-                                                                 const TriRecord* __restrict__ tris) {
+                                                                 const TriRecord* __restrict__ tris,
+                                                                 BoxNode* __restrict__ boxes) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= 4 * n_quads) return;
   const uint32_t slot = __ldg(src + k);
   QuadChild& c = quads[k >> 2].c[k & 3u];
   float b[6];
-  if (slot == kEmptyLeaf) return;
+  if (slot == kEmptyLeaf) {
+    if (boxes) {
+      const float inf = __builtin_huge_valf(), lo = c.link == kEmptyLeaf ? inf : -inf;
+      boxes[k >> 2].c[k & 3u] = BoxChild{{lo, lo, lo}, {inf, inf, inf}, c.link, c.count};
+    }
+    return;
+  }
   if (!(slot & kLeafBit)) {
     const float* f = pairs[slot >> 1].f + 6 * (slot & 1u);
     for (int a = 0; a < 6; ++a) b[a] = f[a];
@@ -110,15 +118,16 @@ __global__ void __launch_bounds__(kRefitBlock) quad_boxes_kernel(QuadNode* __res
   box_centre_half(b[0], b[3], c.c[0], c.h[0]);
   box_centre_half(b[1], b[4], c.c[1], c.h[1]);
   box_centre_half(b[2], b[5], c.cz, c.hz);
+  if (boxes) boxes[k >> 2].c[k & 3u] = BoxChild{{b[0], b[1], b[2]}, {b[3], b[4], b[5]}, c.link, c.count};
 }
 
 }  // namespace dev
 
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
-                              const TriRecord* tris, cudaStream_t stream) {
+                              const TriRecord* tris, BoxNode* boxes, cudaStream_t stream) {
   if (n_quads == 0) return cudaSuccess;
   const unsigned int grid = (unsigned int)((4 * n_quads + dev::kRefitBlock - 1) / dev::kRefitBlock);
-  dev::quad_boxes_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(quads, n_quads, src, pairs, tris);
+  dev::quad_boxes_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(quads, n_quads, src, pairs, tris, boxes);
   return cudaGetLastError();
 }
 
