@@ -16,7 +16,7 @@ ROOT = PKG.parent
 LIB = PKG / "libbvhcuda.so"
 OBJ_DIR = PKG / "_build"
 CSRC = PKG / "csrc"
-SOURCES = [CSRC / n for n in ("api.cu", "kernels_first.cu", "kernels_packet.cu", "kernels_group.cu", "kernels_phased.cu", "kernels_closest.cu", "kernels_all.cu", "kernels_query.cu", "kernels_scene.cu",
+SOURCES = [CSRC / n for n in ("api.cu", "kernels_first.cu", "kernels_packet.cu", "kernels_group.cu", "kernels_phased.cu", "kernels_closest.cu", "kernels_wide.cu", "kernels_all.cu", "kernels_query.cu", "kernels_scene.cu",
                               "adjoint.cu", "noalloc.cu", "raysort.cu", "refit.cu", "gpubuild.cu", "autotune.cu",
                               "builder.cpp")]
 HEADERS = [ROOT / "include" / "bvhcuda.h"] + sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh"))

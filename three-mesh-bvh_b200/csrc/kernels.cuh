@@ -101,6 +101,10 @@ cudaError_t launch_raycast_first_persistent(const MeshDev& m, const BatchDev* ba
                                             bvhc_hit* out, unsigned long long* work, const TraversalConfig& cfg,
                                             cudaStream_t stream, uint32_t* queue = nullptr,
                                             unsigned int* qcount = nullptr, const RaySort* sort = nullptr);
+// The smallest batches: the whole warp on one ray, complete records (group_stack(m) > 0).
+cudaError_t launch_raycast_first_wide(const MeshDev& m, const BatchDev* batch, const float* rays, uint64_t n, int side,
+                                      const SideTable& sides, float near_d, float far_d, bvhc_hit* out,
+                                      cudaStream_t stream, const uint32_t* queue, const unsigned int* qcount);
 // Its traversals over the four-child records (no finalize): four lanes per ray (group_stack(m) > 0) and
 // one (phased_stack(m), n < 2^32).  `work` is reset here when it is used.
 cudaError_t launch_raycast_first_group(const MeshDev& m, const BatchDev* batch, const float* rays, uint64_t n, int side,

@@ -1,4 +1,5 @@
-// closestPointToPoint with minThreshold 0: four lanes per query over the four-child records, and the 32
+// closestPointToPoint with minThreshold 0: four lanes per query (the smaller batches take whole warps,
+// kernels_wide.cu) over the four-child records, and the 32
 // queries of a warp through one shared traversal; and their launches.
 #include <algorithm>
 #include <cfloat>
@@ -9,150 +10,9 @@
 namespace bvhc {
 namespace dev {
 
-constexpr uint32_t kNoRecord = 0xFFFFFFFFu;
-
-// Float32 closest point of a triangle: closest_sq_f's regions (Ericson, Real-Time Collision Detection,
-// 5.1.5) as selections of two numerators over one denominator, l = ab v + ac w, and one reciprocal:
-// the lanes of a warp are at different triangles, and would walk the regions' branches, and their
-// divisions, one after the other.
-struct Candidate {
-  float d2, err;
-  float3 q;
-};
-__device__ __forceinline__ Candidate candidate(float3 p, const Tri& t) {
-  const float abx = t.b.x - t.a.x, aby = t.b.y - t.a.y, abz = t.b.z - t.a.z;
-  const float acx = t.c.x - t.a.x, acy = t.c.y - t.a.y, acz = t.c.z - t.a.z;
-  const float apx = p.x - t.a.x, apy = p.y - t.a.y, apz = p.z - t.a.z;
-  const float sc = max3(fabsf(abx), fabsf(aby), fabsf(abz)) + max3(fabsf(acx), fabsf(acy), fabsf(acz)) +
-                   max3(fabsf(apx), fabsf(apy), fabsf(apz));
-  const float d1 = abx * apx + aby * apy + abz * apz;
-  const float d2 = acx * apx + acy * apy + acz * apz;
-  const float bpx = apx - abx, bpy = apy - aby, bpz = apz - abz;
-  const float d3 = abx * bpx + aby * bpy + abz * bpz;
-  const float d4 = acx * bpx + acy * bpy + acz * bpz;
-  const float cpx = apx - acx, cpy = apy - acy, cpz = apz - acz;
-  const float d5 = abx * cpx + aby * cpy + abz * cpz;
-  const float d6 = acx * cpx + acy * cpy + acz * cpz;
-  const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
-  const float e43 = d4 - d3, e56 = d5 - d6;
-  // the first region that holds wins, so they are taken last to first
-  float nv = vb, nw = vc, den = va + vb + vc;
-  const bool bc = va <= 0.0f && e43 >= 0.0f && e56 >= 0.0f;
-  den = bc ? e43 + e56 : den;
-  nv = bc ? e56 : nv;
-  nw = bc ? e43 : nw;
-  const bool ac = vb <= 0.0f && d2 >= 0.0f && d6 <= 0.0f;
-  den = ac ? d2 - d6 : den;
-  nv = ac ? 0.0f : nv;
-  nw = ac ? d2 : nw;
-  const bool at_c = d6 >= 0.0f && d5 <= d6;
-  den = at_c ? 1.0f : den;
-  nv = at_c ? 0.0f : nv;
-  nw = at_c ? 1.0f : nw;
-  const bool ab = vc <= 0.0f && d1 >= 0.0f && d3 <= 0.0f;
-  den = ab ? d1 - d3 : den;
-  nv = ab ? d1 : nv;
-  nw = ab ? 0.0f : nw;
-  const bool at_b = d3 >= 0.0f && d4 <= d3, at_a = d1 <= 0.0f && d2 <= 0.0f;
-  den = at_a || at_b ? 1.0f : den;
-  nv = at_a ? 0.0f : at_b ? 1.0f : nv;
-  nw = at_a || at_b ? 0.0f : nw;
-  const float rd = rcp_fast(den), v = nv * rd, w = nw * rd;
-  const float lx = abx * v + acx * w, ly = aby * v + acy * w, lz = abz * v + acz * w;
-  const float rx = apx - lx, ry = apy - ly, rz = apz - lz;
-  Candidate c;
-  c.d2 = rx * rx + ry * ry + rz * rz;
-  const float e = 32.0f * kU * sc;  // |error| of each closest-point coordinate (local-frame evaluation)
-  float root;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(c.d2));
-  c.err = 3.501f * e * root + 3.0f * e * e;
-  const bool vb_ = !at_a && at_b, vc_ = !at_a && !at_b && !ab && at_c;
-  c.q.x = vb_ ? t.b.x : vc_ ? t.c.x : t.a.x + lx;
-  c.q.y = vb_ ? t.b.y : vc_ ? t.c.y : t.a.y + ly;
-  c.q.z = vb_ ? t.b.z : vc_ ? t.c.z : t.a.z + lz;
-  return c;
-}
-
-// Which vertex of the triangle q is, bit for bit (3: none).
-__device__ __forceinline__ uint32_t vertex_of(const Tri& t, float3 q) {
-  return q.x == t.a.x && q.y == t.a.y && q.z == t.a.z   ? 0u
-         : q.x == t.b.x && q.y == t.b.y && q.z == t.b.z ? 1u
-         : q.x == t.c.x && q.y == t.c.y && q.z == t.c.z ? 2u
-                                                        : 3u;
-}
-
-// A lane's best candidate: float32 squared distance and its error bound, the triangle record with its
-// vertex above kRunShift, its faceIndex and the float32 closest point; and the candidates that float32
-// cannot tell from it (`ties` of them, in the lane's column of a shared array).
-struct Nearest {
-  float d2, err;
-  uint32_t rec, face;
-  float3 q;
-  int ties;
-};
-__device__ __forceinline__ Nearest nearest_none() {
-  return {kInf, 0.0f, kNoRecord, 0u, make_float3(0.f, 0.f, 0.f), 0};
-}
-
-// Whether candidate `cand` beats `b` where their float32 distances do not tell: the same vertex is an
-// exact tie, else the float-float distances decide; an exact tie goes to the smaller faceIndex.
-static __device__ __noinline__ bool closer_slow(const TriRecord* __restrict__ tris, float3 p, uint32_t cand,
-                                                uint32_t b) {
-  const Tri t = load_tri(tris, cand & kRunFirst), u = load_tri(tris, b & kRunFirst);
-  const uint32_t tv = cand >> kRunShift, uv = b >> kRunShift;
-  if (tv != 3u && uv != 3u && same_vertex(t, tv, u, uv)) return t.face < u.face;
-  const ff d = closest_ff(p, t.a, t.b, t.c).d2, e = closest_ff(p, u.a, u.b, u.c).d2;
-  return ff_lt(d, e) || (!ff_lt(e, d) && t.face < u.face);
-}
-
-// Offers triangle t (record k) at candidate c to a lane's best.  Candidates are ranked by exact distance,
-// then by faceIndex, a total order that does not depend on the order of the offers.  What float32 and
-// the shared vertex do not settle is kept beside the best one for the finalize kernel: most of it is
-// overtaken by a nearer triangle later in the walk, and float-float code in the loop is fetched and
-// executed by whole warps for one lane.
-__device__ __forceinline__ void offer_closest(const TriRecord* __restrict__ tris, float3 p, const Tri& t, uint32_t k,
-                                              const Candidate& c, Nearest& b, uint2 (*s_tie)[kBlock]) {
-  const float hi = c.d2 + c.err, lo = c.d2 - c.err;
-  bool take = b.rec == kNoRecord ? c.d2 < kInf : hi < b.d2 - b.err;
-  uint32_t rec = kNoRecord;
-  if (!take && b.rec != kNoRecord && !(lo > b.d2 + b.err)) {
-    rec = k | vertex_of(t, c.q) << kRunShift;
-    if ((rec >> kRunShift) != 3u && (b.rec >> kRunShift) != 3u && c.q.x == b.q.x && c.q.y == b.q.y && c.q.z == b.q.z) {
-      take = t.face < b.face;  // the same vertex: an exact tie, the smaller faceIndex wins
-    } else if (b.ties < kClosestTies) {
-      take = c.d2 < b.d2;
-      s_tie[b.ties][threadIdx.x] = take ? make_uint2(b.rec, __float_as_uint(b.d2 - b.err))
-                                        : make_uint2(rec, __float_as_uint(lo));
-      ++b.ties;
-    } else {
-      take = closer_slow(tris, p, rec, b.rec);
-    }
-  }
-  if (take) {
-    b.d2 = c.d2;
-    b.err = c.err;
-    b.rec = rec != kNoRecord ? rec : k | vertex_of(t, c.q) << kRunShift;
-    b.face = t.face;
-    b.q = c.q;
-    int kept = 0;  // ties that the new best candidate leaves behind for certain are dropped
-    for (int j = 0; j < b.ties; ++j) {
-      const uint2 e = s_tie[j][threadIdx.x];
-      if (!(__uint_as_float(e.y) > hi)) s_tie[kept++][threadIdx.x] = e;
-    }
-    b.ties = kept;
-  }
-}
-
-// The box of a record's child against maxThreshold^2, exactly.
-static __device__ __noinline__ bool under_max_slow(const BoxChild* c, float3 p, ff max2) {
-  const float b[6] = {c->lo[0], c->lo[1], c->lo[2], c->hi[0], c->hi[1], c->hi[2]};
-  return ff_lt(box_score_ff(b, p), max2);
-}
-
 constexpr int kClosestBlocksPerSm = 8;
 constexpr int kClosestRefill = 2 * kGroup;  // idle lanes at which a warp takes new queries
 
-template <bool MAXED>
 __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_group_kernel(
     MeshDev m, const float* __restrict__ pts, uint32_t n, float max_t, bvhc_closest* __restrict__ out,
     const uint32_t* __restrict__ queue, uint32_t pitch, int rows_log2, int cap) {
@@ -162,23 +22,17 @@ __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_gro
   const unsigned lane = threadIdx.x & 31u, j = lane & 3u, base = lane & ~3u;
   const unsigned below = 0x11111111u & ((1u << base) - 1u);  // first lanes of the groups before this one
   uint2* stack = s_stack + (threadIdx.x / kGroup) * (cap + 1);
-  const ff max2 = two_prod(max_t, max_t);
-  // box distances outside [max_lo, max_hi) are decided by their float32 value (see under_max)
-  const float max_lo = max2.hi * (1.0f - kSlabMargin) * (1.0f - 0x1p-19f), max_hi = max2.hi * (1.0f + 0x1p-18f);
+  const MaxThreshold mx = max_threshold(max_t);
   bool active = false, pending = false, dead = false;  // group-uniform, as in raycast_first_group_kernel
   uint32_t qid = 0, link = 0;
   float3 p = make_float3(0.f, 0.f, 0.f);
   float bound = 0.0f;  // boxes beyond it cannot hold a candidate
   Nearest best = nearest_none();
   int sp = 0, root = 0;
-  // this warp's chunks of 32 queries: every (warps of the grid)-th one
+  // this warp's chunks of 32 queries: every (warps of the grid)-th one (no work counter, which calls on
+  // different streams would share)
   const uint32_t warps = gridDim.x * (kBlock / 32), chunks = (n + 31u) / 32u;
   uint32_t chunk = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), pool = 0, pool_end = 0;
-  if (chunks <= warps / 4) {  // few queries: eight, one per group, for each warp
-    pool = min(chunk * kGroups, n);
-    pool_end = min(pool + kGroups, n);
-    chunk = chunks;
-  }
   auto next_root = [&]() {
     sp = 0;
     dead = false;
@@ -193,62 +47,7 @@ __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_gro
     const unsigned idle = __ballot_sync(full, !active);
     if (idle == full || (__popc(idle) >= kClosestRefill && (chunk < chunks || pool < pool_end))) {
       if (__ballot_sync(full, pending)) {
-        // the four lanes' candidates to one and what is not settled against it
-        const int key = best.rec == kNoRecord ? 0x7FFFFFFF : (int)((__float_as_uint(best.d2) & ~3u) | j);
-        int rank;
-        unsigned first;
-        group_rank(key, rank, first);
-        const unsigned src = base + first;
-        const float hi = __shfl_sync(full, best.d2 + best.err, src);
-        uint32_t rec = __shfl_sync(full, best.rec, src);
-        const uint32_t face = __shfl_sync(full, best.face, src);
-        const float qx = __shfl_sync(full, best.q.x, src), qy = __shfl_sync(full, best.q.y, src),
-                    qz = __shfl_sync(full, best.q.z, src);
-        bool extra = lane != src && best.rec != kNoRecord && !(best.d2 - best.err > hi);
-        const bool same = extra && (rec >> kRunShift) != 3u && (best.rec >> kRunShift) != 3u && best.q.x == qx &&
-                          best.q.y == qy && best.q.z == qz;
-        extra = extra && !same;
-        // of the lanes at the same vertex the smallest faceIndex
-        uint32_t f = same || lane == src ? best.face : 0xFFFFFFFFu;
-        f = min(f, __shfl_xor_sync(full, f, 1));
-        f = min(f, __shfl_xor_sync(full, f, 2));
-        const unsigned winner = (__ballot_sync(full, (same || lane == src) && best.face == f) >> base) & 0xFu;
-        rec = __shfl_sync(full, best.rec, base + (f != face && winner ? (unsigned)__ffs(winner) - 1u : first));
-        int mine = extra ? 1 : 0;
-        for (int k = 0; k < best.ties; ++k) mine += !(__uint_as_float(s_tie[k][threadIdx.x].y) > hi);
-        if (!pending || best.rec == kNoRecord) mine = 0;
-        const int a1 = __shfl_xor_sync(full, mine, 1), pair = mine + a1, other = __shfl_xor_sync(full, pair, 2);
-        const int total = pair + other;
-        int at = ((j & 1u) ? a1 : 0) + ((j & 2u) ? other : 0);
-        if (__ballot_sync(full, pending && total > kClosestTies)) {
-          // more than the record holds: settled here
-          const bool over = pending && total > kClosestTies;
-          uint32_t mine_rec = best.rec;
-          if (over && mine_rec != kNoRecord)
-            for (int k = 0; k < best.ties; ++k)
-              if (closer_slow(m.tris, p, s_tie[k][threadIdx.x].x, mine_rec)) mine_rec = s_tie[k][threadIdx.x].x;
-#pragma unroll
-          for (int x = 1; x <= 2; x <<= 1) {
-            const uint32_t o = __shfl_xor_sync(full, mine_rec, x);
-            if (over && o != kNoRecord && (mine_rec == kNoRecord || closer_slow(m.tris, p, o, mine_rec))) mine_rec = o;
-          }
-          if (over) {
-            rec = mine_rec;
-            mine = 0;
-          }
-        }
-        if (pending) {  // closest_point_finalize_kernel completes it
-          uint32_t* o = reinterpret_cast<uint32_t*>(out + qid);
-          if (j == 0) {
-            o[0] = rec;
-            o[1] = total > kClosestTies ? 0u : (uint32_t)total;
-          }
-          if (mine) {
-            if (extra) o[2 + at++] = best.rec;
-            for (int k = 0; k < best.ties; ++k)
-              if (!(__uint_as_float(s_tie[k][threadIdx.x].y) > hi)) o[2 + at++] = s_tie[k][threadIdx.x].x;
-          }
-        }
+        store_merged<kGroup>(m.tris, p, best, pending, reinterpret_cast<uint32_t*>(out + qid), s_tie);
         pending = false;
       }
       const unsigned want = __popc(idle) / kGroup;
@@ -295,14 +94,7 @@ __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_gro
         }
         if (!dead) {
           const BoxChild* c = m.boxes[link].c + j;
-          float4 a, b;
-          ld8(c, a, b);
-          l = __float_as_uint(b.z);
-          const float dx = max3(a.x - p.x, p.x - a.w, 0.0f), dy = max3(a.y - p.y, p.y - b.x, 0.0f),
-                      dz = max3(a.z - p.z, p.z - b.y, 0.0f);
-          s = dx * dx + dy * dy + dz * dz;
-          w = s <= bound;
-          if (MAXED && w && !(s < max_lo) && __float_as_uint(b.w) == 0u) w = s < max_hi && under_max_slow(c, p, max2);
+          w = box_wanted(c, p, bound, mx, s, l);
         }
       }
       const unsigned hits = (__ballot_sync(full, w) >> base) & 0xFu, oks = (__ballot_sync(full, ok) >> base) & 0xFu;
@@ -500,12 +292,11 @@ cudaError_t launch_closest_phased(const MeshDev& m, const float* pts, uint32_t n
     return cudaGetLastError();
   }
   const int cap = group_stack(m);
-  const bool maxed = !(max_t >= dev::kInf);
-  auto kernel = maxed ? dev::closest_point_group_kernel<true> : dev::closest_point_group_kernel<false>;
+  if (n <= kWideMaxQueries) return launch_closest_wide(m, pts, n, max_t, out, stream);
   const unsigned int resident = (unsigned int)sm_count() * dev::kClosestBlocksPerSm;
   const unsigned int blocks = (n + dev::kBlockGroups - 1) / dev::kBlockGroups;
-  kernel<<<std::min(blocks, resident), dev::kBlock, group_smem(cap), stream>>>(m, pts, n, max_t, out, queue, pitch,
-                                                                              rows_log2, cap);
+  dev::closest_point_group_kernel<<<std::min(blocks, resident), dev::kBlock, group_smem(cap), stream>>>(
+      m, pts, n, max_t, out, queue, pitch, rows_log2, cap);
   return cudaGetLastError();
 }
 

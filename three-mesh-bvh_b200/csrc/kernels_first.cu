@@ -369,6 +369,8 @@ cudaError_t launch_raycast_first_persistent(const MeshDev& m, const BatchDev* ba
     queue = nullptr;
     qcount = nullptr;
   }
+  if (n <= kWideMaxRays && group_stack(m))
+    return launch_raycast_first_wide(m, batch, rays, n, side, sides, near_d, far_d, out, stream, queue, qcount);
   if (n <= kGroupMaxRays && group_stack(m)) {
     e = launch_raycast_first_group(m, batch, rays, n, side, sides, near_d, far_d, out, work, stream, queue, qcount);
   } else if (n < (1ull << 32) && phased_stack(m)) {

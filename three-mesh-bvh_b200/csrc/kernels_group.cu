@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kBlock, kGroupBlocksPerSm) raycast_first_group
         const RayF r = make_ray(rays, rid);
         rg = ray_slab(r);
         best = Best{kInf, 0.0f, 0xFFFFFFFFu};
-        lim = RANGED ? slab_limit(far_d) : kInf;
+        lim = RANGED ? slab_far(far_d) : kInf;
         lim_hit = kInf;
         odd = RANGED && odd_length(r.d);
         int root_end = m.n_roots;

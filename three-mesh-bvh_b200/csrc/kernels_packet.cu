@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
           ck[c] = ch[c].link;
         }
         const float lim_hit = slab_limit((best.t + best.err) * (1.0f + kSlabMargin));
-        const float lim = fminf(slab_limit(far_d), lim_hit);
+        const float lim = fminf(slab_far(far_d), lim_hit);
         float e[4];
         bool h[4];
         unsigned b[4];

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kBlock, kPhasedBlocksPerSm) raycast_first_phas
         rs = ray_slab(r);
         dlen = sqrtf(r.d.x * r.d.x + r.d.y * r.d.y + r.d.z * r.d.z);
         best = Best{kInf, 0.0f, 0xFFFFFFFFu};
-        lim = RANGED ? slab_limit(far_d) : kInf;
+        lim = RANGED ? slab_far(far_d) : kInf;
         lim_hit = kInf;
         odd = RANGED && odd_length(r.d);
         root = 0;

@@ -146,6 +146,7 @@ __device__ __forceinline__ RaySlab ray_slab(const RayF& r) {
 // near.  Every hit has t >= 0, so a negative near acts as 0; with a NaN near nothing is entered.
 __device__ __forceinline__ float slab_near(float near_d) { return near_d <= 0.0f ? 0.0f : near_d * (1.0f - 0x1p-19f); }
 __device__ __forceinline__ float slab_limit(float lim) { return lim * (1.0f + 0x1p-19f); }
+__device__ __forceinline__ float slab_far(float far_d) { return far_d < kInf ? slab_limit(far_d) : kInf; }  // NaN: none
 
 // near and far are distances, and the reference holds them against the ray parameter of its nodes'
 // boxes: for a direction that is not of unit length that drops hits by the extent of their leaf's box.
@@ -467,12 +468,13 @@ static inline int group_stack(const MeshDev& m) {
   return m.quads && m.quad_roots && m.quad_stack <= kMaxGroupStack ? (m.quad_stack < 1 ? 1 : m.quad_stack) : 0;
 }
 
-// Calls of up to this many rays take four lanes per ray, larger ones one lane.  With few rays the
-// longest ray's chain of dependent steps is the time, and four lanes make each step shorter; with many,
-// the chip is full and the lanes' own work counts.  Measured (box / sphere rays on the 10,000-,
-// 80,000- and 2M-triangle knots): 4,097 rays 50 / 64 / 87 us against 110 / 157 / 190 in one lane, 100,000
-// rays about even, 250,000 rays 246 / 294 / 403 against 195 / 254 / 458; between them the two cross.
-constexpr uint64_t kGroupMaxRays = 131072;
+// Calls of up to kWideMaxRays rays take the whole warp for each ray, of up to kGroupMaxRays four lanes,
+// larger ones one lane.  With few rays the longest ray's chain of dependent steps is the time, and more
+// lanes make the chain shorter; with many, the chip is full and the lanes' own work counts.  Measured on
+// the 80,000-triangle knot, rays towards its box: 4,097 rays 24 us by warps (four lanes: 62, one lane 157),
+// 16,000 rays 65 (95), 32,000 rays 118 (110); 100,000 rays 188 by fours (one lane: 200), 250,000 rays 294
+// (254).  Incoherent rays, which mostly miss, cross later.
+constexpr uint64_t kWideMaxRays = 24576, kGroupMaxRays = 131072;
 
 // Root-box pre-pass into `queue`, then (single mesh, sort requested) the ray-ordering sort
 // (kernels_first.cu).
