@@ -109,6 +109,8 @@ struct bvhc_mesh {
     uint32_t* src = nullptr;  // where each child's box comes from (QuadBuilder::src)
     uint64_t n = 0;
     int stack = 0;
+    RayPair* ray_pairs = nullptr;  // the child pairs themselves in the ray traversals' form
+    uint64_t n_pairs = 0;
   };
   QuadSet quad_set[2];
 
@@ -130,6 +132,7 @@ struct bvhc_mesh {
 
  private:
   static void set_quads(MeshDev& v, const QuadSet& q) {
+    v.ray_pairs = q.ray_pairs;
     v.quads = q.quads;
     v.boxes = q.boxes;
     v.quad_roots = q.roots;
@@ -746,15 +749,26 @@ static void free_quads(bvhc_mesh::QuadSet& q) {
   cudaFree(q.boxes);
   cudaFree(q.roots);
   cudaFree(q.src);
+  cudaFree(q.ray_pairs);
   q = bvhc_mesh::QuadSet{};
 }
 
-// Four-child records over a child-pair layout, into set `k`, replacing any before.  A mesh with more
-// triangle records than a run link can name has none: the child-pair kernels run.
+// The ray traversals' records over a child-pair layout (already on the device), into set `k`, replacing
+// any before.  A mesh with more triangle records than a run link can name has no four-child records:
+// the child-pair kernels run.
 static cudaError_t install_quads(bvhc_mesh* m, int k, const std::vector<PairNode>& pairs,
                                  const std::vector<TriRecord>& tris, const std::vector<uint32_t>& roots) {
   free_quads(m->quad_set[k]);
-  if (tris.size() >= kRunFirst) return cudaSuccess;
+  bvhc_mesh::QuadSet q;
+  q.n_pairs = pairs.size();
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&q.ray_pairs), std::max<size_t>(pairs.size(), 1) * sizeof(RayPair));
+  if (e == cudaSuccess) e = launch_ray_pairs(k ? m->d_nodes_f : m->d_nodes, q.n_pairs, q.ray_pairs, nullptr);
+  if (e != cudaSuccess) {
+    free_quads(q);
+    return e;
+  }
+  m->quad_set[k] = q;
+  if (tris.size() >= kRunFirst) return cudaStreamSynchronize(nullptr);
   QuadBuilder qb{pairs, tris};
   std::vector<uint32_t> qroots(roots.size());
   try {
@@ -766,8 +780,7 @@ static cudaError_t install_quads(bvhc_mesh* m, int k, const std::vector<PairNode
   } catch (const std::bad_alloc&) {
     return cudaErrorMemoryAllocation;
   }
-  bvhc_mesh::QuadSet q;
-  cudaError_t e = upload(&q.quads, qb.quads);
+  e = upload(&q.quads, qb.quads);
   if (e == cudaSuccess) e = upload(&q.roots, qroots);
   if (e == cudaSuccess) e = upload(&q.src, qb.src);
   q.n = qb.quads.size();
@@ -775,13 +788,13 @@ static cudaError_t install_quads(bvhc_mesh* m, int k, const std::vector<PairNode
   if (k == 0) {
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&q.boxes), q.n * sizeof(BoxNode));
     if (e == cudaSuccess) e = launch_quad_boxes(q.quads, q.n, q.src, m->d_nodes, m->d_tris, q.boxes, nullptr);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  m->quad_set[k] = q;
   if (e != cudaSuccess) {
-    free_quads(q);
+    free_quads(m->quad_set[k]);
     return e;
   }
-  m->quad_set[k] = q;
   return cudaSuccess;
 }
 
@@ -1372,6 +1385,7 @@ bvhc_status bvhc_mesh_refit(bvhc_mesh* m, const float* positions, uint64_t n_ver
     BVHC_CUDA_TRY(launch_refit(m->refit[1], m->d_nodes_f, m->d_tris_f, m->d_tri_vid, pos, stride_floats, true, s));
   for (int k = 0; k < 2; ++k) {  // the four-child records follow their child pairs
     const bvhc_mesh::QuadSet& q = m->quad_set[k];
+    if (q.ray_pairs) BVHC_CUDA_TRY(launch_ray_pairs(k ? m->d_nodes_f : m->d_nodes, q.n_pairs, q.ray_pairs, s));
     if (q.quads)
       BVHC_CUDA_TRY(launch_quad_boxes(q.quads, q.n, q.src, k ? m->d_nodes_f : m->d_nodes, k ? m->d_tris_f : m->d_tris,
                                       q.boxes, s));

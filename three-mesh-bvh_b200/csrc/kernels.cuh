@@ -22,6 +22,7 @@ struct MeshDev {
   const uint32_t* roots;  // one link per root
   int n_roots;
   unsigned int* err;
+  const RayPair* ray_pairs = nullptr;  // `nodes` with centre / half-extent boxes
   const QuadNode* quads = nullptr;     // four-child copy of `nodes` (same triangle records), if any
   const uint32_t* quad_roots = nullptr;
   const BoxNode* boxes = nullptr;      // the same records with lo / hi bounds (the reference's leaves only)
@@ -252,6 +253,9 @@ cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris
 // (nullable) gets the same records with lo / hi bounds.
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
                               const TriRecord* tris, BoxNode* boxes, cudaStream_t stream);
+
+// `nodes` as RayPairs.
+cudaError_t launch_ray_pairs(const PairNode* pairs, uint64_t n, RayPair* out, cudaStream_t stream);
 
 // What another translation unit needs to launch on a mesh: its device view, traversal variant and
 // device ordinal (defined in api.cu).  Returns false for a null mesh.

@@ -252,6 +252,8 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_all_packet_kernel(
   uint32_t cnt = 0;
   bvhc_hit* out = hits + i * (uint64_t)cap;
   bool overflow = false;
+  const RaySlab rs = ray_slab(r);
+  const float near_s = slab_near(near_d), lim = valid ? slab_far(far_d) : -kInf;  // no ray: enters nothing
   for (int root = 0; root < m.n_roots && !overflow; ++root) {
     uint32_t link = m.roots[root];
     int sp = 0;
@@ -271,10 +273,10 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_all_packet_kernel(
         }
         pop = true;
       } else {
-        Pair p = load_pair(m.nodes, link);
+        const RayPair* rp = m.ray_pairs + link;
+        const ChildBox c0 = load_child(rp->c), c1 = load_child(rp->c + 1);
         float e0, e1;
-        bool h0 = valid && box_hit(p.l[0], p.l[1], p.l[2], p.l[3], p.l[4], p.l[5], r, near_d, far_d, e0);
-        bool h1 = valid && box_hit(p.r[0], p.r[1], p.r[2], p.r[3], p.r[4], p.r[5], r, near_d, far_d, e1);
+        const bool h0 = child_hit(c0, rs, near_s, lim, e0), h1 = child_hit(c1, rs, near_s, lim, e1);
         unsigned b0 = __ballot_sync(full, h0), b1 = __ballot_sync(full, h1);
         if (b0 && b1) {
           if (sp >= kMaxStack) {
@@ -282,14 +284,14 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_all_packet_kernel(
             overflow = true;
             break;
           }
-          if (lane == 0) s_link[w][sp] = p.lr;
+          if (lane == 0) s_link[w][sp] = c1.link;
           ++sp;
-          link = p.ll;
+          link = c0.link;
           __syncwarp();
         } else if (b0) {
-          link = p.ll;
+          link = c0.link;
         } else if (b1) {
-          link = p.lr;
+          link = c1.link;
         } else {
           pop = true;
         }

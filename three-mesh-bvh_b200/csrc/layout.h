@@ -52,7 +52,14 @@ struct alignas(128) QuadNode {
 };
 static_assert(sizeof(QuadNode) == 128, "QuadNode must be 128 bytes");
 
-// The same record for closestPointToPoint, whose maxThreshold is decided on the reference's exact
+// A child pair in the same form, for the warp-shared ray traversals: the two children of a PairNode and,
+// in c[0].count, its split axis (an empty leaf's box is NaN).
+struct alignas(64) RayPair {
+  QuadChild c[2];
+};
+static_assert(sizeof(RayPair) == 64, "RayPair must be 64 bytes");
+
+// The four-child record for closestPointToPoint, whose maxThreshold is decided on the reference's exact
 // boxes: lo / hi bounds, an unused child at infinity.
 struct alignas(32) BoxChild {
   float lo[3], hi[3];

@@ -121,7 +121,32 @@ __global__ void __launch_bounds__(kRefitBlock) quad_boxes_kernel(QuadNode* __res
   if (boxes) boxes[k >> 2].c[k & 3u] = BoxChild{{b[0], b[1], b[2]}, {b[3], b[4], b[5]}, c.link, c.count};
 }
 
+// Child pairs as the warp-shared ray traversals read them.
+__global__ void __launch_bounds__(kRefitBlock) ray_pairs_kernel(const PairNode* __restrict__ pairs, uint64_t n,
+                                                                RayPair* __restrict__ out) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= 2 * n) return;
+  const PairNode& p = pairs[k >> 1];
+  const int s = (int)(k & 1u);
+  const float* b = p.f + 6 * s;
+  QuadChild c;
+  box_centre_half(b[0], b[3], c.c[0], c.h[0]);
+  box_centre_half(b[1], b[4], c.c[1], c.h[1]);
+  box_centre_half(b[2], b[5], c.cz, c.hz);
+  c.link = p.link[s];
+  c.count = s == 0 ? p.axis : 0u;
+  if (c.link == kEmptyLeaf) c.c[0] = c.c[1] = c.cz = __int_as_float(0x7FFFFFFF);
+  out[k >> 1].c[s] = c;
+}
+
 }  // namespace dev
+
+cudaError_t launch_ray_pairs(const PairNode* pairs, uint64_t n, RayPair* out, cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  dev::ray_pairs_kernel<<<(unsigned int)((2 * n + dev::kRefitBlock - 1) / dev::kRefitBlock), dev::kRefitBlock, 0, stream>>>(
+      pairs, n, out);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
                               const TriRecord* tris, BoxNode* boxes, cudaStream_t stream) {
