@@ -107,3 +107,41 @@ def test_closest_matches_the_per_query_kernel(pkg, cuda, mesh, n):
             got = bvh.closest_point_batch(d, 0.0, far)
             bvh.synchronize()
             assert torch.equal(got.view(torch.int32), want), (far, kw)
+
+
+@pytest.mark.parametrize("mesh", ["triangle", "leaf40", "leaves40", "groups", "plain"])
+@pytest.mark.parametrize("n", [1, 5, 33, 32768, 32769, 65537])
+def test_shapes_match(pkg, orc, cuda, mesh, n):
+    """Any-hit spheres and oriented boxes, the whole warp and four lanes per shape: spheres as the
+    per-sphere child-pair walk counts them, boxes as the oracle answers, with boxes that rest on the
+    mesh's vertices (undecided in float32) among them."""
+    import torch
+
+    g, opts = _mesh(pkg, mesh)
+    bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH, **opts})
+    ref = orc.OracleBVH.from_serialized(bvh._roots, g.index, bvh._indirectBuffer, g.position)
+    rng = np.random.default_rng(n)
+    lo, hi = g.position.min(0) - 1, g.position.max(0) + 1
+    c = (lo + rng.random((n, 3)) * (hi - lo)).astype(np.float32)
+    corner = g.position[g.index[rng.integers(0, len(g.index), n)]]
+    spheres = np.concatenate([c, np.exp(rng.uniform(-4, 1, (n, 1)))], 1).astype(np.float32)
+    spheres[::9, 3] = 0.0
+    spheres[::9, :3] = corner[::9]
+    half = (rng.random((n, 3)) * 0.9 + 0.05).astype(np.float32)
+    boxes = np.zeros((n, 24), np.float32)
+    boxes[:, 0:3], boxes[:, 4:7] = -half, half
+    boxes[:, 8] = boxes[:, 13] = boxes[:, 18] = boxes[:, 23] = 1.0
+    a = rng.uniform(0, 6, n)
+    boxes[::2, 8], boxes[::2, 9], boxes[::2, 12], boxes[::2, 13] = (v[::2] for v in (
+        np.cos(a), np.sin(a), -np.sin(a), np.cos(a)))
+    boxes[:, 20:23] = c
+    rest = np.arange(n) % 3 == 1          # one face through a vertex of the mesh, exactly or nearly
+    boxes[rest, 20:23] = corner[rest]
+    boxes[rest, 20] += half[rest, 0] * np.float32(1 + 1e-7)
+    boxes[::11, 19] = 0.01                # projective
+    want_s, want_b = bvh.sphere_triangles_batch(spheres, cap=1)[0] > 0, ref.intersects_box(boxes)
+    got_s = bvh.intersects_sphere_batch(torch.from_numpy(spheres).to(cuda)).cpu().numpy().astype(bool)
+    got_b = bvh.intersects_box_batch(torch.from_numpy(boxes).to(cuda)).cpu().numpy().astype(bool)
+    bvh.synchronize()
+    assert np.array_equal(got_s, want_s)
+    assert np.array_equal(got_b, want_b)

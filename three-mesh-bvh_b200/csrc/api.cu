@@ -1748,10 +1748,10 @@ bvhc_status bvhc_intersects_sphere(bvhc_mesh* m, const float* spheres, uint64_t 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BVHC_CUDA_TRY(cudaSetDevice(m->device));
   if (mem == BVHC_MEM_DEVICE && !aligned(spheres, 16)) return BVHC_ERR_INVALID_ARGUMENT;
-  uint32_t* q;
-  unsigned int* qc;
+  uint32_t* q = nullptr;
+  unsigned int* qc = nullptr;
   RaySort sort{};
-  BVHC_CUDA_TRY(shape_order(m, n, &q, &qc, &sort));
+  if (!shapes_by_group(m->view(), n)) BVHC_CUDA_TRY(shape_order(m, n, &q, &qc, &sort));
   if (mem == BVHC_MEM_DEVICE) return from_cuda(launch_intersects_sphere(m->view(), spheres, n, out, s, q, qc, &sort));
   BVHC_CUDA_TRY(ensure(&m->d_in, &m->in_cap, n * 16));
   BVHC_CUDA_TRY(ensure(&m->d_out, &m->out_cap, n));
@@ -1769,10 +1769,10 @@ bvhc_status bvhc_intersects_box(bvhc_mesh* m, const float* boxes, uint64_t n, ui
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BVHC_CUDA_TRY(cudaSetDevice(m->device));
   if (mem == BVHC_MEM_DEVICE && !aligned(boxes, 16)) return BVHC_ERR_INVALID_ARGUMENT;
-  uint32_t* q;
-  unsigned int* qc;
+  uint32_t* q = nullptr;
+  unsigned int* qc = nullptr;
   RaySort sort{};
-  BVHC_CUDA_TRY(shape_order(m, n, &q, &qc, &sort));
+  if (!shapes_by_group(m->view(), n)) BVHC_CUDA_TRY(shape_order(m, n, &q, &qc, &sort));
   if (mem == BVHC_MEM_DEVICE) return from_cuda(launch_intersects_box(m->view(), boxes, n, out, s, q, qc, &sort));
   BVHC_CUDA_TRY(ensure(&m->d_in, &m->in_cap, n * 96));
   BVHC_CUDA_TRY(ensure(&m->d_out, &m->out_cap, n));

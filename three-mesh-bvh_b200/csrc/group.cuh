@@ -34,8 +34,61 @@ __device__ __forceinline__ void group_rank(int key, int& rank, unsigned& first) 
   first = (unsigned)__vimin3_s32(__vimin3_s32(key, a, b), c, c) & 3u;
 }
 
+// ---------------------------------------------------------------------------------------------
+// A warp takes the up to eight newest entries of its stack at once, four lanes each: an entry that is a
+// record has its four children tested, one that is a run its triangles.  What is entered goes back on
+// the stack, the newest entry's children on top, nearest first.  A step tests what eight steps of a
+// single walk would; some of it the nearer entries' results would have spared, which costs nothing
+// while the chip is otherwise idle.
+// Stack: `cap` entries per warp.  Eight entries are taken while what they can add (32) and one depth-
+// first walk (quad_stack) still fit above the rest, else one, so nothing overflows.
+// ---------------------------------------------------------------------------------------------
+constexpr int kWideSpare = 256;
+__host__ __device__ inline int wide_stack(int quad_stack) { return kWideSpare + 32 + quad_stack; }
+
+struct WideEntry {
+  uint32_t link;
+  float key;
+  bool on;
+};
+// This lane's group's entry, and the stack without what was taken.
+__device__ __forceinline__ WideEntry wide_take(const uint2* stack, int& sp, unsigned lane, int spare = kWideSpare) {
+  const int width = sp <= spare ? 8 : 1, g = (int)(lane / kGroup);
+  WideEntry e{0u, 0.0f, g < width && g < sp};
+  if (e.on) {
+    const uint2 v = stack[sp - 1 - g];
+    e.link = v.x;
+    e.key = __uint_as_float(v.y);
+  }
+  sp -= min(width, sp);
+  __syncwarp();
+  return e;
+}
+// Stacks the children that are entered: the first group's on top, each group's nearest first.
+__device__ __forceinline__ void wide_push(uint2* stack, int& sp, unsigned lane, bool enter, uint32_t link, float key,
+                                          float word) {
+  const unsigned full = 0xFFFFFFFFu, j = lane & 3u, base = lane & ~3u;
+  int rank;
+  unsigned first;
+  group_rank(enter ? (int)((__float_as_uint(key) & ~3u) | j) : 0x7FFFFFFF, rank, first);
+  const unsigned all = __ballot_sync(full, enter);
+  if (enter) {
+    const int later = base == 28u ? 0 : __popc(all >> (base + kGroup)), own = __popc((all >> base) & 0xFu);
+    stack[sp + later + own - 1 - rank] = make_uint2(link, __float_as_uint(word));
+  }
+  sp += __popc(all);
+  __syncwarp();
+}
+__device__ __forceinline__ float warp_min(float v) {
+  for (int x = 1; x < 32; x <<= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, x));
+  return v;
+}
+
 }  // namespace dev
 
+// Shared memory of a block's stacks: four lanes a query, or a warp.
 static inline size_t group_smem(int stack) { return (size_t)dev::kBlockGroups * (stack + 1) * sizeof(uint2); }
+
+static inline size_t wide_smem(int stack) { return (size_t)dev::kWarps * dev::wide_stack(stack) * sizeof(uint2); }
 
 }  // namespace bvhc

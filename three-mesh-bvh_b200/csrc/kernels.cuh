@@ -153,6 +153,8 @@ cudaError_t launch_raycast_all(const MeshDev& m, const float* rays, uint64_t n, 
 // Shapecasts (intersectsSphere, triangles within spheres, intersectsBox): with queue, qcount and
 // sort scratch for n queries, the queries are first sorted by the Morton key of their centres over
 // sort->lo..hi and taken in that order (results stay in input order); otherwise in input order.
+// Where shapes_by_group, intersectsSphere and intersectsBox take them in input order and use no scratch.
+bool shapes_by_group(const MeshDev& m, uint64_t n);
 cudaError_t launch_intersects_sphere(const MeshDev& m, const float* spheres, uint64_t n, uint8_t* out,
                                      cudaStream_t stream, uint32_t* queue = nullptr, unsigned int* qcount = nullptr,
                                      const RaySort* sort = nullptr);

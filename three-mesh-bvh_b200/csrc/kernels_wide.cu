@@ -9,55 +9,6 @@
 namespace bvhc {
 namespace dev {
 
-// ---------------------------------------------------------------------------------------------
-// A warp takes the up to eight newest entries of its stack at once, four lanes each: an entry that is a
-// record has its four children tested, one that is a run its triangles.  What is entered goes back on
-// the stack, the newest entry's children on top, nearest first.  A step tests what eight steps of a
-// single walk would; some of it the nearer entries' results would have spared, which costs nothing
-// while the chip is otherwise idle.
-// Stack: `cap` entries per warp.  Eight entries are taken while what they can add (32) and one depth-
-// first walk (quad_stack) still fit above the rest, else one, so nothing overflows.
-// ---------------------------------------------------------------------------------------------
-constexpr int kWideSpare = 256;
-__host__ __device__ inline int wide_stack(int quad_stack) { return kWideSpare + 32 + quad_stack; }
-
-struct WideEntry {
-  uint32_t link;
-  float key;
-  bool on;
-};
-// This lane's group's entry, and the stack without what was taken.
-__device__ __forceinline__ WideEntry wide_take(const uint2* stack, int& sp, unsigned lane) {
-  const int width = sp <= kWideSpare ? 8 : 1, g = (int)(lane / kGroup);
-  WideEntry e{0u, 0.0f, g < width && g < sp};
-  if (e.on) {
-    const uint2 v = stack[sp - 1 - g];
-    e.link = v.x;
-    e.key = __uint_as_float(v.y);
-  }
-  sp -= min(width, sp);
-  __syncwarp();
-  return e;
-}
-// Stacks the children that are entered: the first group's on top, each group's nearest first.
-__device__ __forceinline__ void wide_push(uint2* stack, int& sp, unsigned lane, bool enter, uint32_t link, float key) {
-  const unsigned full = 0xFFFFFFFFu, j = lane & 3u, base = lane & ~3u;
-  int rank;
-  unsigned first;
-  group_rank(enter ? (int)((__float_as_uint(key) & ~3u) | j) : 0x7FFFFFFF, rank, first);
-  const unsigned all = __ballot_sync(full, enter);
-  if (enter) {
-    const int later = base == 28u ? 0 : __popc(all >> (base + kGroup)), own = __popc((all >> base) & 0xFu);
-    stack[sp + later + own - 1 - rank] = make_uint2(link, __float_as_uint(key));
-  }
-  sp += __popc(all);
-  __syncwarp();
-}
-__device__ __forceinline__ float warp_min(float v) {
-  for (int x = 1; x < 32; x <<= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, x));
-  return v;
-}
-
 template <bool MATERIALS>
 __global__ void __launch_bounds__(kBlock) raycast_first_wide_kernel(MeshDev m, const BatchDev bd, bool batched,
                                                                     const float* __restrict__ rays, uint32_t n, int side,
@@ -111,7 +62,7 @@ __global__ void __launch_bounds__(kBlock) raycast_first_wide_kernel(MeshDev m, c
           lim_hit = slab_limit(warp_min((best.t + best.err) * (1.0f + kSlabMargin)));
           lim = fminf(lim, lim_hit);
         }
-        if (__ballot_sync(full, enter)) wide_push(stack, sp, lane, enter, link, key);
+        if (__ballot_sync(full, enter)) wide_push(stack, sp, lane, enter, link, key, key);
       }
     }
     for (int x = 1; x < 32; x <<= 1) {
@@ -167,7 +118,7 @@ __global__ void __launch_bounds__(kBlock) closest_point_wide_kernel(MeshDev m, c
         }
         if (__ballot_sync(full, leaf))
           bound = fminf(bound, warp_min(fminf((best.d2 + best.err) * (1.0f + 0x1p-18f), FLT_MAX)));
-        if (__ballot_sync(full, enter)) wide_push(stack, sp, lane, enter, link, key);
+        if (__ballot_sync(full, enter)) wide_push(stack, sp, lane, enter, link, key, key);
       }
     }
     store_merged<32>(m.tris, p, best, true, reinterpret_cast<uint32_t*>(out + qid), s_tie);
@@ -180,7 +131,7 @@ cudaError_t launch_raycast_first_wide(const MeshDev& m, const BatchDev* batch, c
                                       const SideTable& sides, float near_d, float far_d, bvhc_hit* out,
                                       cudaStream_t stream, const uint32_t* queue, const unsigned int* qcount) {
   const int cap = dev::wide_stack(group_stack(m));
-  const size_t smem = (size_t)dev::kWarps * cap * sizeof(uint2);
+  const size_t smem = wide_smem(group_stack(m));
   auto kernel = sides.per_material ? dev::raycast_first_wide_kernel<true> : dev::raycast_first_wide_kernel<false>;
   const BatchDev bd = batch ? *batch : BatchDev{nullptr, nullptr, 0};
   const unsigned int grid = (unsigned int)((n + dev::kWarps - 1) / dev::kWarps);
@@ -192,7 +143,7 @@ cudaError_t launch_raycast_first_wide(const MeshDev& m, const BatchDev* batch, c
 cudaError_t launch_closest_wide(const MeshDev& m, const float* pts, uint32_t n, float max_t, bvhc_closest* out,
                                 cudaStream_t stream) {
   const int cap = dev::wide_stack(group_stack(m));
-  const size_t smem = (size_t)dev::kWarps * cap * sizeof(uint2);
+  const size_t smem = wide_smem(group_stack(m));
   const unsigned int grid = std::min((n + dev::kWarps - 1) / dev::kWarps, (unsigned int)sm_count() * 8u);
   dev::closest_point_wide_kernel<<<grid, dev::kBlock, smem, stream>>>(m, pts, n, max_t, out, cap);
   return cudaGetLastError();
