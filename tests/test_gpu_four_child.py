@@ -145,3 +145,29 @@ def test_shapes_match(pkg, orc, cuda, mesh, n):
     bvh.synchronize()
     assert np.array_equal(got_s, want_s)
     assert np.array_equal(got_b, want_b)
+
+
+@pytest.mark.parametrize("n", [100, 30_000, 140_000])
+def test_boxes_outside_their_parents(pkg, cuda, n):
+    """A tree from a file whose inner boxes do not hold their children's: rays miss what the
+    child-pair kernel misses."""
+    import torch
+
+    g, _ = _mesh(pkg, "plain")
+    data = pkg.MeshBVH.serialize(pkg.MeshBVH(g, {"strategy": pkg.SAH}))
+    nodes = np.frombuffer(data["roots"][0], np.float32).reshape(-1, 8).copy()
+    count = nodes.view(np.uint32)[:, 7]
+    for k in range(1, 40):
+        if count[k] >> 16 != 0xFFFF:          # an inner node
+            nodes[k, 3:6] = 0.5 * (nodes[k, 0:3] + nodes[k, 3:6])
+    data["roots"] = [nodes.tobytes()]
+    bvh = pkg.MeshBVH.deserialize(data, g)
+    rays = torch.from_numpy(_rays(pkg, n)).to(cuda)
+    bvh.set_traversal(0, 1)
+    want = bvh.raycast_first_batch(rays)
+    bvh.set_traversal(1, 1)
+    got = bvh.raycast_first_batch(rays)
+    bvh.synchronize()
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    full = pkg.MeshBVH(g, {"strategy": pkg.SAH}).raycast_first_batch(rays)
+    assert not torch.equal(full.view(torch.int32), want.view(torch.int32))

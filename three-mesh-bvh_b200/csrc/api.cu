@@ -478,6 +478,8 @@ struct QuadBuilder {
   std::vector<QuadNode> quads;
   std::vector<uint32_t> src;
   int stack = 0;  // entries a traversal can stack: at most the siblings along one path
+  bool nested = true;  // every box of the tree lies in its parent's, so that those that are not records'
+                       // children need no test (a tree from a file may hold anything)
 
   struct Child {
     uint32_t pair;   // internal: its pair record; else kEmptyLeaf
@@ -485,6 +487,7 @@ struct QuadBuilder {
     uint32_t first, count;  // not internal: its triangle records
     float box[6];
     bool part;       // of a leaf: its box is not one of the tree's
+    bool boxed;      // a node with a box of the tree's (not a root)
     bool internal() const { return pair != kEmptyLeaf; }
     bool splits() const { return internal() || count > (uint32_t)kMaxRun; }
   };
@@ -559,6 +562,7 @@ struct QuadBuilder {
       }
       src.insert(src.end(), part[t].src.begin(), part[t].src.end());
       stack = std::max(stack, part[t].stack);
+      nested = nested && part[t].nested;
       part[t].quads = {};
     }
     later.clear();
@@ -574,6 +578,7 @@ struct QuadBuilder {
     Child c{};
     const uint32_t link = pairs[pair].link[s];
     c.slot = 2 * pair + (uint32_t)s;
+    c.boxed = true;
     std::memcpy(c.box, pairs[pair].f + 6 * s, sizeof c.box);
     c.pair = link & kLeafBit ? kEmptyLeaf : link;
     if (link & kLeafBit && link != kEmptyLeaf) {
@@ -593,10 +598,18 @@ struct QuadBuilder {
     return c;
   }
 
-  void halves(const Child& c, Child& a, Child& b) const {
+  static bool inside(const Child& in, const float* out) {
+    if (!in.internal() && in.count == 0) return true;
+    for (int k = 0; k < 3; ++k)
+      if (!(in.box[k] >= out[k] && in.box[3 + k] <= out[3 + k])) return false;
+    return true;
+  }
+
+  void halves(const Child& c, Child& a, Child& b) {
     if (c.pair != kEmptyLeaf) {
       a = side(c.pair, 0);
       b = side(c.pair, 1);
+      if (c.boxed) nested = nested && inside(a, c.box) && inside(b, c.box);
     } else {
       const uint32_t half = (c.count + 1) / 2;
       a = run(c.first, half);
@@ -780,6 +793,7 @@ static cudaError_t install_quads(bvhc_mesh* m, int k, const std::vector<PairNode
   } catch (const std::bad_alloc&) {
     return cudaErrorMemoryAllocation;
   }
+  if (!qb.nested) return cudaStreamSynchronize(nullptr);  // the child-pair kernels take such a tree
   e = upload(&q.quads, qb.quads);
   if (e == cudaSuccess) e = upload(&q.roots, qroots);
   if (e == cudaSuccess) e = upload(&q.src, qb.src);
