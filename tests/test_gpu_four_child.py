@@ -1,6 +1,7 @@
 """raycastFirst over the four-child records, one lane, four and the whole warp per ray, against the per-ray child-pair
 kernel byte for byte: one candidate order decides in every kernel (the nearest hit, exact ties to the
 smaller record), so neither the records' shape nor the batch size may change a bit."""
+import importlib
 import math
 
 import numpy as np
@@ -171,3 +172,40 @@ def test_boxes_outside_their_parents(pkg, cuda, n):
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
     full = pkg.MeshBVH(g, {"strategy": pkg.SAH}).raycast_first_batch(rays)
     assert not torch.equal(full.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("n", [32, 1000, 5000, 131072, 200_001])
+@pytest.mark.parametrize("near,far", [(0.0, math.inf), (30.0, 900.0)])
+def test_instances_match_fewer_rays_per_call(pkg, cuda, n, near, far):
+    """Instanced raycastFirst, phased: the records of calls of fewer than 32 rays, which go one thread per ray."""
+    import torch
+
+    batched = importlib.import_module(pkg.__name__ + ".batched")
+    rng = np.random.default_rng(n)
+    batch = batched.BatchedMeshBVH([_mesh(pkg, k)[0] for k in ("plain", "leaf40", "triangle")], {"strategy": pkg.SAH})
+    batch.set_leaf_size(3 if n % 2 else 0)
+    k = 70
+    q, _ = np.linalg.qr(rng.standard_normal((k, 3, 3)))
+    m = np.zeros((k, 16))
+    for c in range(3):
+        m[:, 4 * c:4 * c + 3] = q[:, :, c] * rng.uniform(0.4, 2.0, (k, 1))
+    m[:, 12:15] = rng.uniform(-60, 60, (k, 3))
+    m[:, 15] = 1
+    m[1], geometry = m[0], rng.integers(0, 3, k).astype(np.uint32)
+    geometry[1] = geometry[0]              # two instances in one place: the lower index
+    scene = batch.instances(geometry, m)
+    o = rng.standard_normal((n, 3))
+    o *= 150 / np.linalg.norm(o, axis=1, keepdims=True)
+    d = rng.uniform(-60, 60, (n, 3)) - o
+    d[::2] /= np.linalg.norm(d[::2], axis=1, keepdims=True)
+    rays = torch.from_numpy(np.concatenate([o, d], 1).astype(np.float32)).to(cuda)
+    hits, inst = scene.raycast_first(rays, 2, near, far)
+    torch.cuda.synchronize()
+    assert (inst != -1).any()
+    step = max(1, n // 300)
+    for i in range(0, n, 31 * step):
+        one = rays[i:i + 31].clone()
+        h, k1 = scene.raycast_first(one, 2, near, far)
+        torch.cuda.synchronize()
+        assert torch.equal(k1, inst[i:i + 31])
+        assert torch.equal(h.view(torch.int32), hits[i:i + 31].view(torch.int32))

@@ -2029,6 +2029,11 @@ struct bvhc_scene {
   PairNode* d_tlas = nullptr;
   size_t tlas_cap = 0;
   uint32_t root = kEmptyLeaf;
+  QuadNode* d_quads = nullptr;  // the same tree in four-child records; has_quads: of these instances
+  size_t quads_cap = 0;
+  bool has_quads = false;
+  uint32_t quad_root = 0;
+  int quad_stack = 0;
   void* d_in = nullptr;
   size_t in_cap = 0;
   void* d_out = nullptr;
@@ -2109,6 +2114,28 @@ float round_down(double x) {
 float round_up(double x) {
   float f = (float)x;
   return (double)f < x ? std::nextafter(f, INFINITY) : f;
+}
+
+// The instance tree in four-child records, for the phased raycastFirst.
+bvhc_status set_instance_quads(bvhc_scene* sc, const std::vector<PairNode>& nodes) {
+  sc->has_quads = false;
+  try {
+    TriRecord one{};
+    one.flags = kTriLast;  // a leaf's run: its instance
+    const std::vector<TriRecord> leaves(std::max(sc->n_instances, 1), one);
+    QuadBuilder qb{nodes, leaves};
+    sc->quad_root = qb.root(sc->root);
+    if (!qb.nested) return BVHC_OK;
+    BVHC_CUDA_TRY(ensure(reinterpret_cast<void**>(&sc->d_quads), &sc->quads_cap, qb.quads.size() * sizeof(QuadNode)));
+    BVHC_CUDA_TRY(cudaMemcpy(sc->d_quads, qb.quads.data(), qb.quads.size() * sizeof(QuadNode), cudaMemcpyHostToDevice));
+    sc->quad_stack = qb.stack;
+    sc->has_quads = true;
+  } catch (const Status& st) {
+    return st.code;
+  } catch (const std::bad_alloc&) {
+    return BVHC_ERR_OUT_OF_MEMORY;
+  }
+  return BVHC_OK;
 }
 
 bvhc_status set_instances(bvhc_scene* sc, int n, const uint32_t* geometry, const double* matrices,
@@ -2204,7 +2231,7 @@ bvhc_status set_instances(bvhc_scene* sc, int n, const uint32_t* geometry, const
   }
   sc->root = root;
   sc->n_instances = n;
-  return BVHC_OK;
+  return set_instance_quads(sc, nodes);
 }
 
 }  // namespace
@@ -2245,6 +2272,9 @@ bvhc_status bvhc_scene_raycast_first(bvhc_scene* sc, const float* rays, uint64_t
   SceneDev sd{sc->d_tlas, sc->root, sc->d_inst, m->d_mesh_root_off};
   sd.n_instances = sc->n_instances;
   sd.occupancy = sc->variant;
+  sd.quads = sc->has_quads ? sc->d_quads : nullptr;
+  sd.quad_root = sc->quad_root;
+  sd.quad_stack = sc->quad_stack;
   if (mem == BVHC_MEM_HOST && n > kPipeChunk) {
     // Large host batches: chunks of kPipeChunk rays rotate over the batch mesh's three pipeline
     // streams and staging slots (instance ids in a slot of the scene's own), so the copies of some
@@ -2361,6 +2391,7 @@ void bvhc_scene_destroy(bvhc_scene* sc) {
   if (sc->batch) cudaSetDevice(sc->batch->device);
   cudaFree(sc->d_inst);
   cudaFree(sc->d_tlas);
+  cudaFree(sc->d_quads);
   cudaFree(sc->d_in);
   cudaFree(sc->d_out);
   cudaFree(sc->d_ids);

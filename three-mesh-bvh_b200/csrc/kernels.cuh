@@ -177,6 +177,10 @@ struct SceneDev {
   const uint32_t* mesh_root_off;
   int n_instances = 1 << 30;   // bounds the instance tree's depth (a median split)
   int occupancy = 0;           // raycastFirst kernel variant (bvhc_scene_set_variant)
+  // the instance tree in four-child records (a leaf's run is its instance); null: not to be had
+  const QuadNode* quads = nullptr;
+  uint32_t quad_root = 0;
+  int quad_stack = 0;
 };
 // World-space raycastFirst over the instances: hits[i] in world space (distance, point; local
 // barycoord and faceIndex), instance[i] the hit instance (0xFFFFFFFF: none).  With `sort` (kind

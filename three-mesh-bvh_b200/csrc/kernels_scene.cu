@@ -28,7 +28,7 @@ __device__ __forceinline__ RayF ray_from(float3 o, float3 d) {
   const float dx = fabsf(d.x) < kTiny ? copysignf(kTiny, d.x) : d.x;
   const float dy = fabsf(d.y) < kTiny ? copysignf(kTiny, d.y) : d.y;
   const float dz = fabsf(d.z) < kTiny ? copysignf(kTiny, d.z) : d.z;
-  r.inv = make_float3(__frcp_rn(dx), __frcp_rn(dy), __frcp_rn(dz));
+  r.inv = make_float3(rcp_fast(dx), rcp_fast(dy), rcp_fast(dz));
   r.dk = kFilterK * (fabsf(d.x) + fabsf(d.y) + fabsf(d.z));
   return r;
 }
@@ -324,6 +324,315 @@ __global__ void __launch_bounds__(kBlock, MINB) scene_raycast_first_kernel(MeshD
   inst_out[i] = best_inst;
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same over four-child records of both levels, one ray per lane in warp-wide phases as
+// raycast_first_phased_kernel has them: node steps (records of the instance tree under the world ray and
+// of a geometry's tree under the local one alike, only the base pointer and the ray's slab constants
+// differ), leaf steps, and instance steps, which leave a finished instance or enter the next (the local
+// ray, in float-float).  An instance step costs about three node steps, so lanes wait for it until
+// kSceneSwitch of them are ready or the others are fewer than they.
+// What bounds it: instructions issued with 11 of 32 lanes, six tenths of them in node steps.  World records
+// are left to scene_finalize_kernel: made at each hit, by two lanes on average, their long float-float
+// chains evicted the walk's own code from the instruction cache (20 of 29 stalled cycles per instruction,
+// 5.7 ms).  1,048,576 rays over 512 instances of 20,000-triangle knots: 3.2 ms with one thread per ray
+// throughout, 1.6-1.7 ms here; over 4,096 instances 8.0 ms, 3.4 ms here.
+// ---------------------------------------------------------------------------------------------
+// The nearest hit over the instances so far: its world ray parameter is within lo..hi.
+struct WorldBest {
+  float lo, hi;
+  uint32_t inst, rec;
+};
+__device__ __forceinline__ WorldBest world_none() { return {kInf, kInf, 0xFFFFFFFFu, 0xFFFFFFFFu}; }
+
+// Whether instance a's hit goes before instance b's: by world distance in float-float, then by index.
+static __device__ __noinline__ bool world_before(const MeshDev& m, const SceneDev& sc, const RayF& w, uint32_t a,
+                                                 uint32_t rec_a, uint32_t b, uint32_t rec_b) {
+  ff d[2];
+  for (int k = 0; k < 2; ++k) {
+    const InstanceDev& I = sc.inst[k ? b : a];
+    LocalRay L;
+    local_ray(I, w, 0.0f, kInf, L);
+    bvhc_hit h;
+    d[k] = world_record(m, I, k ? rec_b : rec_a, w, L.r, h);
+  }
+  return ff_lt(d[0], d[1]) || (!ff_lt(d[1], d[0]) && a < b);
+}
+
+// Offers an instance's nearest hit.  The world distance is that of the exact ray; the local ray, rounded to
+// float32 (its origin by 2^-24 |o|, its direction by 2^-24 |d|), meets the triangle's plane (normal n, N = n . d)
+// within (|o|_1 + t |d|_1) 2^-24 |n| / |N| of it, taken fourfold, unless N is so small that its float32 value or
+// the bound is in doubt.  2^-16 of the distance covers the transforms themselves.
+__device__ __forceinline__ void offer_world(const MeshDev& m, const SceneDev& sc, const RayF& w, const RayF& r,
+                                            const Best& best, uint32_t inst, float vlen, WorldBest& wb) {
+  const Tri t = load_tri(m.tris, best.rec);
+  const float3 e1 = make_float3(t.b.x - t.a.x, t.b.y - t.a.y, t.b.z - t.a.z),
+               e2 = make_float3(t.c.x - t.a.x, t.c.y - t.a.y, t.c.z - t.a.z);
+  const float3 n = make_float3(e1.y * e2.z - e1.z * e2.y, e1.z * e2.x - e1.x * e2.z, e1.x * e2.y - e1.y * e2.x);
+  const float l1 = fabsf(e1.x) + fabsf(e1.y) + fabsf(e1.z), l2 = fabsf(e2.x) + fabsf(e2.y) + fabsf(e2.z);
+  const float d1 = fabsf(r.d.x) + fabsf(r.d.y) + fabsf(r.d.z), o1 = fabsf(r.o.x) + fabsf(r.o.y) + fabsf(r.o.z);
+  const float nd = fabsf(r.d.x * n.x + r.d.y * n.y + r.d.z * n.z);
+  const float at = best.t / vlen;
+  float slack = kInf;
+  if (nd > 0x1p-16f * l1 * l2 * d1)
+    slack = ((o1 + best.t * d1) * 0x1p-22f * fmaxf(fmaxf(fabsf(n.x), fabsf(n.y)), fabsf(n.z)) / nd + best.err) / vlen;
+  slack = slack * (1.0f + 0x1p-16f) + at * 0x1p-16f;
+  const WorldBest c{at - slack, at + slack, inst, best.rec};
+  bool first = c.hi < wb.lo || wb.inst == 0xFFFFFFFFu;
+  if (!first && !(c.lo > wb.hi)) first = world_before(m, sc, w, inst, best.rec, wb.inst, wb.rec);
+  if (first) wb = c;
+}
+
+static __device__ __noinline__ void scene_record(const MeshDev& m, const SceneDev& sc, const float* __restrict__ rays,
+                                                 uint64_t i, uint32_t inst, uint32_t rec, bvhc_hit* __restrict__ out) {
+  const RayF w = make_ray(rays, i);
+  LocalRay L;
+  local_ray(sc.inst[inst], w, 0.0f, kInf, L);
+  bvhc_hit h;
+  world_record(m, sc.inst[inst], rec, w, L.r, h);
+  store_hit(out + i, h);
+}
+
+constexpr int kSceneBlocksPerSm = 6;  // 80 registers; 8, 5 and 4 blocks 6, 3 and 11% slower
+constexpr int kSceneSwitch = 16;     // 8 and 12: 14 and 3% slower; 20: the same
+constexpr int kSceneRefill = 6;      // idle lanes at which a warp takes new rays; 12 and 20: 4 and 14% slower
+constexpr int kSceneTop = 12;     // stack entries in shared memory
+constexpr int kSceneStack = 96;   // of both levels together
+
+template <bool RANGED>
+__global__ void __launch_bounds__(kBlock, kSceneBlocksPerSm) scene_first_phased_kernel(
+    MeshDev m, SceneDev sc, const float* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ queue, int side,
+    float near_d, float far_d, bvhc_hit* __restrict__ out, uint32_t* __restrict__ inst_out, uint32_t take,
+    bool complete) {
+  const unsigned full = 0xFFFFFFFFu;
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  const SideTable no_sides{};
+  // a lane's state: `alive` until its ray is finished; inst: the instance it is in, or kNone; `walking`
+  // while the instance's walk (or the instance tree's) goes on; link, dead, nl, leaf0, leaf1 as in
+  // raycast_first_phased_kernel
+  constexpr uint32_t kNone = 0xFFFFFFFFu;
+  bool alive = false, walking = false, dead = false, pending = false;
+  uint32_t inst = kNone, rid = 0, link = 0, leaf0 = 0, leaf1 = 0;
+  int nl = 0, sp = 0, bsp = 0, root = 0, root_end = 0;
+  RayF r{};  // the local ray
+  RaySlab rs{};
+  float dlen = 0.0f, vlen = 1.0f, near_l = 0.0f, far_l = 0.0f, lim = 0.0f, lim_hit = 0.0f, near_s = 0.0f;
+  bool odd = false;
+  Best best{kInf, 0.0f, kNone};
+  WorldBest wb = world_none();
+  __shared__ uint2 s_top[kSceneTop][kBlock];
+  uint2 rest[kSceneStack - kSceneTop];
+  auto push = [&](uint32_t l, int key) {
+    const uint2 e = make_uint2(l, (uint32_t)key);
+    if (sp < kSceneTop) s_top[sp][threadIdx.x] = e;
+    else rest[sp - kSceneTop] = e;
+    ++sp;
+  };
+  auto pop = [&]() {
+    dead = true;
+    if (sp > bsp) {
+      --sp;
+      const uint2 e = sp < kSceneTop ? s_top[sp][threadIdx.x] : rest[sp - kSceneTop];
+      link = e.x;
+      dead = !(__uint_as_float(e.y) <= (RANGED ? lim_hit : lim));
+    } else {
+      dead = false;
+      walking = inst != kNone && ++root < root_end;
+      if (walking) link = m.quad_roots[root];
+      alive = inst != kNone;
+    }
+  };
+  // the world ray's limit: nothing beyond the nearest hit so far
+  auto world = [&](const RayF& w) {
+    lim = slab_limit(wb.hi);
+    if (RANGED) {
+      lim_hit = lim;
+      near_s = 0.0f;
+      odd = false;
+    }
+    rs = ray_slab(w);
+    inst = kNone;
+    bsp = 0;
+    walking = true;
+  };
+  // this warp's chunks of `take` rays (at most 32): every (warps of the grid)-th one
+  const uint32_t warps = gridDim.x * kWarps, chunks = (n + take - 1u) / take;
+  uint32_t chunk = blockIdx.x * kWarps + (threadIdx.x >> 5), pool = 0, pool_end = 0;
+  for (;;) {
+    const unsigned idle = __ballot_sync(full, !alive);
+    if (idle == full || (__popc(idle) >= kSceneRefill && (chunk < chunks || pool < pool_end))) {
+      if (!alive && pending) {
+        if (!complete) store_pending_record(out + rid, wb.rec, wb.hi);  // scene_finalize_kernel completes it
+        else if (wb.inst == kNone) store_miss(out + rid);
+        else scene_record(m, sc, rays, rid, wb.inst, wb.rec, out);
+        inst_out[rid] = wb.inst;
+        pending = false;
+      }
+      if (pool == pool_end && chunk < chunks) {
+        pool = chunk * take;
+        pool_end = n - pool > take ? pool + take : n;
+        chunk += warps;
+      }
+      const unsigned want = __popc(idle), avail = pool_end - pool, rank = __popc(idle & below);
+      if (!alive && rank < avail) {
+        rid = pool + rank;
+        if (queue) rid = __ldg(queue + rid);
+        alive = pending = true;
+        dead = false;
+        wb = world_none();
+        world(make_ray(rays, rid));
+        sp = 0;
+        link = sc.quad_root;
+      }
+      pool += want < avail ? want : avail;
+      if (!__ballot_sync(full, alive)) {
+        if (chunk >= chunks && pool == pool_end) break;
+        continue;
+      }
+    }
+    const int keep = chunk >= chunks && pool == pool_end ? 1 : 33 - kSceneRefill;
+    for (;;) {
+      const bool at_node = alive && walking && (dead || !(link & kLeafBit));
+      const bool at_switch = alive && (inst == kNone ? walking && !dead && (link & kLeafBit) : !walking && nl == 0);
+      const unsigned nodes = __ballot_sync(full, at_node), leaves = __ballot_sync(full, nl > 0),
+                     switches = __ballot_sync(full, at_switch);
+      const int N = __popc(nodes), L = __popc(leaves), S = __popc(switches);
+      if (__popc(nodes | leaves | switches) < keep) break;
+      if (S >= kSceneSwitch || S >= N + L) {
+        if (at_switch) {
+          const RayF w = make_ray(rays, rid);
+          if (inst != kNone) {
+            if (best.rec != kNone) offer_world(m, sc, w, r, best, inst, vlen, wb);
+            world(w);
+            pop();
+          }
+          // a lane that left one instance may have the next at hand
+          if (alive && !dead && (link & kLeafBit)) {
+            const uint32_t j = link & kRunFirst;
+            const InstanceDev& I = sc.inst[j];
+            LocalRay lr;
+            dead = true;
+            if (local_ray(I, w, near_d, far_d, lr)) {
+              const float tlim = wb.hi * lr.vlen * (1.0f + 0x1p-20f);
+              vlen = lr.vlen;
+              r = lr.r;
+              rs = ray_slab(r);
+              dlen = lr.len;
+              far_l = fminf(lr.far_d, tlim);
+              near_l = lr.near_d;
+              if (RANGED) {
+                near_s = slab_near(near_l);
+                lim_hit = slab_limit(tlim);
+                odd = odd_length(r.d);
+              }
+              lim = slab_far(far_l);
+              best = Best{kInf, 0.0f, kNone};
+              inst = j;
+              bsp = sp;
+              root = (int)__ldg(sc.mesh_root_off + I.geometry);
+              root_end = (int)__ldg(sc.mesh_root_off + I.geometry + 1);
+              dead = false;
+              walking = root < root_end;
+              if (walking) link = m.quad_roots[root];
+            }
+          }
+        }
+      } else if (N >= L) {
+        if (at_node) {
+          bool none = true;
+          if (!dead) {
+            const QuadNode* q = (inst == kNone ? sc.quads : m.quads) + link;
+            int key[4];
+            uint32_t l[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const ChildBox b = load_child(q->c + c);
+              float e;
+              const bool free_box = RANGED && odd && b.part;
+              const bool h = child_hit(b, rs, RANGED && !free_box ? near_s : 0.0f, free_box ? lim_hit : lim, e);
+              key[c] = h ? (int)((__float_as_uint(e) & ~3u) | c) : 0x7FFFFFFF;
+              l[c] = b.link;
+            }
+            auto cas = [&](int a, int b) {
+              const int lo = min(key[a], key[b]), hi = max(key[a], key[b]);
+              key[a] = lo;
+              key[b] = hi;
+            };
+            cas(0, 1);
+            cas(2, 3);
+            cas(0, 2);
+            cas(1, 3);
+            cas(1, 2);
+            auto pick = [&](int k) {
+              const uint32_t a = (k & 1) ? l[1] : l[0], b = (k & 1) ? l[3] : l[2];
+              return (k & 2) ? b : a;
+            };
+#pragma unroll
+            for (int k = 3; k >= 1; --k)
+              if (key[k] != 0x7FFFFFFF) push(pick(key[k]), key[k]);
+            link = pick(key[0]);
+            none = key[0] == 0x7FFFFFFF;
+          }
+          if (none) pop();
+          if (inst != kNone && walking && !dead && (link & kLeafBit) && nl < 2) {
+            if (nl == 0) leaf0 = link;
+            else leaf1 = link;
+            ++nl;
+            pop();
+          }
+        }
+      } else if (nl > 0) {
+        const uint32_t k = leaf0 & kRunFirst;
+        const Tri t = load_tri(m.tris, k);
+        const int ts = tri_side(t, side, no_sides);
+        if (ts >= 0) offer_first(m, t, k, r, dlen, ts, near_l, far_l, best);
+        const float nearest = slab_limit((best.t + best.err) * (1.0f + kSlabMargin));
+        lim = fminf(lim, nearest);
+        if (RANGED) lim_hit = fminf(lim_hit, nearest);
+        if (!(leaf0 & ~(kLeafBit | kRunFirst))) {
+          leaf0 = leaf1;
+          --nl;
+          if (walking && !dead && (link & kLeafBit)) {  // the leaf that waited for a slot
+            if (nl == 0) leaf0 = link;
+            else leaf1 = link;
+            ++nl;
+            dead = true;
+          }
+        } else {
+          leaf0 += 1u - (1u << kRunShift);
+        }
+      }
+    }
+  }
+}
+
+// The records of the nearest hits that scene_first_phased_kernel found.  A block lists its rays' hits first,
+// so that the long float-float chains run on full warps (4,700 instructions a warp, and 13 of 32 lanes where
+// two of five rays hit).
+constexpr int kSceneFinalize = 512;  // rays a block
+__global__ void __launch_bounds__(kBlock) scene_finalize_kernel(MeshDev m, SceneDev sc, const float* __restrict__ rays,
+                                                                uint64_t n, bvhc_hit* __restrict__ out,
+                                                                const uint32_t* __restrict__ inst_out) {
+  __shared__ uint16_t s_hit[kSceneFinalize];
+  __shared__ int s_hits;
+  const uint64_t first = (uint64_t)blockIdx.x * kSceneFinalize;
+  if (threadIdx.x == 0) s_hits = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < kSceneFinalize; k += kBlock) {
+    const bool in = first + k < n, hit = in && __ldg(inst_out + first + k) != 0xFFFFFFFFu;
+    if (in && !hit) store_miss(out + first + k);
+    const unsigned hits = __ballot_sync(0xFFFFFFFFu, hit), lane = threadIdx.x & 31u;
+    int at = 0;
+    if (lane == 0 && hits) at = atomicAdd(&s_hits, __popc(hits));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (hit) s_hit[at + __popc(hits & ((1u << lane) - 1u))] = (uint16_t)k;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < s_hits; q += kBlock) {
+    const uint64_t i = first + s_hit[q];
+    scene_record(m, sc, rays, i, __ldg(inst_out + i), *reinterpret_cast<const uint32_t*>(out + i), out);
+  }
+}
+
 // Instanced raycast (all hits): the BatchedMesh raycast without firstHitOnly.  Every entered
 // instance box (no pruning: the count covers every hit) is walked in the instance's frame with the
 // reference's all-hits DFS (left child before right), each hit converted to world space and
@@ -522,6 +831,30 @@ cudaError_t launch_scene_raycast_first(const MeshDev& blas, const SceneDev& scen
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if ((e = launch_ray_sort(sort->kind, n, qcount, sort->scratch, queue, stream)) != cudaSuccess) return e;
+  }
+  // The phased kernel, but for a few instances unless there are many rays, and a few rays: its steps are
+  // longer, and pay where there is divergence to be saved.  30 instances: 16,000 rays 46 us one thread
+  // per ray, 66 phased; 64,000 65 / 82; 128,000 89 / 91; 3 instances, 1,048,576 rays 145 / 117.  64 instances:
+  // 64 rays 34 / 33, 1,000 60 / 51, 64,000 136 / 127.  512 instances: 1 ray 64 / 83, 64 rays 168 / 76, 16,000
+  // 245 / 212, 128,000 623 / 378.
+  const bool many = n >= 131072 || (n >= 32 && scene.n_instances >= 64);
+  if (many && phased_stack(blas) && scene.quads && blas.quad_stack + scene.quad_stack <= dev::kSceneStack &&
+      n < (1ull << 32)) {
+    auto phased = dev::ranged(near_d, far_d) ? dev::scene_first_phased_kernel<true>
+                                             : dev::scene_first_phased_kernel<false>;
+    // all resident warps, with fewer than 32 rays to start with where the batch is small
+    const uint64_t resident = (uint64_t)sm_count() * dev::kSceneBlocksPerSm * dev::kWarps;
+    const uint32_t take = (uint32_t)std::min<uint64_t>(32, (n + resident - 1) / resident);
+    const uint64_t warps = std::min<uint64_t>((n + take - 1) / take, resident);
+    const unsigned int grid = (unsigned int)((warps + dev::kWarps - 1) / dev::kWarps);
+    const bool complete = take == 1;  // one ray a warp
+    phased<<<grid, dev::kBlock, 0, stream>>>(blas, scene, rays, (uint32_t)n, sorted ? queue : nullptr, side, near_d,
+                                             far_d, hits, instance, take, complete);
+    if (!complete) {
+      const unsigned int blocks = (unsigned int)((n + dev::kSceneFinalize - 1) / dev::kSceneFinalize);
+      dev::scene_finalize_kernel<<<blocks, dev::kBlock, 0, stream>>>(blas, scene, rays, n, hits, instance);
+    }
+    return cudaGetLastError();
   }
   // the small stacks when both trees allow them, else the large ones; resident blocks per SM by
   // the scene's variant (0: 14, 1: 10, 2: 8)
