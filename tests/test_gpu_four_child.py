@@ -209,3 +209,19 @@ def test_instances_match_fewer_rays_per_call(pkg, cuda, n, near, far):
         torch.cuda.synchronize()
         assert torch.equal(k1, inst[i:i + 31])
         assert torch.equal(h.view(torch.int32), hits[i:i + 31].view(torch.int32))
+
+
+@pytest.mark.parametrize("n", [1, 511, 512, 513])
+@pytest.mark.parametrize("config", [(0, 1), (1, 1), (1, 1, 16, 0, 1)])
+def test_host_rays_match_device_rays(pkg, cuda, n, config):
+    """Up to 512 host rays are read and written in page-locked memory, more through device buffers."""
+    import torch
+
+    bvh = pkg.MeshBVH(_mesh(pkg, "plain")[0], {"strategy": pkg.SAH})
+    bvh.set_traversal(*config)
+    rays = _rays(pkg, n)
+    want = bvh.raycast_first_batch(torch.from_numpy(rays).to(cuda))
+    bvh.synchronize()
+    for _ in range(2):
+        got = np.ascontiguousarray(bvh.raycast_first_batch(rays)).view(np.int32).reshape(n, 8)
+        assert np.array_equal(got, want.view(torch.int32).cpu().numpy())

@@ -114,6 +114,17 @@ struct bvhc_mesh {
   };
   QuadSet quad_set[2];
 
+  // Host-memory raycastFirst of a few rays (a pick): page-locked memory that the kernels read and write in
+  // place, made on first need, instead of three copies through pageable memory that are waited for one by
+  // one.  1 ray 48 -> 34 us, 256 rays 47 -> 36, 512 rays 48 -> 40; 1,024 rays 47 -> 48.
+  static constexpr uint64_t kFewRays = 512;
+  struct Few {
+    alignas(16) bvhc_hit hits[kFewRays];
+    float rays[6 * kFewRays];
+    unsigned int err;
+  };
+  Few* few = nullptr;
+
   // the records raycastFirst traverses
   MeshDev view_first() const {
     if (!leaf_size) return view();
@@ -1148,6 +1159,7 @@ void bvhc_mesh_destroy(bvhc_mesh* m) {
   cudaFree(m->d_work);
   cudaFree(m->d_work_all);
   cudaFree(m->d_in);
+  if (m->few) cudaFreeHost(m->few);
   cudaFree(m->d_out);
   cudaFree(m->d_out2);
   for (int k = 0; k < bvhc_mesh::kPipes; ++k) {
@@ -1473,6 +1485,16 @@ static bvhc_status raycast_first_impl(bvhc_mesh* m, const float* rays, uint64_t 
   if (mem == BVHC_MEM_DEVICE) {
     if (!aligned(rays, 8) || !aligned(out, 16)) return BVHC_ERR_INVALID_ARGUMENT;
     return from_cuda(dispatch_first(m, rays, n, side, tab, near_d, far_d, out, m->d_work, s));
+  }
+  if (n <= bvhc_mesh::kFewRays) {
+    if (!m->few) BVHC_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&m->few), sizeof(bvhc_mesh::Few)));
+    bvhc_mesh::Few& f = *m->few;
+    std::memcpy(f.rays, rays, n * 24);
+    BVHC_CUDA_TRY(dispatch_first(m, f.rays, n, side, tab, near_d, far_d, f.hits, m->d_work, s));
+    BVHC_CUDA_TRY(cudaMemcpyAsync(&f.err, m->d_err, sizeof f.err, cudaMemcpyDeviceToHost, s));
+    BVHC_CUDA_TRY(cudaStreamSynchronize(s));
+    std::memcpy(out, f.hits, n * sizeof(bvhc_hit));
+    return f.err ? read_and_clear_error(m, s) : BVHC_OK;
   }
   if (n <= kPipeChunk) {
     BVHC_CUDA_TRY(ensure(&m->d_in, &m->in_cap, n * 24));

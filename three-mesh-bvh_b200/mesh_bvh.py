@@ -425,7 +425,8 @@ class MeshBVH:
             a, b, c = (int(v) for v in self.geometry.index[base:base + 3])
         else:
             a, b, c = base, base + 1, base + 2
-        n = np.cross(tri[2] - tri[1], tri[0] - tri[1])       # Triangle.getNormal
+        u, v = tri[2] - tri[1], tri[0] - tri[1]              # Triangle.getNormal (np.cross takes 15 us)
+        n = np.array([u[1] * v[2] - u[2] * v[1], u[2] * v[0] - u[0] * v[2], u[0] * v[1] - u[1] * v[0]])
         ln = float(np.dot(n, n))
         n = n / math.sqrt(ln) if ln > 0 else np.zeros(3)
         bary = np.array(rec["barycoord"], dtype=np.float64)
