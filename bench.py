@@ -233,7 +233,8 @@ def traversal_kernel(cfg):
     p = 1 if cfg is None else cfg[0]
     if p == 2 and cfg is not None and len(cfg) > 7 and cfg[7]:
         return "raycast_first_packet4_kernel"
-    return {0: "raycast_first_kernel", 1: "raycast_first_persistent_kernel", 2: "raycast_first_packet_kernel"}[p]
+    # the persistent form's kernel for batches of more than 131,072 rays
+    return {0: "raycast_first_kernel", 1: "raycast_first_phased_kernel", 2: "raycast_first_packet_kernel"}[p]
 
 
 def kernel_launches(cfg):
@@ -686,7 +687,7 @@ def run_batched(args, ws, rank, local):
 
 
 def closest_launches(variant: int) -> int:
-    """Kernels one closestPointToPoint call launches: the traversal (per query or warp-cooperative)
+    """Kernels one closestPointToPoint call launches: the traversal (lane groups or warp-cooperative)
     and the finalize kernel, after the query box, the Morton keys and a three-pass radix sort
     (three kernels a pass) for the sorted forms."""
     if variant == 0:
@@ -772,7 +773,7 @@ def run_closest(args, ws, rank, local):
                 "traffic": None, "peak_source": how, "algorithmic_bytes_per_launch": n * per_query,
                 "reference_node_reads_per_query": float(nn.mean()),
                 "reference_triangle_tests_per_query": float(nt.mean()),
-                "kernel": "closest_point_kernel" if tuned["setting"]["closest"] == 0 else "closest_point_packet_kernel"}
+                "kernel": "closest_point_group_kernel" if tuned["setting"]["closest"] == 0 else "closest_point_packet_kernel"}
         prof = "closest_point_k3.md"
         roof["issue"] = {"source": f"profiles/{prof}",
                          "warp_instructions_per_query": profile_value(prof, "warp_instructions_per_query"),
@@ -1160,7 +1161,7 @@ def run_scene(args, ws, rank, local):
                         "h2d_bytes_per_step": int(rays_h.nbytes), "d2h_bytes_per_step": int(n_rays * 36)},
                 "roofline": None, "roofline_note": "two-level traversal (instance tree, then a geometry tree per "
                 "entered instance box) is latency-bound", "cpu_baseline": cpu, "clocks": clk.summary(),
-                "gpu_launches": args.steps * (1 if best_order == 0 else 6)}
+                "gpu_launches": args.steps * (2 if best_order == 0 else 7)}
         print(json.dumps(line), flush=True)
     scene.dispose()
     batch.dispose()

@@ -146,12 +146,17 @@ bvhc_status bvhc_mesh_create(int device, int version, const void* const* roots, 
 void bvhc_mesh_destroy(bvhc_mesh* mesh);
 bvhc_status bvhc_mesh_get_info(const bvhc_mesh* mesh, bvhc_mesh_info* info);
 /* Traversal variant used by this mesh's raycastFirst calls (no reference counterpart: the
- * reference has one recursive traversal).  persistent = 1 runs a grid of resident warps that
- * refill idle lanes from a work counter once `refill` (1..32) lanes are idle; 0 runs one ray per
+ * reference has one recursive traversal).  persistent = 1 walks four-child records (collapsed
+ * from raycastFirst's child pairs, same leaves; children nearest first) with as many lanes per ray as
+ * the batch leaves idle: a warp for up to 24,576 rays, four lanes for up to 131,072, else one, in
+ * resident warps that refill idle lanes from a work counter; a tree too deep for those records' stack
+ * (or whose boxes do not nest) is walked over child pairs by resident warps that refill once `refill`
+ * (1..32) lanes are idle.  0 runs one ray per
  * thread; 2 runs the 32 rays of a warp through one shared traversal (for coherent rays such as a
  * camera's).  Batched launches always use the persistent form.  order = 0 visits the near child
  * by the sign of the ray direction on the split axis (the reference's order), 1 by the smaller
- * entry distance.  occupancy selects the register budget of the persistent and warp-cooperative
+ * entry distance (persistent = 0 and 2 over child pairs; elsewhere nearest first).  occupancy selects
+ * the register budget of the warp-cooperative
  * kernels: 0 the compiler's choice, 1 at least six and 2 at least eight resident 128-thread
  * blocks per SM.  compact = 1
  * (persistent = 1 or 2) first finishes, in one coalesced pass, the rays that miss every root's
@@ -159,14 +164,13 @@ bvhc_status bvhc_mesh_get_info(const bvhc_mesh* mesh, bvhc_mesh_info* info);
  * the compaction pass) orders the remaining rays by a Morton key before the traversal: 1 the ray
  * direction (cube-map coordinates), 2 the point where the ray enters the mesh's bounding box, 3
  * that point (coarser) followed by the direction; 0 keeps the input order.  wide = 1 makes the
- * warp-cooperative and persistent forms (and batched launches) walk four-child records (collapsed
- * from raycastFirst's child pairs, same leaves; children taken nearest first, 64-entry stack).
- * closest selects closestPointToPoint's kernel: 0 one query per thread, 1 the 32 queries of a warp
- * through one shared traversal (for spatially coherent queries such as grids), 2 the same over the
- * queries sorted by a Morton key of the point, 3 and 4 as 1 and 2 with groups of 16 consecutive
- * queries (two shared traversals per warp), 5 and 6 with groups of 8; 1 to 6 apply with
- * minThreshold 0 (otherwise 0 runs), and use the occupancy setting too; 1, 3 and 5 also read the
- * queries in tiled order when `tile` is set (rows of `tile` points, e.g. a grid's row).
+ * warp-cooperative form walk four-child records (64-entry stack); the persistent form always does.
+ * closest selects closestPointToPoint's kernel: 0 the queries in input order over four-child records
+ * (a warp per query for up to 200,000, else four lanes), 1 the same unless `tile` is set, in which case
+ * the 32 queries of a warp (a tile of the rows of `tile` points, e.g. a grid's row) go
+ * through one shared traversal, 2 one shared traversal for the 32 queries of a warp over the
+ * queries sorted by a Morton key of the point; 3 and 5 run as 1, 4 and 6 as 2.  With a
+ * minThreshold above 0, and for trees without four-child records, one query per thread runs.
  * All forms return the same bytes.  all selects raycast's
  * (all hits) kernel: 0 one ray per thread, 1 the rays of a warp through one shared left-first
  * traversal (each ray's hits stay in the reference's DFS order), 2, 3 and 4 the same over the rays

@@ -38,16 +38,17 @@ cudaError_t launch_raycast_first(const MeshDev& m, const float* rays, uint64_t n
 inline int tile_rows_log2(int rows) { return rows == 2 ? 1 : rows == 8 ? 3 : 2; }
 
 struct TraversalConfig {
-  int persistent;  // 1: persistent warps with lane refill; 0: one ray per thread; 2: warp-cooperative
+  int persistent;  // 1: four-child records, a warp, four lanes or one lane per ray by the batch's size;
+                   // 0: one ray per thread; 2: warp-cooperative
   int order;       // 0: split-axis direction sign (reference order); 1: nearest entry first
-  int refill;      // idle lanes (1..32) that trigger a refill in the persistent form
-  int occupancy;   // persistent form register budget: 0 compiler's choice, 1 six blocks/SM, 2 eight
+  int refill;      // idle lanes (1..32) that trigger a refill in the persistent form over child pairs
+  int occupancy;   // warp-cooperative register budget: 0 compiler's choice, 1 six blocks/SM, 2 eight
   int compact;     // 1 runs the root-box pre-pass and traverses only queued rays (persistent and
                    // warp-cooperative forms)
   int sort;        // 0: queue in ray order; 1..3: queue sorted by a Morton key (raysort.cu), implies
                    // the pre-pass
-  int closest;     // closestPointToPoint: 0 one query per thread, 1 warp-cooperative, 2 warp-cooperative
-                   // over Morton-sorted queries (1 and 2 only with minThreshold 0)
+  int closest;     // closestPointToPoint: 0 a warp or four lanes per query, 1 (3, 5) the same unless
+                   // tiled, then warp-cooperative, 2 (4, 6) warp-cooperative over Morton-sorted queries
   int wide;        // warp-cooperative raycastFirst: 1 walks the four-child records
   int all;         // raycast (all hits): 0 one ray per thread, 1 warp-cooperative, 2..4 warp-cooperative
                    // over the rays that enter the tree, sorted by key kind all - 1, 5..8 one ray per

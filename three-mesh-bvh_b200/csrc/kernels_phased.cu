@@ -18,7 +18,7 @@ namespace dev {
 // What bounds it: instructions issued with part of the lanes (about 18 of 32 in a node step and 16 in
 // a leaf step, where descending each lane to its next leaf gave 5.5 in all) and the L1's wavefronts, one
 // per lane and load when the lanes are at different records.  1,000,000 rays on the 80,000-triangle
-// knot: 1780 us over child pairs, 585 us here (365 instead of 790 warp instructions a ray; two pending
+// knot: 1780 us over child pairs, 600 us here (365 instead of 790 warp instructions a ray; two pending
 // leaves against none 6%, sorted children against only the nearest first 6%, the stack's first
 // twelve entries in shared memory 7%: in thread-local memory lanes at different depths each cost a
 // wavefront).
