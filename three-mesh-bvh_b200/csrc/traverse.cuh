@@ -124,21 +124,38 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
 // rounding of o inv and of the sum) plus 5u (|o| + |c| + h) |inv| (radius and final sum) of t_c -+ r;
 // the half extent's slack of 16u (|c| + h) and s = 16u |o| |inv| cover that, so entry and exit here
 // lie outside the exact ones.
+// That takes an o inv that is finite.  A zero direction component has 1 / kTiny for its inv, and an origin
+// beyond 2^126 kTiny takes 2^126 / |o| in its place: any finite number serves that is large enough that a
+// box's planes are behind or far ahead.  (t_c can be infinite still, for a box beside the ray; where the ray
+// is between the box's planes, |c - o| <= h, r is as large, and t_c -+ r a NaN or an infinity that lets the
+// box in.)  Another component whose o inv overflows (a direction far from unit length) rules no box out: s
+// is infinite.  An infinite o stays as it comes out: every box is missed.
+__device__ __forceinline__ void slab_axis(float o, float d, float& inv, float& noi, float& s) {
+  const float ao = fabsf(o);
+  if (d == 0.0f && ao > 0x1p126f * kTiny) inv = copysignf(fmaxf(0x1p126f * rcp_fast(ao), 0.125f), inv);
+  noi = -o * inv;
+  s = 0x1p-20f * ao * fabsf(inv);
+  if (fabsf(noi) == kInf && ao < kInf) {
+    noi = 0.0f;
+    s = kInf;
+  }
+}
 struct RaySlab {
   f2 inv, noi, ainv, s;          // x, y
   float invz, noiz, ainvz, sz;
 };
 __device__ __forceinline__ RaySlab ray_slab(const RayF& r) {
   RaySlab q;
-  const float ax = fabsf(r.inv.x), ay = fabsf(r.inv.y);
-  q.inv = f2_make(r.inv.x, r.inv.y);
-  q.noi = f2_make(-r.o.x * r.inv.x, -r.o.y * r.inv.y);
-  q.ainv = f2_make(ax, ay);
-  q.s = f2_make(0x1p-20f * fabsf(r.o.x) * ax, 0x1p-20f * fabsf(r.o.y) * ay);
+  float ix = r.inv.x, iy = r.inv.y, nx, ny, sx, sy;
   q.invz = r.inv.z;
-  q.noiz = -r.o.z * r.inv.z;
-  q.ainvz = fabsf(r.inv.z);
-  q.sz = 0x1p-20f * fabsf(r.o.z) * q.ainvz;
+  slab_axis(r.o.x, r.d.x, ix, nx, sx);
+  slab_axis(r.o.y, r.d.y, iy, ny, sy);
+  slab_axis(r.o.z, r.d.z, q.invz, q.noiz, q.sz);
+  q.inv = f2_make(ix, iy);
+  q.noi = f2_make(nx, ny);
+  q.ainv = f2_make(fabsf(ix), fabsf(iy));
+  q.s = f2_make(sx, sy);
+  q.ainvz = fabsf(q.invz);
   return q;
 }
 
