@@ -25,10 +25,7 @@ __device__ __forceinline__ RayF ray_from(float3 o, float3 d) {
   RayF r;
   r.o = o;
   r.d = d;
-  const float dx = fabsf(d.x) < kTiny ? copysignf(kTiny, d.x) : d.x;
-  const float dy = fabsf(d.y) < kTiny ? copysignf(kTiny, d.y) : d.y;
-  const float dz = fabsf(d.z) < kTiny ? copysignf(kTiny, d.z) : d.z;
-  r.inv = make_float3(rcp_fast(dx), rcp_fast(dy), rcp_fast(dz));
+  r.inv = ray_reciprocals(o, d);
   r.dk = kFilterK * (fabsf(d.x) + fabsf(d.y) + fabsf(d.z));
   return r;
 }

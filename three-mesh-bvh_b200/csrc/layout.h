@@ -88,15 +88,16 @@ __host__ __device__
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-    // One axis of a box as centre and half extent.  The half extent carries 2^-20 (|c| + h) of slack:
-    // its own two roundings and the ray test's error in c (kernels' slab test) are under 8u (|c| + h),
-    // u = 2^-24.  Swapped bounds count as the box between them, as in the slab test with minimum and
-    // maximum; bounds that are not numbers, or too large, give an unbounded axis.
+    // One axis of a box as centre and half extent.  The half extent reaches the farther bound (a difference
+    // of float32 values, rounded once) and carries 64u of itself, u = 2^-24, for the ray test (traverse.cuh's
+    // slab_axis), or more where that is lost below 2^-126.  Swapped bounds count as the box between them, as
+    // in the slab test with minimum and maximum; bounds that are not numbers, or too large, give an
+    // unbounded axis.
     inline void box_centre_half(float lo, float hi, float& c, float& h) {
   c = 0.5f * lo + 0.5f * hi;
   const float a = hi - c, b = c - lo;
-  const float aa = a < 0.0f ? -a : a, ab = b < 0.0f ? -b : b, ac = c < 0.0f ? -c : c;
-  h = (aa > ab ? aa : ab) * (1.0f + 9.5367431640625e-07f) + ac * 9.5367431640625e-07f;
+  const float aa = a < 0.0f ? -a : a, ab = b < 0.0f ? -b : b;
+  h = (aa > ab ? aa : ab) * (1.0f + 3.814697265625e-06f) + 7.174648137343064e-43f;
   if (!(aa < kBoxUnbounded && ab < kBoxUnbounded && h < kBoxUnbounded)) {
     c = 0.0f;
     h = kBoxUnbounded;
