@@ -777,50 +777,41 @@ static void free_quads(bvhc_mesh::QuadSet& q) {
   q = bvhc_mesh::QuadSet{};
 }
 
-// The ray traversals' records over a child-pair layout (already on the device), into set `k`, replacing
-// any before.  A mesh with more triangle records than a run link can name has no four-child records:
-// the child-pair kernels run.
-static cudaError_t install_quads(bvhc_mesh* m, int k, const std::vector<PairNode>& pairs,
-                                 const std::vector<TriRecord>& tris, const std::vector<uint32_t>& roots) {
-  free_quads(m->quad_set[k]);
-  bvhc_mesh::QuadSet q;
+// The ray traversals' records over a child-pair layout (`nodes` and `recs` on the device), into the empty
+// set `q`; with_boxes: also in the lo / hi form.  A mesh with more triangle records than a run link can name
+// has no four-child records, nor has a tree whose boxes do not nest: the child-pair kernels run.
+static cudaError_t make_quads(bvhc_mesh::QuadSet& q, bool with_boxes, const PairNode* nodes, const TriRecord* recs,
+                              const std::vector<PairNode>& pairs, const std::vector<TriRecord>& tris,
+                              const std::vector<uint32_t>& roots) {
   q.n_pairs = pairs.size();
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&q.ray_pairs), std::max<size_t>(pairs.size(), 1) * sizeof(RayPair));
-  if (e == cudaSuccess) e = launch_ray_pairs(k ? m->d_nodes_f : m->d_nodes, q.n_pairs, q.ray_pairs, nullptr);
-  if (e != cudaSuccess) {
-    free_quads(q);
-    return e;
-  }
-  m->quad_set[k] = q;
-  if (tris.size() >= kRunFirst) return cudaStreamSynchronize(nullptr);
+  if (e == cudaSuccess) e = launch_ray_pairs(nodes, q.n_pairs, q.ray_pairs, nullptr);
   QuadBuilder qb{pairs, tris};
-  std::vector<uint32_t> qroots(roots.size());
-  try {
+  std::vector<uint32_t> qroots;
+  if (e == cudaSuccess && tris.size() < kRunFirst) try {
+    qroots.resize(roots.size());
     if (tris.size() > 50000) qb.defer = roots.size() > 64 ? 0 : 3;  // 1 or 64 subtrees a root and up
     for (size_t r = 0; r < roots.size(); ++r) qroots[r] = qb.root(roots[r]);
     qb.finish();
   } catch (const Status&) {
-    return cudaErrorInvalidValue;
+    e = cudaErrorInvalidValue;
   } catch (const std::bad_alloc&) {
-    return cudaErrorMemoryAllocation;
+    e = cudaErrorMemoryAllocation;
   }
-  if (!qb.nested) return cudaStreamSynchronize(nullptr);  // the child-pair kernels take such a tree
-  e = upload(&q.quads, qb.quads);
-  if (e == cudaSuccess) e = upload(&q.roots, qroots);
-  if (e == cudaSuccess) e = upload(&q.src, qb.src);
-  q.n = qb.quads.size();
-  q.stack = qb.stack;
-  if (k == 0) {
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&q.boxes), q.n * sizeof(BoxNode));
-    if (e == cudaSuccess) e = launch_quad_boxes(q.quads, q.n, q.src, m->d_nodes, m->d_tris, q.boxes, nullptr);
+  if (e == cudaSuccess && !qroots.empty() && qb.nested) {
+    e = upload(&q.quads, qb.quads);
+    if (e == cudaSuccess) e = upload(&q.roots, qroots);
+    if (e == cudaSuccess) e = upload(&q.src, qb.src);
+    q.n = qb.quads.size();
+    q.stack = qb.stack;
+    if (with_boxes) {
+      if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&q.boxes), q.n * sizeof(BoxNode));
+      if (e == cudaSuccess) e = launch_quad_boxes(q.quads, q.n, q.src, nodes, recs, q.boxes, nullptr);
+    }
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-  m->quad_set[k] = q;
-  if (e != cudaSuccess) {
-    free_quads(m->quad_set[k]);
-    return e;
-  }
-  return cudaSuccess;
+  if (e != cudaSuccess) free_quads(q);
+  return e;
 }
 
 // 3 vertex ids per triangle on the device, from the geometry index (or 3t + k without one).
@@ -1066,7 +1057,8 @@ bvhc_status bvhc_mesh_create(int device, int version, const void* const* roots, 
   bvhc_status st = finish_mesh(device, pairs, tris, root_links, max_depth, {}, out);
   if (st == BVHC_OK) {
     keep_serialized(*out, std::move(copies), std::move(slot_nodes), index, index_elem_bytes, index_count, n_verts);
-    cudaError_t e = install_quads(*out, 0, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
+    bvhc_mesh* m = *out;
+    cudaError_t e = make_quads(m->quad_set[0], true, m->d_nodes, m->d_tris, m->h_pairs, m->h_tris, m->h_roots);
     if (e != cudaSuccess) {
       bvhc_mesh_destroy(*out);
       *out = nullptr;
@@ -1131,7 +1123,8 @@ bvhc_status bvhc_batch_create(int device, int n_meshes, const int32_t* roots_per
   bvhc_status st = finish_mesh(device, pairs, tris, root_links, max_depth, mesh_root_off, out);
   if (st == BVHC_OK) {
     keep_serialized(*out, std::move(copies), std::move(slot_nodes), index, index_elem_bytes, index_count, n_verts);
-    cudaError_t e = install_quads(*out, 0, (*out)->h_pairs, (*out)->h_tris, (*out)->h_roots);
+    bvhc_mesh* m = *out;
+    cudaError_t e = make_quads(m->quad_set[0], true, m->d_nodes, m->d_tris, m->h_pairs, m->h_tris, m->h_roots);
     if (e != cudaSuccess) {
       bvhc_mesh_destroy(*out);
       *out = nullptr;
@@ -1351,14 +1344,28 @@ bvhc_status bvhc_mesh_set_leaf_size(bvhc_mesh* m, int max_leaf) {
   }
   BVHC_CUDA_TRY(cudaSetDevice(m->device));
   BVHC_CUDA_TRY(cudaDeviceSynchronize());  // no launch may still read the old records
+  // all of the new layout is made before any of the old one goes
   PairNode* nodes = nullptr;
   TriRecord* recs = nullptr;
   uint32_t* rts = nullptr;
+  RefitPlan plan;
+  bvhc_mesh::QuadSet quads;
+  std::vector<uint32_t> faces;
   if (max_leaf > 0) {
     cudaError_t e = upload(&nodes, pairs);
     if (e == cudaSuccess) e = upload(&recs, tris);
     if (e == cudaSuccess) e = upload(&rts, roots);
+    try {
+      faces.resize(tris.size());
+      for (size_t k = 0; k < tris.size(); ++k) faces[k] = tris[k].face;
+      if (e == cudaSuccess && !m->h_root_bytes.empty())  // so that a refit keeps this copy in step
+        e = build_refit_plan(pairs, tris, roots, serialized_root_boxes(m), plan);
+    } catch (const std::bad_alloc&) {
+      e = cudaErrorMemoryAllocation;
+    }
+    if (e == cudaSuccess) e = make_quads(quads, false, nodes, recs, pairs, tris, roots);
     if (e != cudaSuccess) {
+      free_refit_plan(plan);
       cudaFree(nodes);
       cudaFree(recs);
       cudaFree(rts);
@@ -1368,20 +1375,18 @@ bvhc_status bvhc_mesh_set_leaf_size(bvhc_mesh* m, int max_leaf) {
   cudaFree(m->d_nodes_f);
   cudaFree(m->d_tris_f);
   cudaFree(m->d_roots_f);
+  free_refit_plan(m->refit[1]);
+  free_quads(m->quad_set[1]);
   m->d_nodes_f = nodes;
   m->d_tris_f = recs;
   m->d_roots_f = rts;
   m->n_nodes_f = pairs.size();
   m->n_tris_f = tris.size();
   m->max_depth_f = depth;
-  m->rec_face_f.resize(tris.size());
-  for (size_t k = 0; k < tris.size(); ++k) m->rec_face_f[k] = tris[k].face;
+  m->rec_face_f = std::move(faces);
+  m->refit[1] = plan;
+  m->quad_set[1] = quads;
   m->leaf_size = max_leaf;
-  free_refit_plan(m->refit[1]);
-  if (max_leaf > 0 && !m->h_root_bytes.empty())  // so that a refit keeps this copy in step
-    BVHC_CUDA_TRY(build_refit_plan(pairs, tris, roots, serialized_root_boxes(m), m->refit[1]));
-  if (max_leaf > 0) BVHC_CUDA_TRY(install_quads(m, 1, pairs, tris, roots));
-  else free_quads(m->quad_set[1]);
   return BVHC_OK;
 }
 

@@ -358,6 +358,7 @@ static cudaError_t traverse_all(const MeshDev& m, const float* rays, uint64_t n,
                                                                       counts, hits, queue, qcount);
     return cudaGetLastError();
   }
+  if (!m.ray_pairs) return cudaErrorInvalidValue;
   if (variant == 2) {
     // the root-box pre-pass gives the rays that miss a count of 0 and queues the others with their
     // keys, which are then sorted

@@ -286,6 +286,7 @@ cudaError_t launch_raycast_first_packet(const MeshDev& m, const float* rays, uin
                                         const TraversalConfig& cfg, cudaStream_t stream, uint32_t* queue,
                                         unsigned int* qcount, const RaySort* sort) {
   if (n == 0) return cudaSuccess;
+  if (!m.ray_pairs) return cudaErrorInvalidValue;
   const bool compact = queue != nullptr && qcount != nullptr && n < (1ull << 32);
   if (compact) {
     cudaError_t e = prepare_queue(m, nullptr, rays, n, near_d, far_d, out, queue, qcount, sort, stream);
