@@ -125,6 +125,27 @@ __device__ __forceinline__ Nearest nearest_none() {
   return {kInf, 0.0f, kNoRecord, 0u, make_float3(0.f, 0.f, 0.f), 0};
 }
 
+// A candidate whose float32 closest point is 0 / 0, or may be.  Where the first two corners coincide (a zero
+// denominator on their edge) it is in the reference's arithmetic too, unless another region is nearest, and
+// the reference then does not take the triangle: d2 is not a number.  Elsewhere float32 has underflowed.
+static __device__ __noinline__ Candidate candidate_slow(float3 p, float3 a, float3 b, float3 c) {
+  const CPFF e = closest_ff(p, a, b, c);
+  Candidate r;
+  r.d2 = e.d2.hi;
+  r.err = fabsf(e.d2.hi) * 0x1p-40f + 1e-37f;
+  r.q = make_float3(ff_to_f(e.q.x), ff_to_f(e.q.y), ff_to_f(e.q.z));
+  return r;
+}
+__device__ __forceinline__ bool no_first_edge(const Tri& t) {
+  return t.a.x == t.b.x && t.a.y == t.b.y && t.a.z == t.b.z;
+}
+
+// Whether squared distance d of faceIndex fd goes before e of fe: nearer, or an exact tie and the smaller
+// faceIndex.  What is not a number goes before nothing.
+__device__ __forceinline__ bool nearer(ff d, uint32_t fd, ff e, uint32_t fe) {
+  return ff_lt(d, e) || (d.hi == e.hi && d.lo == e.lo && fd < fe) || (e.hi != e.hi && d.hi == d.hi);
+}
+
 // Whether candidate `cand` beats `b` where their float32 distances do not tell: the same vertex is an
 // exact tie, else the float-float distances decide; an exact tie goes to the smaller faceIndex.
 static __device__ __noinline__ bool closer_slow(const TriRecord* __restrict__ tris, float3 p, uint32_t cand,
@@ -132,8 +153,7 @@ static __device__ __noinline__ bool closer_slow(const TriRecord* __restrict__ tr
   const Tri t = load_tri(tris, cand & kRunFirst), u = load_tri(tris, b & kRunFirst);
   const uint32_t tv = cand >> kRunShift, uv = b >> kRunShift;
   if (tv != 3u && uv != 3u && same_vertex(t, tv, u, uv)) return t.face < u.face;
-  const ff d = closest_ff(p, t.a, t.b, t.c).d2, e = closest_ff(p, u.a, u.b, u.c).d2;
-  return ff_lt(d, e) || (!ff_lt(e, d) && t.face < u.face);
+  return nearer(closest_ff(p, t.a, t.b, t.c).d2, t.face, closest_ff(p, u.a, u.b, u.c).d2, u.face);
 }
 
 // Offers triangle t (record k) at candidate c to a lane's best.  Candidates are ranked by exact distance,
@@ -142,7 +162,12 @@ static __device__ __noinline__ bool closer_slow(const TriRecord* __restrict__ tr
 // overtaken by a nearer triangle later in the walk, and float-float code in the loop is fetched and
 // executed by whole warps for one lane.
 __device__ __forceinline__ void offer_closest(const TriRecord* __restrict__ tris, float3 p, const Tri& t, uint32_t k,
-                                              const Candidate& c, Nearest& b, uint2 (*s_tie)[kBlock]) {
+                                              Candidate c, Nearest& b, uint2 (*s_tie)[kBlock]) {
+  if (c.d2 - c.err > b.d2 + b.err) return;
+  if (no_first_edge(t) || c.d2 != c.d2) {
+    c = candidate_slow(p, t.a, t.b, t.c);
+    if (!(c.d2 < kInf)) return;
+  }
   const float hi = c.d2 + c.err, lo = c.d2 - c.err;
   bool take = b.rec == kNoRecord ? c.d2 < kInf : hi < b.d2 - b.err;
   uint32_t rec = kNoRecord;

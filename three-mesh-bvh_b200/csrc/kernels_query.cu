@@ -57,11 +57,16 @@ __device__ __forceinline__ void cp_offer(const MeshDev& m, float3 p, const Tri& 
   // |error| of each closest-point coordinate <= e (local-frame evaluation)
   float e = 32.0f * kU * sc;
   err = 3.5f * e * sqrtf(d2) + 3.0f * e * e;
-  bool is_vertex = (q.x == t.a.x && q.y == t.a.y && q.z == t.a.z) ||
-                   (q.x == t.b.x && q.y == t.b.y && q.z == t.b.z) ||
-                   (q.x == t.c.x && q.y == t.c.y && q.z == t.c.z);
-  bool take;
   have_ff = false;
+  if (no_first_edge(t) || d2 != d2) {
+    const Candidate c = candidate_slow(p, t.a, t.b, t.c);
+    d2 = c.d2;
+    err = c.err;
+    q = c.q;
+    if (!(d2 < kInf)) return;
+  }
+  const bool is_vertex = vertex_of(t, q) != 3u;
+  bool take;
   if (b.rec == 0xFFFFFFFFu) {
     take = d2 < kInf;  // the first finite candidate (distSq < Infinity)
   } else if (d2 + err < b.d2 - b.err) {
@@ -83,7 +88,7 @@ __device__ __forceinline__ void cp_offer(const MeshDev& m, float3 p, const Tri& 
     }
     cand_ff = closest_ff(p, t.a, t.b, t.c).d2;
     have_ff = true;
-    take = ff_lt(cand_ff, b.ffv) || (!ff_lt(b.ffv, cand_ff) && t.face < b.face);
+    take = nearer(cand_ff, t.face, b.ffv, b.face);
   }
   if (take) {
     b.d2 = d2;
@@ -235,7 +240,7 @@ __global__ void __launch_bounds__(kBlock) closest_point_finalize_kernel(MeshDev 
     const Tri u = load_tri(m.tris, cand & kRunFirst);
     const ff e = s_d2[k][threadIdx.x];
     const bool same = cv != 3u && vertex != 3u && same_vertex(t, vertex, u, cv);
-    if (same ? u.face < t.face : ff_lt(e, d2) || (!ff_lt(d2, e) && u.face < t.face)) {
+    if (same ? u.face < t.face : nearer(e, u.face, d2, t.face)) {
       t = u;
       vertex = cv;
       d2 = e;
