@@ -1,6 +1,6 @@
-"""closestPointToPoint on meshes with triangles whose first two corners coincide: the closest point on their
-first edge is 0 / 0 where that edge is the nearest region, in the reference's arithmetic too, which then does not
-take them.  Every form against the oracle, whatever lane meets them first."""
+"""closestPointToPoint on meshes with triangles two of whose corners coincide: with the first two, the closest
+point on their first edge is 0 / 0 where that edge is the nearest region, in the reference's arithmetic too, which
+then does not take them; with the last two they are segments.  Every form against the oracle, whatever lane meets them first."""
 import math
 
 import numpy as np
@@ -10,13 +10,13 @@ pytestmark = pytest.mark.gpu
 
 
 def _mesh(pkg, only):
-    """A knot with a quarter of its triangles (the lowest face indices among them) degenerate: a = b, a = c
-    or all three; or nothing but a = b."""
+    """A knot with a quarter of its triangles (the lowest face indices among them) degenerate: a = b, b = c,
+    a = c, or all three; or nothing but a = b."""
     g = pkg.torus_knot(10, 3, 60, 12, noise_sigma=0.05, noise_seed=3)
     tri = g.index.reshape(-1, 3).copy()
     k = np.arange(len(tri))
     pick = np.ones(len(tri), bool) if only else (k < 40) | (k % 5 == 0)
-    kind = np.zeros(len(tri), int) if only else np.where(k % 2 == 0, 0, 2 + k % 7 % 2)
+    kind = np.zeros(len(tri), int) if only else np.where(k % 2 == 0, 0, 1 + k % 7 % 3)
     for which, (to, of) in enumerate(((1, 0), (2, 1), (2, 0))):
         rows = pick & (kind == which)
         tri[rows, to] = tri[rows, of]

@@ -262,7 +262,7 @@ __device__ __forceinline__ float closest_sq_f(float3 p, float3 a, float3 b, floa
   float cpx = apx - acx, cpy = apy - acy, cpz = apz - acz;
   float d5 = abx * cpx + aby * cpy + abz * cpz;
   float d6 = acx * cpx + acy * cpy + acz * cpz;
-  float vc = d1 * d4 - d3 * d2;
+  float vc = __fmul_rn(d1, d4) - __fmul_rn(d3, d2);  // zero where b = c
   float vb = d5 * d2 - d1 * d6;
   float va = d3 * d6 - d5 * d4;
   if (d1 <= 0.0f && d2 <= 0.0f) {
@@ -319,7 +319,9 @@ static __device__ __noinline__ CPFF closest_ff(float3 p, float3 a, float3 b, flo
     l = ab;
     wb = 1.0f;
   } else {
-    ff vc = ff_sub(ff_mul(d1, d4), ff_mul(d3, d2));
+    // zero where b = c (a segment, met on its edge a b); the products' low parts do not round alike
+    const bool segment = b.x == c.x && b.y == c.y && b.z == c.z;
+    ff vc = segment ? zero : ff_sub(ff_mul(d1, d4), ff_mul(d3, d2));
     if (ff_sign(vc) <= 0 && ff_sign(d1) >= 0 && ff_sign(d3) <= 0) {
       ff v = ff_div(d1, ff_sub(d1, d3));
       l = ff3_scale(ab, v);
