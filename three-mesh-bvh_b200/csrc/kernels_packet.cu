@@ -298,7 +298,8 @@ cudaError_t launch_raycast_first_packet(const MeshDev& m, const float* rays, uin
   // the tiled order applies to the whole ray range (a queue is already in its own order)
   const int rl = tile_rows_log2(cfg.tile_rows);
   const uint64_t pitch = (!queue && cfg.tile >= 8 && cfg.tile % (32 >> rl) == 0) ? (uint64_t)cfg.tile : 0;
-  if (cfg.wide && m.quads && m.quad_roots) {
+  // the four-child form stacks up to three children a step, and gives up where three no longer fit
+  if (cfg.wide && m.quads && m.quad_roots && m.quad_stack + 3 <= kMaxStack) {
     auto k4 = cfg.occupancy == 0   ? dev::raycast_first_packet4_kernel<1>
               : cfg.occupancy == 1 ? dev::raycast_first_packet4_kernel<6>
                                    : dev::raycast_first_packet4_kernel<8>;
