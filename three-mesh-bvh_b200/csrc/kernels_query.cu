@@ -522,7 +522,11 @@ struct ObbS {
   float n1[3];  // L1 norms of the axes
   float mag;    // >= every corner's sum of term magnitudes; 0 when the box is too large (undecided)
   bool exact;   // non-affine matrix: every test goes to binary64
+  bool skew;    // edges not at right angles, or without length (box_f); beside `exact`: a word more costs 3%
 };
+static_assert(sizeof(ObbS) == 200, "eight of them in other banks");
+// By how much of the coordinates' size an aligned axis has to separate a box of the tree, and a part of a leaf.
+constexpr float kApart = 0x1p-20f, kPartApart = 0x1p-14f;
 
 __device__ __forceinline__ float dotf(float3 a, float3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
 __device__ __forceinline__ float l1f(float3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
@@ -578,20 +582,37 @@ __device__ __forceinline__ void make_s(const float* q, ObbS& s) {
     s.amax[d] = mx;
   }
   s.mag = mag < 1e30f ? mag : 0.0f;
+  s.skew = false;
+}
+
+// Whether axes i and i + 1 are at right angles to 2^-20 (a float32 rotation's are to 2^-21) and axis i is not
+// too short to have a direction.
+__device__ __forceinline__ bool right_angle(const ObbS& s, int i) {
+  const float3 a = s.ax[i], b = s.ax[i == 2 ? 0 : i + 1];
+  const float ab = dotf(a, b);
+  return s.n1[i] > kApart * s.mag && ab * ab < 0x1p-40f * dotf(a, a) * dotf(b, b);
 }
 
 // OrientedBox.intersectsBox on a node box: 1 meets, 0 separated, -1 undecided.
-__device__ __forceinline__ int box_f(const ObbS& o, const float* b) {
+// A part of a leaf (apart: kPartApart, or infinite), whose box the reference does not have, may only be dropped where the
+// reference separates every triangle in it.  The box's own axes are among a triangle's axes, so where they
+// separate the part they do.  The aligned axes are not: where the box's edges are not at right angles, or one
+// has no length, the reference's axes leave unseparated what the aligned ones separate, and they drop nothing.
+// At right angles the distance D between the part and the box is that of a vertex, edge or face of the box,
+// whose normals span at most an octant; of the triangle's axes that span its share of it one separates by
+// D / sqrt(3) or more.  The reference takes edges for face normals: at 2^-20 off, that moves the ends of what
+// has a size of 2 sqrt(3) m by less than 2^-16 m, so separation by kPartApart m is enough.
+__device__ __forceinline__ int box_f(const ObbS& o, const float* b, float apart = kApart) {
   float m = o.mag;
   for (int k = 0; k < 6; ++k) m = fmaxf(m, fabsf(b[k]));
   if (!(o.mag > 0.0f) || !(m < 1e30f)) return -1;
   // aligned bounds: |error| <= 3.01 u M + 2 u m
-  const float md = 0x1p-20f * m + 0x1p-120f;
+  const float md = kApart * m + 0x1p-120f, ms = apart * m + 0x1p-120f;
   bool undecided = false;
   for (int d = 0; d < 3; ++d) {
-    const int r = sep_f(o.amin[d], o.amax[d], b[d], b[d + 3], md);
-    if (r == 1) return 0;
-    undecided |= r < 0;
+    const float d1 = o.amin[d] - b[d + 3], d2 = b[d] - o.amax[d];
+    if (d1 > ms || d2 > ms) return 0;
+    undecided |= !(d1 < -md && d2 < -md);
   }
   // the node box's interval on a box axis is sum_d min / max(a_d lo_d, a_d hi_d) (the extremes
   // over its 8 corners); |error| <= |a|_1 (6.02 u B + 9.02 u M)
@@ -1058,6 +1079,7 @@ struct SphereShape {
   ff r2;
   float lim;
   static __device__ __forceinline__ void stage(const float*, Shared&) {}
+  static __device__ __forceinline__ void restage(Shared&, unsigned) {}
   __device__ __forceinline__ void start(const float* __restrict__ q, const Shared&) {
     const float4 v = ld4(q);
     c = make_float3(v.x, v.y, v.z);
@@ -1117,7 +1139,8 @@ struct BoxShape {
   using Shared = obb::ObbS;  // in shared memory: 50 words that a lane would keep in registers
   const float* q;
   float3 c;
-  // stage: by the first lane of those that share it; start: by each of them, after a __syncwarp
+  // stage: by the first lane of those that share it; restage: by the next three, after a __syncwarp; start: by
+  // each of them, after another
   static __device__ __forceinline__ void stage(const float* __restrict__ query, Shared& sh) {
     float v[24];
     for (int k = 0; k < 6; ++k) {
@@ -1131,6 +1154,9 @@ struct BoxShape {
     obb::make_s(v, s);
     sh = s;
   }
+  static __device__ __forceinline__ void restage(Shared& sh, unsigned j) {
+    if (!obb::right_angle(sh, (int)j - 1)) sh.skew = true;
+  }
   __device__ __forceinline__ void start(const float* __restrict__ query, const Shared& sh) {
     q = query;
     c = make_float3(0.5f * (sh.p[0].x + sh.p[7].x), 0.5f * (sh.p[0].y + sh.p[7].y), 0.5f * (sh.p[0].z + sh.p[7].z));
@@ -1142,7 +1168,7 @@ struct BoxShape {
     if (n.link == kEmptyLeaf) return 0;
     key = fmaxf(box_score(n.b, c), 0.0f);  // any order where it is not a number
     if (unbounded(n)) return 1;
-    return sh.exact ? -1 : obb::box_f(sh, n.b);
+    return sh.exact ? -1 : obb::box_f(sh, n.b, !n.part ? obb::kApart : sh.skew ? kInf : obb::kPartApart);
   }
   __device__ __forceinline__ int box_slow(const BoxBounds& n, Slow& slow) const {
     return obb_box_slow(q, slow, n.b) ? 1 : 0;
@@ -1205,7 +1231,7 @@ __device__ __forceinline__ uint8_t shape_walk_wide(const MeshDev& m, const Shape
       if (__ballot_sync(full, r > 0)) return 1;
       if (__ballot_sync(full, w != 0)) wide_push(stack, sp, lane, w != 0, link, key, __uint_as_float(below));
       if (Shape::kDoubtful) {
-        lazy += __popc(__ballot_sync(full, w < 0));
+        lazy += __popc(__ballot_sync(full, w < 0 && below != flag));  // of the tree's boxes
         const unsigned open = __ballot_sync(full, r < 0);
         if (SETTLE && open) {
           if (r < 0) doubt[doubts + __popc(open & ((1u << lane) - 1u))] = make_uint2(k, flag);
@@ -1295,6 +1321,8 @@ __global__ void __launch_bounds__(kBlock, kShapeBlocksPerSm) shape_group_kernel(
       const float* query = shapes + (size_t)Shape::kFloats * qid;
       if (starts && j == 0) Shape::stage(query, s_shape[gi]);
       __syncwarp();
+      if (starts && j != 0) Shape::restage(s_shape[gi], j);
+      __syncwarp();
       if (starts) {
         shape.start(query, s_shape[gi]);
         if (Shape::kDoubtful && shape.all_doubts(s_shape[gi])) finish(kPending);
@@ -1354,7 +1382,7 @@ __global__ void __launch_bounds__(kBlock, kShapeBlocksPerSm) shape_group_kernel(
       uint32_t nearest_flag = kNoDoubt;
       if (Shape::kDoubtful) {
         nearest_flag = __shfl_sync(full, child.y, base + first);
-        lazy += __popc((__ballot_sync(full, w < 0) >> base) & 0xFu);
+        lazy += __popc((__ballot_sync(full, w < 0 && child.y != flag) >> base) & 0xFu);  // of the tree's boxes
       }
       if (at_node) {
         const int nh = __popc(hits);
@@ -1419,6 +1447,8 @@ __global__ void __launch_bounds__(kBlock) shape_wide_kernel(MeshDev m, const flo
     const float* query = shapes + (size_t)Shape::kFloats * qid;
     if (lane == 0) Shape::stage(query, s_shape[wi]);
     if (lane == 0) stack[0] = make_uint2(m.quad_roots[0], kNoDoubt);
+    __syncwarp();
+    if (lane - 1u < 3u) Shape::restage(s_shape[wi], lane);
     __syncwarp();
     shape.start(query, s_shape[wi]);
     const bool none = Shape::kDoubtful && shape.all_doubts(s_shape[wi]);
