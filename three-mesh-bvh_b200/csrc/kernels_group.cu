@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kBlock, kGroupBlocksPerSm) raycast_first_group
         best = Best{kInf, 0.0f, 0xFFFFFFFFu};
         lim = RANGED ? slab_far(far_d) : kInf;
         lim_hit = kInf;
-        odd = RANGED && odd_length(r.d);
+        odd = RANGED && free_parts(r.d, near_d);
         int root_end = m.n_roots;
         root = 0;
         if (BATCHED) {

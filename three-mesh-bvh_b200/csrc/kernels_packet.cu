@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_first_packet4_kernel(
   }
   const RaySlab rs = ray_slab(r);
   const float near_s = slab_near(near_d);
-  const bool odd = ranged_call && odd_length(r.d);  // parts of leaves are not held against near and far
+  const bool odd = ranged_call && free_parts(r.d, near_d);  // parts of leaves are not held against near and far
   Best best{kInf, 0.0f, 0xFFFFFFFFu};
   float lane_t[kMaxStack];
   for (int root = 0; root < m.n_roots; ++root) {

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kBlock, kPhasedBlocksPerSm) raycast_first_phas
         best = Best{kInf, 0.0f, 0xFFFFFFFFu};
         lim = RANGED ? slab_far(far_d) : kInf;
         lim_hit = kInf;
-        odd = RANGED && odd_length(r.d);
+        odd = RANGED && free_parts(r.d, near_d);
         root = 0;
         if (BATCHED) {
           const int mesh = mesh_of_ray(bd, rid);

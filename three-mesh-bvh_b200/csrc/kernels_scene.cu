@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(kBlock, kSceneBlocksPerSm) scene_first_phased_
               if (RANGED) {
                 near_s = slab_near(near_l);
                 lim_hit = slab_limit(tlim);
-                odd = odd_length(r.d);
+                odd = free_parts(r.d, near_l);
               }
               lim = slab_far(far_l);
               best = Best{kInf, 0.0f, kNone};

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(kBlock) raycast_first_wide_kernel(MeshDev m, c
     const RayF r = make_ray(rays, rid);
     const RaySlab rs = ray_slab(r);
     const float dlen = sqrtf(r.d.x * r.d.x + r.d.y * r.d.y + r.d.z * r.d.z);
-    const bool odd = ranged_call && odd_length(r.d);
+    const bool odd = ranged_call && free_parts(r.d, near_d);
     int root = 0, root_end = m.n_roots;
     if (batched) {
       const int mesh = mesh_of_ray(bd, rid);

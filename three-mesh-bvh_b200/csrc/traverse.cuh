@@ -172,10 +172,11 @@ __device__ __forceinline__ float slab_far(float far_d) { return far_d < kInf ? s
 // boxes: for a direction that is not of unit length that drops hits by the extent of their leaf's box.
 // Parts of leaves, whose boxes the reference does not have, must then not be held against them: a
 // direction counts as of unit length while the difference is within the slack of the widened limits.
+// Nor against a near that is not a number, which no box of the tree passes but a root that is a leaf does.
 // Calls with near <= 0 and no far have nothing to hold (RANGED false).
 static inline bool ranged(float near_d, float far_d) { return !(near_d <= 0.0f && far_d >= kInf); }
-__device__ __forceinline__ bool odd_length(float3 d) {
-  return !(fabsf(d.x * d.x + d.y * d.y + d.z * d.z - 1.0f) <= 0x1p-20f);
+__device__ __forceinline__ bool free_parts(float3 d, float near_d) {
+  return !(fabsf(d.x * d.x + d.y * d.y + d.z * d.z - 1.0f) <= 0x1p-20f) || near_d != near_d;
 }
 
 struct ChildBox {
