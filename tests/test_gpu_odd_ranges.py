@@ -44,3 +44,19 @@ def test_first_hits(pkg, cuda, mesh, near, far):
                 got = bvh.raycast_first_batch(rays, 2, near, far)
                 bvh.synchronize()
                 assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (n, leaf, kw)
+
+
+@pytest.mark.parametrize("mesh", ["triangle", "leaf40", "plain"])
+@pytest.mark.parametrize("near,far", [(NAN, INF), (0.0, NAN), (NAN, NAN), (0.0, -1.0), (30.0, 10.0), (2.0, 35.0)])
+def test_all_hits(pkg, cuda, mesh, near, far):
+    import torch
+
+    g, opts = _mesh(pkg, mesh)
+    bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH, **opts})
+    rays = torch.from_numpy(_rays(pkg, 20_000)).to(cuda)
+    bvh.set_traversal(all=0)
+    want = bvh.raycast_batch(rays, 2, near, far, cap=4)[0]
+    bvh.set_traversal(all=1)
+    got = bvh.raycast_batch(rays, 2, near, far, cap=4)[0]
+    bvh.synchronize()
+    assert torch.equal(got, want)

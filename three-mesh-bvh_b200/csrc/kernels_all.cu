@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(kBlock, MINB) raycast_all_packet_kernel(
   bvhc_hit* out = hits + i * (uint64_t)cap;
   bool overflow = false;
   const RaySlab rs = ray_slab(r);
-  const float near_s = slab_near(near_d), lim = valid ? slab_far(far_d) : -kInf;  // no ray: enters nothing
+  // no ray, or a far that is not a number: enters nothing
+  const float near_s = slab_near(near_d), lim = valid && far_d == far_d ? slab_far(far_d) : -kInf;
   for (int root = 0; root < m.n_roots && !overflow; ++root) {
     uint32_t link = m.roots[root];
     int sp = 0;
