@@ -26,7 +26,8 @@ __global__ void __launch_bounds__(kBlock) raycast_first_kernel(MeshDev m, const 
     int sp = 0;
     for (;;) {
       if (link & kLeafBit) {
-        if (link != kEmptyLeaf) leaf_first(m, link & ~kLeafBit, r, dlen, side, sides, near_d, far_d, best);
+        if (link != kEmptyLeaf)
+          leaf_first<ORDER == 0>(m, link & ~kLeafBit, r, dlen, side, sides, near_d, far_d, best);
       } else {
         Pair p = load_pair(m.nodes, link);
         float lim = fminf(far_d, (best.t + best.err) * (1.0f + kSlabMargin));

@@ -294,8 +294,9 @@ __device__ __forceinline__ void store_miss(bvhc_hit* p) {
 // ---------------------------------------------------------------------------------------------
 // raycastFirst leaf step shared by both kernel forms.  Candidate hits are ordered with float32 t
 // values and their error bounds; float-float only settles candidates the bounds cannot separate
-// (the reference keeps the strictly closer one; of exact ties, here, the smaller record, which is the
-// one it finds first in left-to-right order).
+// (the reference keeps the strictly closer one; of exact ties, here, the smaller record, which no order of
+// the visits changes.  The form that visits as the reference does, one ray per thread by the direction's
+// sign, keeps the one found first, as the reference does).
 // ---------------------------------------------------------------------------------------------
 constexpr float kTwoU = 1.1920928955078125e-07f;  // 2u
 
@@ -335,7 +336,9 @@ struct Best {
   uint32_t rec;
 };
 
-// Offers triangle record k to `best` in float-float: an exact tie goes to the smaller record.
+// Offers triangle record k to `best` in float-float: an exact tie goes to the smaller record, or with
+// FIRST_FOUND stays with the record found first.
+template <bool FIRST_FOUND = false>
 static __device__ __noinline__ Best offer_slow(const TriRecord* __restrict__ tris, uint32_t k, float3 o, float3 d,
                                                int side, float near_d, float far_d, Best best) {
   ff tn;
@@ -345,12 +348,13 @@ static __device__ __noinline__ Best offer_slow(const TriRecord* __restrict__ tri
   if (!take && !(tn.hi - err > best.t + best.err)) {
     const Tri bt = load_tri(tris, best.rec);
     const ff tb = tri_t_ff(tri_eval_ff(bt.a, bt.b, bt.c, o, d));
-    take = ff_lt(tn, tb) || (!ff_lt(tb, tn) && k < best.rec);
+    take = ff_lt(tn, tb) || (!FIRST_FOUND && !ff_lt(tb, tn) && k < best.rec);
   }
   return take ? Best{tn.hi, err, k} : best;
 }
 
 // Offers triangle record k (loaded as `tr`): the float32 values and bounds decide, else offer_slow.
+template <bool FIRST_FOUND = false>
 __device__ __forceinline__ void offer_first(const MeshDev& m, const Tri& tr, uint32_t k, const RayF& r, float dlen,
                                             int side, float near_d, float far_d, Best& best) {
   float t, t_err;
@@ -359,15 +363,16 @@ __device__ __forceinline__ void offer_first(const MeshDev& m, const Tri& tr, uin
   // none yet: best.t is infinite and its bound 0, so every hit is nearer
   if (st > 0) st = t + t_err < best.t - best.err ? 1 : (t - t_err > best.t + best.err ? 0 : -1);
   if (st > 0) best = Best{t, t_err, k};
-  else if (st < 0) best = offer_slow(m.tris, k, r.o, r.d, side, near_d, far_d, best);
+  else if (st < 0) best = offer_slow<FIRST_FOUND>(m.tris, k, r.o, r.d, side, near_d, far_d, best);
 }
 
+template <bool FIRST_FOUND = false>
 __device__ __forceinline__ void leaf_first(const MeshDev& m, uint32_t k, const RayF& r, float dlen, int side,
                                            const SideTable& sides, float near_d, float far_d, Best& best) {
   for (;;) {
     const Tri t = load_tri(m.tris, k);
     const int ts = tri_side(t, side, sides);
-    if (ts >= 0) offer_first(m, t, k, r, dlen, ts, near_d, far_d, best);
+    if (ts >= 0) offer_first<FIRST_FOUND>(m, t, k, r, dlen, ts, near_d, far_d, best);
     if (t.flags & kTriLast) break;
     ++k;
   }
