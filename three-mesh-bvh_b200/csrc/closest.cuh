@@ -113,6 +113,15 @@ __device__ __forceinline__ uint32_t vertex_of(const Tri& t, float3 q) {
                                                         : 3u;
 }
 
+// Whether the triangle's box is farther than the best candidate for certain: at most 4 roundings above
+// the exact value's relative 2^-22, so the 2^-20 shrink keeps the distance a lower bound.
+__device__ __forceinline__ bool beyond(float3 p, const Tri& t, float best_hi) {
+  const float dx = fmaxf(fmaxf(fminf(t.a.x, fminf(t.b.x, t.c.x)) - p.x, p.x - fmaxf(t.a.x, fmaxf(t.b.x, t.c.x))), 0.0f);
+  const float dy = fmaxf(fmaxf(fminf(t.a.y, fminf(t.b.y, t.c.y)) - p.y, p.y - fmaxf(t.a.y, fmaxf(t.b.y, t.c.y))), 0.0f);
+  const float dz = fmaxf(fmaxf(fminf(t.a.z, fminf(t.b.z, t.c.z)) - p.z, p.z - fmaxf(t.a.z, fmaxf(t.b.z, t.c.z))), 0.0f);
+  return (dx * dx + dy * dy + dz * dz) * (1.0f - 0x1p-20f) > best_hi;
+}
+
 // A lane's best candidate: float32 squared distance and its error bound, the triangle record with its
 // vertex above kRunShift, its faceIndex and the float32 closest point; and the candidates that float32
 // cannot tell from it (`ties` of them, in the lane's column of a shared array).

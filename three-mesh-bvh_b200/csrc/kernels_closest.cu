@@ -163,15 +163,6 @@ __device__ __forceinline__ bool right_nearer(const Pair& pr, float s0, float s1,
   return centre_d2(pr.r, p) < centre_d2(pr.l, p);
 }
 
-// Whether the triangle's box is farther than the best candidate for certain: at most 4 roundings above
-// the exact value's relative 2^-22, so the 2^-20 shrink keeps the distance a lower bound.
-__device__ __forceinline__ bool beyond(float3 p, const Tri& t, const Nearest& b) {
-  const float dx = fmaxf(fmaxf(fminf(t.a.x, fminf(t.b.x, t.c.x)) - p.x, p.x - fmaxf(t.a.x, fmaxf(t.b.x, t.c.x))), 0.0f);
-  const float dy = fmaxf(fmaxf(fminf(t.a.y, fminf(t.b.y, t.c.y)) - p.y, p.y - fmaxf(t.a.y, fmaxf(t.b.y, t.c.y))), 0.0f);
-  const float dz = fmaxf(fmaxf(fminf(t.a.z, fminf(t.b.z, t.c.z)) - p.z, p.z - fmaxf(t.a.z, fmaxf(t.b.z, t.c.z))), 0.0f);
-  return (dx * dx + dy * dy + dz * dz) * (1.0f - 0x1p-20f) > b.d2 + b.err;
-}
-
 // ---------------------------------------------------------------------------------------------
 // closestPointToPoint, warp-cooperative form for spatially coherent queries (grids, SDF samples)
 // with minThreshold 0.  The 32 queries of a warp walk the tree together with one shared stack of
@@ -217,7 +208,7 @@ __global__ void __launch_bounds__(kBlock, MINB) closest_point_packet_kernel(
           uint32_t k = link & ~kLeafBit;
           for (;;) {
             Tri t = load_tri(m.tris, k);
-            if (!beyond(p, t, b)) offer_closest(m.tris, p, t, k, candidate(p, t), b, s_tie);
+            if (!beyond(p, t, b.d2 + b.err)) offer_closest(m.tris, p, t, k, candidate(p, t), b, s_tie);
             if (t.flags & kTriLast) break;
             ++k;
           }

@@ -123,17 +123,20 @@ __global__ void __launch_bounds__(kBlock) closest_point_kernel(MeshDev m, const 
           uint32_t k = link & ~kLeafBit;
           for (;;) {
             Tri t = load_tri(m.tris, k);
-            float d2, err;
-            bool have_ff;
-            ff cand_ff;
-            cp_offer(m, p, t, k, b, d2, err, have_ff, cand_ff);
-            // early out below minThreshold (closestPointToPoint.js:55-57)
-            if (min2.hi > 0.0f) {
-              bool below;
-              if (d2 + err < min2.hi * (1.0f - kSlabMargin)) below = true;
-              else if (d2 - err > min2.hi * (1.0f + kSlabMargin)) below = false;
-              else below = ff_lt(have_ff ? cand_ff : closest_ff(p, t.a, t.b, t.c).d2, min2);
-              if (below) { stop = true; break; }
+            // (nor can what is beyond the best candidate be below minThreshold, which stops at the first that is)
+            if (!beyond(p, t, b.d2 + b.err)) {
+              float d2, err;
+              bool have_ff;
+              ff cand_ff;
+              cp_offer(m, p, t, k, b, d2, err, have_ff, cand_ff);
+              // early out below minThreshold (closestPointToPoint.js:55-57)
+              if (min2.hi > 0.0f) {
+                bool below;
+                if (d2 + err < min2.hi * (1.0f - kSlabMargin)) below = true;
+                else if (d2 - err > min2.hi * (1.0f + kSlabMargin)) below = false;
+                else below = ff_lt(have_ff ? cand_ff : closest_ff(p, t.a, t.b, t.c).d2, min2);
+                if (below) { stop = true; break; }
+              }
             }
             if (t.flags & kTriLast) break;
             ++k;
