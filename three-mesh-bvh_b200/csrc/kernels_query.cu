@@ -102,7 +102,8 @@ __device__ __forceinline__ void cp_offer(const MeshDev& m, float3 p, const Tri& 
   }
 }
 
-__global__ void __launch_bounds__(kBlock) closest_point_kernel(MeshDev m, const float* __restrict__ pts, uint64_t n,
+// Six blocks an SM: left to itself the compiler takes 96 registers, and 128^3 grid points 12.1 ms instead of 11.5.
+__global__ void __launch_bounds__(kBlock, 6) closest_point_kernel(MeshDev m, const float* __restrict__ pts, uint64_t n,
                                                                float min_t, float max_t,
                                                                bvhc_closest* __restrict__ out) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
