@@ -276,8 +276,9 @@ __global__ void __launch_bounds__(kBlock, MINB) closest_point_packet_kernel(
 }  // namespace dev
 
 cudaError_t launch_closest_phased(const MeshDev& m, const float* pts, uint32_t n, float max_t, bvhc_closest* out,
-                                  const uint32_t* queue, uint32_t pitch, int rows_log2, cudaStream_t stream) {
-  if (pitch || queue) {
+                                  bool shared, const uint32_t* queue, uint32_t pitch, int rows_log2,
+                                  cudaStream_t stream) {
+  if (shared) {
     dev::closest_point_packet_kernel<8><<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, max_t, out, queue, pitch,
                                                                                 rows_log2);
     return cudaGetLastError();

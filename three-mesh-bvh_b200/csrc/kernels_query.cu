@@ -1568,8 +1568,13 @@ cudaError_t launch_closest_point(const MeshDev& m, const float* pts, uint64_t n,
   if (n == 0) return cudaSuccess;
   const bool sorted = variant > 0 && variant % 2 == 0 && queue && qcount && sort && n < (1ull << 32);
   cudaError_t e;
+  // input order (odd variants) may be read in tiles: rows of `tile` points (a grid's row), 2-D blocks
+  const int rl = tile_rows_log2(tile_rows);
+  const uint32_t pitch = (variant % 2 == 1 && tile >= 8 && tile % (32u >> rl) == 0) ? tile : 0;
+  const bool records = group_stack(m) > 0 && m.boxes;
+  const bool shared = sorted || pitch || (variant % 2 == 1 && !records);
   // minThreshold > 0 stops at the first triangle below it in the reference's order
-  if (!(min_t <= 0.0f) || n >= (1ull << 32) || !group_stack(m) || !m.boxes) {
+  if (!(min_t <= 0.0f) || n >= (1ull << 32) || !m.packs || !(records || shared)) {
     dev::closest_point_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, min_t, max_t, out);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     dev::closest_point_finalize_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, out, false);
@@ -1592,10 +1597,8 @@ cudaError_t launch_closest_point(const MeshDev& m, const float* pts, uint64_t n,
   } else {
     queue = nullptr;
   }
-  // input order (odd variants) may be read in tiles: rows of `tile` points (a grid's row), 2-D blocks
-  const int rl = tile_rows_log2(tile_rows);
-  const uint32_t pitch = (variant % 2 == 1 && tile >= 8 && tile % (32u >> rl) == 0) ? tile : 0;
-  if ((e = launch_closest_phased(m, pts, (uint32_t)n, max_t, out, queue, pitch, rl, stream)) != cudaSuccess) return e;
+  e = launch_closest_phased(m, pts, (uint32_t)n, max_t, out, shared, queue, pitch, rl, stream);
+  if (e != cudaSuccess) return e;
   dev::closest_point_finalize_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, out, true);
   return cudaGetLastError();
 }
