@@ -136,7 +136,7 @@ struct bvhc_mesh {
 
   MeshDev view() const {
     MeshDev v{d_nodes, d_tris, d_roots, n_roots, d_err};
-    v.packs = n_tris < kRunFirst;
+    v.n_tris = n_tris;
     set_quads(v, quad_set[0]);
     v.depth = max_depth;
     return v;

@@ -2,7 +2,9 @@
 // maxThreshold test on it, and the phased kernel's launch.
 #pragma once
 
-#include "traverse.cuh"
+#include <cfloat>
+
+#include "group.cuh"
 
 namespace bvhc {
 namespace dev {
@@ -303,20 +305,58 @@ __device__ __forceinline__ bool box_wanted(const BoxChild* __restrict__ c, float
   return s < mx.hi && under_max_slow(c, p, mx.max2);
 }
 
+// A query's walk by its whole warp, `sp` stacked entries (squared distance and link) under `root`: the lanes'
+// best candidates.
+__device__ __forceinline__ void closest_walk_wide(const MeshDev& m, float3 p, const MaxThreshold& mx, uint2* stack,
+                                                  int spare, int sp, int root, float bound, Nearest& best,
+                                                  uint2 (*s_tie)[kBlock]) {
+  const unsigned full = 0xFFFFFFFFu, lane = threadIdx.x & 31u, j = lane & 3u;
+  for (;;) {
+    while (sp > 0) {
+      WideEntry e = wide_take(stack, sp, lane, spare);
+      e.on = e.on && e.key <= bound;
+      const bool leaf = e.on && (e.link & kLeafBit);
+      bool enter = false;
+      uint32_t link = 0u;
+      float key = 0.0f;
+      if (e.on && !leaf) {
+        const BoxChild* c = m.boxes[e.link].c + j;
+        enter = box_wanted(c, p, bound, mx, key, link);
+      }
+      if (leaf && j <= ((e.link >> kRunShift) & 3u)) {
+        const uint32_t k = (e.link & kRunFirst) + j;
+        const Tri t = load_tri(m.tris, k);
+        offer_closest(m.tris, p, t, k, candidate(p, t), best, s_tie);
+      }
+      if (__ballot_sync(full, leaf))
+        bound = fminf(bound, warp_min(fminf((best.d2 + best.err) * (1.0f + 0x1p-18f), FLT_MAX)));
+      if (__ballot_sync(full, enter)) wide_push(stack, sp, lane, enter, link, key, key);
+    }
+    if (++root >= m.n_roots) return;
+    sp = 1;
+    if (lane == 0) stack[0] = make_uint2(m.quad_roots[root], 0u);
+    __syncwarp();
+  }
+}
+
 }  // namespace dev
 
-// Up to this many queries take the whole warp each (kernels_wide.cu), more four lanes.  A query about as
-// far from many triangles (on the axis of a tube) walks hundreds of steps after the others are done,
-// and the whole warp takes up to eight of them at once.  Scattered points on the 80,000-triangle knot:
-// 4,000 points 67 us (four lanes: 407), 100,003 points 650 us (978), 200,000 points 1196 us (1279), 400,000
-// points 2262 us (1841).
-constexpr uint32_t kWideMaxQueries = 200000;
+// Up to this many queries take the whole warp each (kernels_wide.cu), more four lanes, the last of a warp again
+// all 32.  A query about as far from many triangles (on the axis of a tube) walks hundreds of steps after the
+// others are done, and the whole warp takes up to eight of them at once; a query near the surface is done in a
+// few, and the whole warp is wasted on it.  So the line depends on the queries, and on how long walks are.
+// 80,000-triangle knot, points about the surface, seven tenths of them so and the rest spread, all spread, a grid:
+// 32,000 points 200, 265, 331, 278 us by warps (four lanes 120, 304, 413, 445), 70,000 points 359, 484, 624, 462
+// (185, 490, 652, 714), 100,000 points 507, 650, 863, 628 (234, 503, 751, 802).  10,000 triangles: 16,000 points
+// 93, 106, 128, 97 (81, 114, 167, 155), 32,000 points 157, 183, 204, 165 (97, 148, 183, 194), 70,000 points
+// 288, 329, 388, 285 (144, 218, 292, 269).
+static inline uint32_t wide_queries(const MeshDev& m) { return m.n_tris < 50000 ? 32768 : 65536; }
 cudaError_t launch_closest_wide(const MeshDev& m, const float* pts, uint32_t n, float max_t, bvhc_closest* out,
                                 cudaStream_t stream);
 
 // closestPointToPoint's traversals with minThreshold 0 (kernels_closest.cu): pending records of five words
 // (triangle record and vertex, or 0xFFFFFFFF; number of undecided candidates; those).  shared: the 32 queries of
-// a warp in one traversal of the child pairs (m.packs), in the order of `queue` (nullable), or with pitch > 0 in
+// a warp in one traversal of the child pairs (m.n_tris < kRunFirst), in the order of `queue` (nullable), or with pitch > 0 in
 // tiled order with 2^rows_log2 rows a tile; else over the four-child records (group_stack(m) > 0).
 cudaError_t launch_closest_phased(const MeshDev& m, const float* pts, uint32_t n, float max_t, bvhc_closest* out,
                                   bool shared, const uint32_t* queue, uint32_t pitch, int rows_log2,

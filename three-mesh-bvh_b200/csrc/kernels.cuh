@@ -26,7 +26,7 @@ struct MeshDev {
   const QuadNode* quads = nullptr;     // four-child copy of `nodes` (same triangle records), if any
   const uint32_t* quad_roots = nullptr;
   const BoxNode* boxes = nullptr;      // the same records with lo / hi bounds (the reference's leaves only)
-  bool packs = false;                  // every triangle record fits kRunShift bits
+  uint64_t n_tris = 0;                 // triangle records, where the launch asks (closestPointToPoint)
   int quad_stack = 0;                  // entries a traversal of the four-child records can stack
   int depth = kMaxStack - 2;           // deepest node level of these records (bounds the stack use)
 };

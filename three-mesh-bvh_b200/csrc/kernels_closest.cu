@@ -1,6 +1,6 @@
 // closestPointToPoint with minThreshold 0: four lanes per query (the smaller batches take whole warps,
-// kernels_wide.cu) over the four-child records, and the 32
-// queries of a warp through one shared traversal; and their launches.
+// kernels_wide.cu) over the four-child records, and the 32 queries of a warp through one shared traversal;
+// and their launches.
 #include <algorithm>
 #include <cfloat>
 
@@ -15,7 +15,7 @@ constexpr int kClosestRefill = 2 * kGroup;  // idle lanes at which a warp takes 
 
 __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_group_kernel(
     MeshDev m, const float* __restrict__ pts, uint32_t n, float max_t, bvhc_closest* __restrict__ out,
-    const uint32_t* __restrict__ queue, uint32_t pitch, int rows_log2, int cap) {
+    uint32_t take, int cap) {
   extern __shared__ uint2 s_stack[];
   __shared__ uint2 s_tie[kClosestTies][kBlock];
   const unsigned full = 0xFFFFFFFFu;
@@ -29,9 +29,9 @@ __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_gro
   float bound = 0.0f;  // boxes beyond it cannot hold a candidate
   Nearest best = nearest_none();
   int sp = 0, root = 0;
-  // this warp's chunks of 32 queries: every (warps of the grid)-th one (no work counter, which calls on
+  // this warp's chunks of `take` queries: every (warps of the grid)-th one (no work counter, which calls on
   // different streams would share)
-  const uint32_t warps = gridDim.x * (kBlock / 32), chunks = (n + 31u) / 32u;
+  const uint32_t warps = gridDim.x * (kBlock / 32), chunks = (n + take - 1u) / take;
   uint32_t chunk = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), pool = 0, pool_end = 0;
   auto next_root = [&]() {
     sp = 0;
@@ -52,15 +52,13 @@ __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_gro
       }
       const unsigned want = __popc(idle) / kGroup;
       if (pool == pool_end && chunk < chunks) {
-        pool = chunk * 32u;
-        pool_end = n - pool > 32u ? pool + 32u : n;
+        pool = chunk * take;
+        pool_end = n - pool > take ? pool + take : n;
         chunk += warps;
       }
       const unsigned avail = pool_end - pool, mine = __popc(idle & below);
       if (!active && mine < avail) {
         qid = pool + mine;
-        if (queue) qid = __ldg(queue + qid);
-        else if (pitch) qid = (uint32_t)tiled_index(qid, pitch, rows_log2, n);
         const float* q = pts + 3 * (size_t)qid;
         p = make_float3(__ldg(q), __ldg(q + 1), __ldg(q + 2));
         // a point that is not finite reaches no leaf
@@ -77,6 +75,40 @@ __global__ void __launch_bounds__(kBlock, kClosestBlocksPerSm) closest_point_gro
       if (!__ballot_sync(full, active)) {
         if (chunk >= chunks && pool == pool_end && !__ballot_sync(full, pending)) break;
         continue;
+      }
+    }
+    if (idle && chunk >= chunks && pool == pool_end) {
+      const unsigned walking = __ballot_sync(full, active);
+      if (__popc(walking) == kGroup) {  // the last one: all 32 lanes
+        if (__ballot_sync(full, pending)) {
+          store_merged<kGroup>(m.tris, p, best, pending, reinterpret_cast<uint32_t*>(out + qid), s_tie);
+          pending = false;
+        }
+        const int from = __ffs(walking) - 1;
+        if (!active) best = nearest_none();
+        qid = __shfl_sync(full, qid, from);
+        p.x = __shfl_sync(full, p.x, from);
+        p.y = __shfl_sync(full, p.y, from);
+        p.z = __shfl_sync(full, p.z, from);
+        bound = __shfl_sync(full, bound, from);
+        sp = __shfl_sync(full, sp, from);
+        link = __shfl_sync(full, link, from);
+        dead = __shfl_sync(full, dead, from);
+        root = __shfl_sync(full, root, from);
+        const int wg = (int)(threadIdx.x >> 5) * kGroups, g = wg + from / kGroup;
+        uint2 v[kMaxGroupStack / 32];
+        for (int i = 0; i < kMaxGroupStack / 32; ++i)
+          if (32 * i + (int)lane < sp) v[i] = s_stack[g * (cap + 1) + 32 * i + lane];
+        __syncwarp();
+        stack = s_stack + wg * (cap + 1);  // all the groups' stacks
+        for (int i = 0; i < kMaxGroupStack / 32; ++i)
+          if (32 * i + (int)lane < sp) stack[32 * i + lane] = v[i];
+        if (!dead && lane == 0) stack[sp] = make_uint2(link, 0u);
+        __syncwarp();
+        // eight entries at once while what they add and one depth-first walk fit above the rest
+        closest_walk_wide(m, p, mx, stack, kGroups * (cap + 1) - 32 - cap, sp + (dead ? 0 : 1), root, bound, best, s_tie);
+        store_merged<32>(m.tris, p, best, true, reinterpret_cast<uint32_t*>(out + qid), s_tie);
+        break;
       }
     }
     // node steps, while no more groups wait at leaves than are at records
@@ -284,11 +316,13 @@ cudaError_t launch_closest_phased(const MeshDev& m, const float* pts, uint32_t n
     return cudaGetLastError();
   }
   const int cap = group_stack(m);
-  if (n <= kWideMaxQueries) return launch_closest_wide(m, pts, n, max_t, out, stream);
+  if (n <= wide_queries(m)) return launch_closest_wide(m, pts, n, max_t, out, stream);
   const unsigned int resident = (unsigned int)sm_count() * dev::kClosestBlocksPerSm;
   const unsigned int blocks = (n + dev::kBlockGroups - 1) / dev::kBlockGroups;
+  // queries a warp takes at once: 100,000 points 503 us by 8 (4: 519, 16: 558, 32: 599), 300,000 the same by all
+  const uint32_t take = 8;
   dev::closest_point_group_kernel<<<std::min(blocks, resident), dev::kBlock, group_smem(cap), stream>>>(
-      m, pts, n, max_t, out, queue, pitch, rows_log2, cap);
+      m, pts, n, max_t, out, take, cap);
   return cudaGetLastError();
 }
 

@@ -86,40 +86,19 @@ __global__ void __launch_bounds__(kBlock) closest_point_wide_kernel(MeshDev m, c
                                                                     int cap) {
   extern __shared__ uint2 s_stack[];
   __shared__ uint2 s_tie[kClosestTies][kBlock];
-  const unsigned full = 0xFFFFFFFFu, lane = threadIdx.x & 31u, j = lane & 3u;
+  const unsigned lane = threadIdx.x & 31u;
   uint2* stack = s_stack + (threadIdx.x >> 5) * cap;
   const MaxThreshold mx = max_threshold(max_t);
   for (uint32_t qid = blockIdx.x * kWarps + (threadIdx.x >> 5); qid < n; qid += gridDim.x * kWarps) {
     const float* q = pts + 3 * (size_t)qid;
     const float3 p = make_float3(__ldg(q), __ldg(q + 1), __ldg(q + 2));
-    float bound = FLT_MAX;
     // a point that is not finite reaches no leaf
     const bool finite = fabsf(p.x) <= FLT_MAX && fabsf(p.y) <= FLT_MAX && fabsf(p.z) <= FLT_MAX;
     Nearest best = nearest_none();
-    for (int root = finite ? 0 : m.n_roots; root < m.n_roots; ++root) {
-      int sp = 1;
-      if (lane == 0) stack[0] = make_uint2(m.quad_roots[root], 0u);
+    if (finite && m.n_roots > 0) {
+      if (lane == 0) stack[0] = make_uint2(m.quad_roots[0], 0u);
       __syncwarp();
-      while (sp > 0) {
-        WideEntry e = wide_take(stack, sp, lane);
-        e.on = e.on && e.key <= bound;
-        const bool leaf = e.on && (e.link & kLeafBit);
-        bool enter = false;
-        uint32_t link = 0u;
-        float key = 0.0f;
-        if (e.on && !leaf) {
-          const BoxChild* c = m.boxes[e.link].c + j;
-          enter = box_wanted(c, p, bound, mx, key, link);
-        }
-        if (leaf && j <= ((e.link >> kRunShift) & 3u)) {
-          const uint32_t k = (e.link & kRunFirst) + j;
-          const Tri t = load_tri(m.tris, k);
-          offer_closest(m.tris, p, t, k, candidate(p, t), best, s_tie);
-        }
-        if (__ballot_sync(full, leaf))
-          bound = fminf(bound, warp_min(fminf((best.d2 + best.err) * (1.0f + 0x1p-18f), FLT_MAX)));
-        if (__ballot_sync(full, enter)) wide_push(stack, sp, lane, enter, link, key, key);
-      }
+      closest_walk_wide(m, p, mx, stack, kWideSpare, 1, 0, FLT_MAX, best, s_tie);
     }
     store_merged<32>(m.tris, p, best, true, reinterpret_cast<uint32_t*>(out + qid), s_tie);
   }
