@@ -166,11 +166,11 @@ bvhc_status bvhc_mesh_get_info(const bvhc_mesh* mesh, bvhc_mesh_info* info);
  * that point (coarser) followed by the direction; 0 keeps the input order.  wide = 1 makes the
  * warp-cooperative form walk four-child records (64-entry stack); the persistent form always does.
  * closest selects closestPointToPoint's kernel: 0 the queries in input order over four-child records
- * (a warp per query for up to 200,000, else four lanes), 1 the same unless `tile` is set, in which case
- * the 32 queries of a warp (a tile of the rows of `tile` points, e.g. a grid's row) go
- * through one shared traversal, 2 one shared traversal for the 32 queries of a warp over the
- * queries sorted by a Morton key of the point; 3 and 5 run as 1, 4 and 6 as 2.  With a
- * minThreshold above 0, and for trees without four-child records, one query per thread runs.
+ * (a warp per query for the smaller batches, else four lanes), 1 one shared traversal for the 32 queries
+ * of a warp, in input order (up to 200,000 queries the same as 0), or with `tile` set a tile of the rows of
+ * `tile` points (e.g. a grid's row) a warp, 2 the same shared traversal over the queries sorted by a Morton
+ * key of the point; 3 and 5 run as 1, 4 and 6 as 2.  With a minThreshold above 0 one query per thread runs,
+ * and for trees without four-child records where those would.
  * All forms return the same bytes.  all selects raycast's
  * (all hits) kernel: 0 one ray per thread, 1 the rays of a warp through one shared left-first
  * traversal (each ray's hits stay in the reference's DFS order), 2, 3 and 4 the same over the rays

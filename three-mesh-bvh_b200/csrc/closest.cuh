@@ -350,6 +350,10 @@ __device__ __forceinline__ void closest_walk_wide(const MeshDev& m, float3 p, co
 // (185, 490, 652, 714), 100,000 points 507, 650, 863, 628 (234, 503, 751, 802).  10,000 triangles: 16,000 points
 // 93, 106, 128, 97 (81, 114, 167, 155), 32,000 points 157, 183, 204, 165 (97, 148, 183, 194), 70,000 points
 // 288, 329, 388, 285 (144, 218, 292, 269).
+// Odd variants without tiles, which are for coherent queries, take the shared traversal in input order beyond this
+// many: grids on the 80,000-triangle knot, 140,000 points 1.25 ms shared (four lanes 1.06), 195,112 1.25 (1.10),
+// 300,000 1.37 (1.60), 2,097,152 4.1 (8.7), 16,777,216 21 (61).
+constexpr uint64_t kSharedQueries = 200000;
 static inline uint32_t wide_queries(const MeshDev& m) { return m.n_tris < 50000 ? 32768 : 65536; }
 cudaError_t launch_closest_wide(const MeshDev& m, const float* pts, uint32_t n, float max_t, bvhc_closest* out,
                                 cudaStream_t stream);

@@ -48,8 +48,8 @@ struct TraversalConfig {
                    // warp-cooperative forms)
   int sort;        // 0: queue in ray order; 1..3: queue sorted by a Morton key (raysort.cu), implies
                    // the pre-pass
-  int closest;     // closestPointToPoint: 0 a warp or four lanes per query, 1 (3, 5) the same unless
-                   // tiled, then warp-cooperative, 2 (4, 6) warp-cooperative over Morton-sorted queries
+  int closest;     // closestPointToPoint: 0 a warp or four lanes per query, 1 (3, 5) warp-cooperative
+                   // in input or tiled order, 2 (4, 6) over Morton-sorted queries
   int wide;        // warp-cooperative raycastFirst: 1 walks the four-child records
   int all;         // raycast (all hits): 0 one ray per thread, 1 warp-cooperative, 2..4 warp-cooperative
                    // over the rays that enter the tree, sorted by key kind all - 1, 5..8 one ray per

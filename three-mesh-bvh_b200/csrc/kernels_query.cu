@@ -1572,7 +1572,7 @@ cudaError_t launch_closest_point(const MeshDev& m, const float* pts, uint64_t n,
   const int rl = tile_rows_log2(tile_rows);
   const uint32_t pitch = (variant % 2 == 1 && tile >= 8 && tile % (32u >> rl) == 0) ? tile : 0;
   const bool records = group_stack(m) > 0 && m.boxes;
-  const bool shared = sorted || pitch || (variant % 2 == 1 && !records);
+  const bool shared = sorted || pitch || (variant % 2 == 1 && (!records || n > kSharedQueries));
   // minThreshold > 0 stops at the first triangle below it in the reference's order
   if (!(min_t <= 0.0f) || n >= (1ull << 32) || m.n_tris >= kRunFirst || !(records || shared)) {
     dev::closest_point_kernel<<<grid_for(n), dev::kBlock, 0, stream>>>(m, pts, n, min_t, max_t, out);
