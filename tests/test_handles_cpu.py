@@ -17,7 +17,7 @@ def lib(pkg, tmp_path_factory):
     out = tmp_path_factory.mktemp("fake") / "libfake.so"
     csrc = os.path.join(ROOT, "three-mesh-bvh_b200", "csrc")
     cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-include", "cmath", "-I", csrc, "-I",
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-include", "cmath", "-I", csrc, "-I",
                     os.path.join(ROOT, "include"), "-I", cuda, "-x", "c++", os.path.join(csrc, "api.cu"),
                     os.path.join(csrc, "builder.cpp"), os.path.join(ROOT, "tests", "native", "fake_cuda.cpp"),
                     "-o", str(out)], check=True)
