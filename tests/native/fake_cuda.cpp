@@ -76,9 +76,20 @@ cudaError_t launch_ray_pairs(const PairNode* pairs, uint64_t n, RayPair* out, cu
   return cudaSuccess;
 }
 
-cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n, const uint32_t* src, const PairNode*, const TriRecord*,
-                              BoxNode*, cudaStream_t) {
-  check(live(quads, n * sizeof(QuadNode)) && live(src, 4 * n * sizeof(uint32_t)));
+cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n, const QuadShape* shape, const PairNode* pairs,
+                              const TriRecord* tris, BoxNode*, cudaStream_t) {
+  check(live(quads, n * sizeof(QuadNode)) && live(shape, 4 * n * sizeof(QuadShape)));
+  auto p = held.find(const_cast<PairNode*>(pairs)), t = held.find(const_cast<TriRecord*>(tris));
+  check(p != held.end() && t != held.end());
+  if (p == held.end() || t == held.end()) return cudaErrorInvalidValue;
+  float box[6];
+  for (uint64_t k = 0; k < 4 * n; ++k) {
+    const QuadShape& s = shape[k];
+    const bool in = s.src == kEmptyLeaf || (s.src & kLeafBit ? (s.src & ~kLeafBit) + s.count <= t->second / sizeof(TriRecord)
+                                                             : s.src / 2 < p->second / sizeof(PairNode));
+    check(in);
+    if (in) quads[k / 4].c[k % 4] = quad_child(s, pairs, tris, box);
+  }
   return cudaSuccess;
 }
 

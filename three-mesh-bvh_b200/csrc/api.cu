@@ -7,7 +7,6 @@
 #include <cstdint>
 #include <cstring>
 #include <exception>
-#include <limits>
 #include <new>
 #include <stdexcept>
 #include <thread>
@@ -106,7 +105,7 @@ struct bvhc_mesh {
     QuadNode* quads = nullptr;
     BoxNode* boxes = nullptr;
     uint32_t* roots = nullptr;
-    uint32_t* src = nullptr;  // where each child's box comes from (QuadBuilder::src)
+    QuadShape* shape = nullptr;  // four a record
     uint64_t n = 0;
     int stack = 0;
     RayPair* ray_pairs = nullptr;  // the child pairs themselves in the ray traversals' form
@@ -481,14 +480,11 @@ struct LeafSplitter {
 // with the largest box surface area is replaced in place by its own two children until there are four
 // children or only leaves.  A leaf of more than kMaxRun triangles has a record of its own, made the
 // same way from its halves; the leaf's own box stays in its parent's record, because the reference
-// tests it against near and far.  `src` keeps, per quad child, where its box comes from, for refits: the child-pair slot
-// (2 * pair + side), or kLeafBit | the first of its `count` triangle records; kEmptyLeaf: unused, or a
-// root leaf's unbounded box.
+// tests it against near and far.  The boxes are filled in on the device, where a refit fills them in again.
 struct QuadBuilder {
   const std::vector<PairNode>& pairs;
   const std::vector<TriRecord>& tris;
-  std::vector<QuadNode> quads;
-  std::vector<uint32_t> src;
+  std::vector<QuadShape> shape;  // four a record
   int stack = 0;  // entries a traversal can stack: at most the siblings along one path
   bool nested = true;  // every box of the tree lies in its parent's, so that those that are not records'
                        // children need no test (a tree from a file may hold anything)
@@ -519,13 +515,10 @@ struct QuadBuilder {
   std::vector<Later> later;
 
   uint32_t add() {
-    if (quads.size() >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
-    const uint32_t idx = (uint32_t)quads.size();
-    const float nan = std::numeric_limits<float>::quiet_NaN();
-    const QuadChild unused{{nan, nan}, {nan, nan}, nan, nan, kEmptyLeaf, 0};  // until a child is put in
-    quads.push_back(QuadNode{{unused, unused, unused, unused}});
-    src.insert(src.end(), 4, kEmptyLeaf);
-    return idx;
+    const size_t idx = shape.size() / 4;
+    if (idx >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
+    shape.insert(shape.end(), 4, QuadShape{kEmptyLeaf, 0, kEmptyLeaf});
+    return (uint32_t)idx;
   }
 
   // Builds what was put off: each subtree by one of the host's threads into records of its own, which
@@ -559,23 +552,20 @@ struct QuadBuilder {
     for (auto& th : pool) th.join();
     if (failed == 1) throw Status{BVHC_ERR_UNSUPPORTED};
     if (failed) throw std::bad_alloc();
-    size_t total = quads.size();
-    for (const QuadBuilder& p : part) total += p.quads.size();
-    if (total >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
-    quads.reserve(total);
-    src.reserve(4 * total);
+    size_t total = shape.size();
+    for (const QuadBuilder& p : part) total += p.shape.size();
+    if (total / 4 >= (uint64_t)kLeafBit) throw Status{BVHC_ERR_UNSUPPORTED};
+    shape.reserve(total);
     for (size_t t = 0; t < part.size(); ++t) {
-      const uint32_t base = (uint32_t)quads.size();
-      quads[later[t].quad].c[later[t].k].link = base;
-      for (QuadNode q : part[t].quads) {
-        for (QuadChild& c : q.c)
-          if (!(c.link & kLeafBit)) c.link += base;
-        quads.push_back(q);
+      const uint32_t base = (uint32_t)(shape.size() / 4);
+      shape[4 * (size_t)later[t].quad + later[t].k].link = base;
+      for (QuadShape c : part[t].shape) {
+        if (!(c.link & kLeafBit)) c.link += base;
+        shape.push_back(c);
       }
-      src.insert(src.end(), part[t].src.begin(), part[t].src.end());
       stack = std::max(stack, part[t].stack);
       nested = nested && part[t].nested;
-      part[t].quads = {};
+      part[t].shape = {};
     }
     later.clear();
   }
@@ -606,7 +596,7 @@ struct QuadBuilder {
     c.first = first;
     c.count = count;
     c.part = true;
-    LeafSplitter::bounds(&tris[first], count, c.box);
+    if (c.splits()) LeafSplitter::bounds(&tris[first], count, c.box);  // which part to split next
     return c;
   }
 
@@ -644,11 +634,7 @@ struct QuadBuilder {
     c.first = link & ~kLeafBit;
     c.count = leaf_count(c.first);
     const uint32_t l = c.splits() ? build(c, 0) : run_link(c.first, (int)c.count);
-    QuadChild& q = quads[idx].c[0];
-    q.c[0] = q.c[1] = q.cz = 0.0f;
-    q.h[0] = q.h[1] = q.hz = kBoxUnbounded;
-    q.link = l;
-    q.count = c.count;
+    shape[4 * (size_t)idx] = QuadShape{l, c.count, kEmptyLeaf};
     return idx;
   }
 
@@ -676,13 +662,9 @@ struct QuadBuilder {
     const uint32_t idx = add();
     for (int k = 0; k < n; ++k) {
       if (ch[k].pair == kEmptyLeaf && ch[k].count == 0) continue;  // an empty leaf
-      QuadChild& q = quads[idx].c[k];
-      const float* b = ch[k].box;
-      box_centre_half(b[0], b[3], q.c[0], q.h[0]);
-      box_centre_half(b[1], b[4], q.c[1], q.h[1]);
-      box_centre_half(b[2], b[5], q.cz, q.hz);
+      QuadShape& q = shape[4 * (size_t)idx + k];
       if (!ch[k].splits()) q.link = run_link(ch[k].first, (int)ch[k].count);
-      src[4 * (size_t)idx + k] = ch[k].part ? kLeafBit | ch[k].first : ch[k].slot;
+      q.src = ch[k].part ? kLeafBit | ch[k].first : ch[k].slot;
       if (ch[k].part) q.count = ch[k].count;
     }
     stack = std::max(stack, below + n - 1);
@@ -693,7 +675,7 @@ struct QuadBuilder {
           continue;
         }
         uint32_t q = build(ch[k], below + n - 1, level + 1);
-        quads[idx].c[k].link = q;
+        shape[4 * (size_t)idx + k].link = q;
       }
     return idx;
   }
@@ -773,7 +755,7 @@ static void free_quads(bvhc_mesh::QuadSet& q) {
   cudaFree(q.quads);
   cudaFree(q.boxes);
   cudaFree(q.roots);
-  cudaFree(q.src);
+  cudaFree(q.shape);
   cudaFree(q.ray_pairs);
   q = bvhc_mesh::QuadSet{};
 }
@@ -800,15 +782,13 @@ static cudaError_t make_quads(bvhc_mesh::QuadSet& q, bool with_boxes, const Pair
     e = cudaErrorMemoryAllocation;
   }
   if (e == cudaSuccess && !qroots.empty() && qb.nested) {
-    e = upload(&q.quads, qb.quads);
-    if (e == cudaSuccess) e = upload(&q.roots, qroots);
-    if (e == cudaSuccess) e = upload(&q.src, qb.src);
-    q.n = qb.quads.size();
+    q.n = qb.shape.size() / 4;
     q.stack = qb.stack;
-    if (with_boxes) {
-      if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&q.boxes), q.n * sizeof(BoxNode));
-      if (e == cudaSuccess) e = launch_quad_boxes(q.quads, q.n, q.src, nodes, recs, q.boxes, nullptr);
-    }
+    e = upload(&q.shape, qb.shape);
+    if (e == cudaSuccess) e = upload(&q.roots, qroots);
+    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&q.quads), q.n * sizeof(QuadNode));
+    if (e == cudaSuccess && with_boxes) e = cudaMalloc(reinterpret_cast<void**>(&q.boxes), q.n * sizeof(BoxNode));
+    if (e == cudaSuccess) e = launch_quad_boxes(q.quads, q.n, q.shape, nodes, recs, q.boxes, nullptr);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e != cudaSuccess) free_quads(q);
@@ -1419,7 +1399,7 @@ bvhc_status bvhc_mesh_refit(bvhc_mesh* m, const float* positions, uint64_t n_ver
     const bvhc_mesh::QuadSet& q = m->quad_set[k];
     if (q.ray_pairs) BVHC_CUDA_TRY(launch_ray_pairs(k ? m->d_nodes_f : m->d_nodes, q.n_pairs, q.ray_pairs, s));
     if (q.quads)
-      BVHC_CUDA_TRY(launch_quad_boxes(q.quads, q.n, q.src, k ? m->d_nodes_f : m->d_nodes, k ? m->d_tris_f : m->d_tris,
+      BVHC_CUDA_TRY(launch_quad_boxes(q.quads, q.n, q.shape, k ? m->d_nodes_f : m->d_nodes, k ? m->d_tris_f : m->d_tris,
                                       q.boxes, s));
   }
   if (m->d_pos && m->grad_verts <= n_verts) {  // the adjoint's vertex copy follows the geometry
@@ -2154,8 +2134,12 @@ bvhc_status set_instance_quads(bvhc_scene* sc, const std::vector<PairNode>& node
     QuadBuilder qb{nodes, leaves};
     sc->quad_root = qb.root(sc->root);
     if (!qb.nested) return BVHC_OK;
-    BVHC_CUDA_TRY(ensure(reinterpret_cast<void**>(&sc->d_quads), &sc->quads_cap, qb.quads.size() * sizeof(QuadNode)));
-    BVHC_CUDA_TRY(cudaMemcpy(sc->d_quads, qb.quads.data(), qb.quads.size() * sizeof(QuadNode), cudaMemcpyHostToDevice));
+    std::vector<QuadNode> quads(qb.shape.size() / 4);
+    float box[6];
+    for (size_t k = 0; k < qb.shape.size(); ++k)
+      quads[k / 4].c[k % 4] = quad_child(qb.shape[k], nodes.data(), nullptr, box);
+    BVHC_CUDA_TRY(ensure(reinterpret_cast<void**>(&sc->d_quads), &sc->quads_cap, quads.size() * sizeof(QuadNode)));
+    BVHC_CUDA_TRY(cudaMemcpy(sc->d_quads, quads.data(), quads.size() * sizeof(QuadNode), cudaMemcpyHostToDevice));
     sc->quad_stack = qb.stack;
     sc->has_quads = true;
   } catch (const Status& st) {

@@ -256,10 +256,9 @@ struct RefitPlan {
 // changed; force = true recomputes every box.  tri_vid: 3 vertex ids per triangle (faceIndex).
 cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris, const uint32_t* tri_vid,
                          const float* pos, int stride, bool force, cudaStream_t stream);
-// Every four-child record's child boxes, from the child-pair slots they were collapsed from (src: 4
-// per record) or, for parts of a leaf (src kLeafBit | first), from their triangle records; `boxes`
-// (nullable) gets the same records with lo / hi bounds.
-cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
+// Every four-child record from its shape (4 per record), the child pairs and, for parts of leaves, the triangle
+// records; `boxes` (nullable) gets the same records with lo / hi bounds.
+cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const QuadShape* shape, const PairNode* pairs,
                               const TriRecord* tris, BoxNode* boxes, cudaStream_t stream);
 
 // `nodes` as RayPairs.

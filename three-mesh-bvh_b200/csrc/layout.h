@@ -12,6 +12,8 @@
 // leaf is one contiguous run of 16-byte-aligned loads and needs no index indirection.
 #pragma once
 
+#include <math.h>
+
 #include <cstdint>
 
 namespace bvhc {
@@ -51,6 +53,13 @@ struct alignas(128) QuadNode {
   QuadChild c[4];
 };
 static_assert(sizeof(QuadNode) == 128, "QuadNode must be 128 bytes");
+
+// What a child of a four-child record is made from: its link and count, and where its box comes from: the
+// child-pair slot (2 * pair + side), or kLeafBit | the first of its `count` triangle records; kEmptyLeaf: unused,
+// or with another link a root leaf's unbounded box.
+struct QuadShape {
+  uint32_t link, count, src;
+};
 
 // A child pair in the same form, for the warp-shared ray traversals: the two children of a PairNode and,
 // in c[0].count, its split axis (an empty leaf's box is NaN).
@@ -117,6 +126,43 @@ static_assert(sizeof(TriRecord) == 48, "TriRecord must be 48 bytes");
 constexpr uint32_t kTriLast = 1u;
 constexpr uint32_t kNoMaterial = 0xFFFFFFFFu;
 constexpr int kMaxMaterials = 64;
+
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+    // A child of a four-child record; b (lo, hi) gets its box, which is that of its child-pair slot, or for a
+    // part of a leaf the bounds of its triangles.
+    inline QuadChild quad_child(const QuadShape& s, const PairNode* pairs, const TriRecord* tris, float* b) {
+  QuadChild c;
+  c.link = s.link;
+  c.count = s.count;
+  if (s.src == kEmptyLeaf) {
+    const bool unused = s.link == kEmptyLeaf;
+    for (int a = 0; a < 3; ++a) {
+      b[a] = unused ? INFINITY : -INFINITY;
+      b[3 + a] = INFINITY;
+    }
+    c.c[0] = c.c[1] = c.cz = unused ? NAN : 0.0f;
+    c.h[0] = c.h[1] = c.hz = unused ? NAN : kBoxUnbounded;
+    return c;
+  }
+  if (!(s.src & kLeafBit)) {
+    const float* f = pairs[s.src >> 1].f + 6 * (s.src & 1u);
+    for (int a = 0; a < 6; ++a) b[a] = f[a];
+  } else {
+    const TriRecord* t = tris + (s.src & ~kLeafBit);
+    for (int a = 0; a < 3; ++a) b[a] = b[3 + a] = t->v[a];
+    for (uint32_t q = 0; q < s.count; ++q)
+      for (int a = 0; a < 9; ++a) {
+        b[a % 3] = fminf(b[a % 3], t[q].v[a]);
+        b[3 + a % 3] = fmaxf(b[3 + a % 3], t[q].v[a]);
+      }
+  }
+  box_centre_half(b[0], b[3], c.c[0], c.h[0]);
+  box_centre_half(b[1], b[4], c.c[1], c.h[1]);
+  box_centre_half(b[2], b[5], c.cz, c.hz);
+  return c;
+}
 
 // Per-call side selection: a single side for every triangle, or one side per material.
 struct SideTable {

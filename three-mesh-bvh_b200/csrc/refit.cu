@@ -82,42 +82,18 @@ __global__ void __launch_bounds__(kRefitBlock) refit_kernel(RefitPlan plan, Pair
   }
 }
 
-// Four-child records: a child's box is that of the child-pair slot it was collapsed from, or for a part
-// of a leaf (src kLeafBit | first record) the bounds of its triangles.  The unbounded child of a root
-// that is a leaf (src kEmptyLeaf, link not) keeps its box.  `boxes` (nullable): the lo / hi form of the
-// same records, written whole.
+// Four-child records from their shape (layout.h); `boxes` (nullable): the lo / hi form of the same records.
+// One child a thread, written whole.
 __global__ void __launch_bounds__(kRefitBlock) quad_boxes_kernel(QuadNode* __restrict__ quads, uint64_t n_quads,
-                                                                 const uint32_t* __restrict__ src,
+                                                                 const QuadShape* __restrict__ shape,
                                                                  const PairNode* __restrict__ pairs,
                                                                  const TriRecord* __restrict__ tris,
                                                                  BoxNode* __restrict__ boxes) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= 4 * n_quads) return;
-  const uint32_t slot = __ldg(src + k);
-  QuadChild& c = quads[k >> 2].c[k & 3u];
   float b[6];
-  if (slot == kEmptyLeaf) {
-    if (boxes) {
-      const float inf = __builtin_huge_valf(), lo = c.link == kEmptyLeaf ? inf : -inf;
-      boxes[k >> 2].c[k & 3u] = BoxChild{{lo, lo, lo}, {inf, inf, inf}, c.link, c.count};
-    }
-    return;
-  }
-  if (!(slot & kLeafBit)) {
-    const float* f = pairs[slot >> 1].f + 6 * (slot & 1u);
-    for (int a = 0; a < 6; ++a) b[a] = f[a];
-  } else {
-    const TriRecord* t = tris + (slot & ~kLeafBit);
-    for (int a = 0; a < 3; ++a) b[a] = b[3 + a] = t->v[a];
-    for (uint32_t q = 0; q < c.count; ++q)
-      for (int a = 0; a < 9; ++a) {
-        b[a % 3] = fminf(b[a % 3], t[q].v[a]);
-        b[3 + a % 3] = fmaxf(b[3 + a % 3], t[q].v[a]);
-      }
-  }
-  box_centre_half(b[0], b[3], c.c[0], c.h[0]);
-  box_centre_half(b[1], b[4], c.c[1], c.h[1]);
-  box_centre_half(b[2], b[5], c.cz, c.hz);
+  const QuadChild c = quad_child(shape[k], pairs, tris, b);
+  quads[k >> 2].c[k & 3u] = c;
   if (boxes) boxes[k >> 2].c[k & 3u] = BoxChild{{b[0], b[1], b[2]}, {b[3], b[4], b[5]}, c.link, c.count};
 }
 
@@ -148,11 +124,11 @@ cudaError_t launch_ray_pairs(const PairNode* pairs, uint64_t n, RayPair* out, cu
   return cudaGetLastError();
 }
 
-cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const uint32_t* src, const PairNode* pairs,
+cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const QuadShape* shape, const PairNode* pairs,
                               const TriRecord* tris, BoxNode* boxes, cudaStream_t stream) {
   if (n_quads == 0) return cudaSuccess;
   const unsigned int grid = (unsigned int)((4 * n_quads + dev::kRefitBlock - 1) / dev::kRefitBlock);
-  dev::quad_boxes_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(quads, n_quads, src, pairs, tris, boxes);
+  dev::quad_boxes_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(quads, n_quads, shape, pairs, tris, boxes);
   return cudaGetLastError();
 }
 
