@@ -93,8 +93,9 @@ cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n, const QuadShape* shap
   return cudaSuccess;
 }
 
-cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris, const uint32_t*, const float*, int,
-                         bool, cudaStream_t) {
+cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, RayPair* rays, TriRecord* tris, const uint32_t*,
+                         const float*, int, bool, cudaStream_t) {
+  check(live(rays, plan.n_pairs * sizeof(RayPair)) && live(plan.arrive, 8 * plan.n_pairs));
   check(live(pairs, plan.n_pairs * sizeof(PairNode)) && live(plan.leaves, plan.n_leaves * sizeof(RefitLeaf)));
   for (uint32_t k = 0; k < plan.n_leaves; ++k) {  // each leaf's run ends where the records say
     const RefitLeaf& l = plan.leaves[k];

@@ -109,7 +109,6 @@ struct bvhc_mesh {
     uint64_t n = 0;
     int stack = 0;
     RayPair* ray_pairs = nullptr;  // the child pairs themselves in the ray traversals' form
-    uint64_t n_pairs = 0;
   };
   QuadSet quad_set[2];
 
@@ -766,9 +765,8 @@ static void free_quads(bvhc_mesh::QuadSet& q) {
 static cudaError_t make_quads(bvhc_mesh::QuadSet& q, bool with_boxes, const PairNode* nodes, const TriRecord* recs,
                               const std::vector<PairNode>& pairs, const std::vector<TriRecord>& tris,
                               const std::vector<uint32_t>& roots) {
-  q.n_pairs = pairs.size();
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&q.ray_pairs), std::max<size_t>(pairs.size(), 1) * sizeof(RayPair));
-  if (e == cudaSuccess) e = launch_ray_pairs(nodes, q.n_pairs, q.ray_pairs, nullptr);
+  if (e == cudaSuccess) e = launch_ray_pairs(nodes, pairs.size(), q.ray_pairs, nullptr);
   QuadBuilder qb{pairs, tris};
   std::vector<uint32_t> qroots;
   if (e == cudaSuccess && tris.size() < kRunFirst) try {
@@ -808,7 +806,6 @@ static void free_refit_plan(RefitPlan& p) {
   cudaFree(p.leaves);
   cudaFree(p.parent);
   cudaFree(p.arrive);
-  cudaFree(p.flags);
   cudaFree(p.root_box);
   p = RefitPlan{};
 }
@@ -848,8 +845,8 @@ static cudaError_t build_refit_plan(const std::vector<PairNode>& pairs, const st
   np.n_pairs = (uint32_t)pairs.size();
   cudaError_t e = upload(&np.leaves, leaves);
   if (e == cudaSuccess) e = upload(&np.parent, parent);
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&np.arrive), std::max<size_t>(pairs.size(), 1) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&np.flags), std::max<size_t>(pairs.size(), 1) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&np.arrive), std::max<size_t>(pairs.size(), 1) * 8);
+  if (e == cudaSuccess) np.flags = np.arrive + pairs.size();
   if (e == cudaSuccess) e = upload(&np.root_box, root_boxes);
   if (e != cudaSuccess) {
     free_refit_plan(np);
@@ -1392,12 +1389,13 @@ bvhc_status bvhc_mesh_refit(bvhc_mesh* m, const float* positions, uint64_t n_ver
   } else if (!aligned(positions, 4)) {
     return BVHC_ERR_INVALID_ARGUMENT;
   }
-  BVHC_CUDA_TRY(launch_refit(m->refit[0], m->d_nodes, m->d_tris, m->d_tri_vid, pos, stride_floats, false, s));
+  BVHC_CUDA_TRY(launch_refit(m->refit[0], m->d_nodes, m->quad_set[0].ray_pairs, m->d_tris, m->d_tri_vid, pos,
+                             stride_floats, false, s));
   if (m->leaf_size > 0 && m->refit[1].leaves)  // raycastFirst's copy: every box recomputed
-    BVHC_CUDA_TRY(launch_refit(m->refit[1], m->d_nodes_f, m->d_tris_f, m->d_tri_vid, pos, stride_floats, true, s));
+    BVHC_CUDA_TRY(launch_refit(m->refit[1], m->d_nodes_f, m->quad_set[1].ray_pairs, m->d_tris_f, m->d_tri_vid, pos,
+                               stride_floats, true, s));
   for (int k = 0; k < 2; ++k) {  // the four-child records follow their child pairs
     const bvhc_mesh::QuadSet& q = m->quad_set[k];
-    if (q.ray_pairs) BVHC_CUDA_TRY(launch_ray_pairs(k ? m->d_nodes_f : m->d_nodes, q.n_pairs, q.ray_pairs, s));
     if (q.quads)
       BVHC_CUDA_TRY(launch_quad_boxes(q.quads, q.n, q.shape, k ? m->d_nodes_f : m->d_nodes, k ? m->d_tris_f : m->d_tris,
                                       q.boxes, s));

@@ -244,7 +244,7 @@ struct RefitPlan {
   uint32_t n_leaves = 0;
   uint32_t* parent = nullptr;   // per pair record: the slot holding the pair's own box
   uint32_t* arrive = nullptr;   // per pair record: children finished (zeroed before each refit)
-  uint32_t* flags = nullptr;    // per pair record: bit s = child s's box changed
+  uint32_t* flags = nullptr;    // per pair record: bit s = child s's box changed; in arrive's allocation
   uint32_t n_pairs = 0;
   float* root_box = nullptr;    // 6 floats per root
 };
@@ -254,8 +254,9 @@ struct RefitPlan {
 // follows the reference's rule (MeshBVH#refit, refit.template.js:4-196): a leaf box is rewritten
 // and reported changed only when it differs, a parent's box is recomputed only when a child
 // changed; force = true recomputes every box.  tri_vid: 3 vertex ids per triangle (faceIndex).
-cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris, const uint32_t* tri_vid,
-                         const float* pos, int stride, bool force, cudaStream_t stream);
+// `rays`: the pairs' ray form (nullable), which follows.
+cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, RayPair* rays, TriRecord* tris,
+                         const uint32_t* tri_vid, const float* pos, int stride, bool force, cudaStream_t stream);
 // Every four-child record from its shape (4 per record), the child pairs and, for parts of leaves, the triangle
 // records; `boxes` (nullable) gets the same records with lo / hi bounds.
 cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const QuadShape* shape, const PairNode* pairs,

@@ -28,8 +28,16 @@ __device__ __forceinline__ float* slot_box(PairNode* pairs, float* root_box, uin
   return pairs[slot >> 1].f + 6 * (slot & 1u);
 }
 
+// A child pair's child as the warp-shared ray traversals read it.
+__device__ __forceinline__ void set_ray_child(QuadChild& c, const float* b) {
+  box_centre_half(b[0], b[3], c.c[0], c.h[0]);
+  box_centre_half(b[1], b[4], c.c[1], c.h[1]);
+  box_centre_half(b[2], b[5], c.cz, c.hz);
+}
+
+// `rays` (nullable): the pairs' ray form, in which a box is set with the pair's own.
 __global__ void __launch_bounds__(kRefitBlock) refit_kernel(RefitPlan plan, PairNode* __restrict__ pairs,
-                                                            TriRecord* __restrict__ tris,
+                                                            RayPair* __restrict__ rays, TriRecord* __restrict__ tris,
                                                             const uint32_t* __restrict__ tri_vid,
                                                             const float* __restrict__ pos, int stride, bool force) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -58,6 +66,10 @@ __global__ void __launch_bounds__(kRefitBlock) refit_kernel(RefitPlan plan, Pair
       box[a] = lo[a];
       box[3 + a] = hi[a];
     }
+    if (rays && leaf.count && !(leaf.slot & kRootSlot)) {
+      const float b[6] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
+      set_ray_child(rays[leaf.slot >> 1].c[leaf.slot & 1u], b);
+    }
   }
   uint32_t slot = leaf.slot;
   while (!(slot & kRootSlot)) {
@@ -72,12 +84,14 @@ __global__ void __launch_bounds__(kRefitBlock) refit_kernel(RefitPlan plan, Pair
       // both child boxes, read past L1 (the sibling may have written from another SM)
       const float* f = pairs[p].f;
       float* out = slot_box(pairs, plan.root_box, slot);
+      float b[6];
       for (int a = 0; a < 3; ++a) {
         float l0 = __ldcg(f + a), r0 = __ldcg(f + 6 + a);
         float l1 = __ldcg(f + 3 + a), r1 = __ldcg(f + 9 + a);
-        out[a] = l0 < r0 ? l0 : r0;
-        out[3 + a] = l1 > r1 ? l1 : r1;
+        out[a] = b[a] = l0 < r0 ? l0 : r0;
+        out[3 + a] = b[3 + a] = l1 > r1 ? l1 : r1;
       }
+      if (rays && !(slot & kRootSlot)) set_ray_child(rays[slot >> 1].c[slot & 1u], b);
     }
   }
 }
@@ -106,9 +120,7 @@ __global__ void __launch_bounds__(kRefitBlock) ray_pairs_kernel(const PairNode* 
   const int s = (int)(k & 1u);
   const float* b = p.f + 6 * s;
   QuadChild c;
-  box_centre_half(b[0], b[3], c.c[0], c.h[0]);
-  box_centre_half(b[1], b[4], c.c[1], c.h[1]);
-  box_centre_half(b[2], b[5], c.cz, c.hz);
+  set_ray_child(c, b);
   c.link = p.link[s];
   c.count = s == 0 ? p.axis : 0u;
   if (c.link == kEmptyLeaf) c.c[0] = c.c[1] = c.cz = __int_as_float(0x7FFFFFFF);
@@ -132,17 +144,15 @@ cudaError_t launch_quad_boxes(QuadNode* quads, uint64_t n_quads, const QuadShape
   return cudaGetLastError();
 }
 
-cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, TriRecord* tris, const uint32_t* tri_vid,
-                         const float* pos, int stride, bool force, cudaStream_t stream) {
+cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, RayPair* rays, TriRecord* tris,
+                         const uint32_t* tri_vid, const float* pos, int stride, bool force, cudaStream_t stream) {
   if (plan.n_leaves == 0) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-  if (plan.n_pairs) {
-    e = cudaMemsetAsync(plan.arrive, 0, plan.n_pairs * sizeof(uint32_t), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(plan.flags, 0, plan.n_pairs * sizeof(uint32_t), stream);
+  if (plan.n_pairs) {  // `flags` follows in the same allocation
+    cudaError_t e = cudaMemsetAsync(plan.arrive, 0, 2 * (size_t)plan.n_pairs * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
   }
   const unsigned int grid = (plan.n_leaves + dev::kRefitBlock - 1) / dev::kRefitBlock;
-  dev::refit_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(plan, pairs, tris, tri_vid, pos, stride, force);
+  dev::refit_kernel<<<grid, dev::kRefitBlock, 0, stream>>>(plan, pairs, rays, tris, tri_vid, pos, stride, force);
   return cudaGetLastError();
 }
 
