@@ -482,7 +482,7 @@ struct LeafSplitter {
 // tests it against near and far.  The boxes are filled in on the device, where a refit fills them in again.
 struct QuadBuilder {
   const std::vector<PairNode>& pairs;
-  const std::vector<TriRecord>& tris;
+  const TriRecord* tris;  // null: every leaf holds one
   std::vector<QuadShape> shape;  // four a record
   int stack = 0;  // entries a traversal can stack: at most the siblings along one path
   bool nested = true;  // every box of the tree lies in its parent's, so that those that are not records'
@@ -571,7 +571,7 @@ struct QuadBuilder {
 
   uint32_t leaf_count(uint32_t first) const {
     uint32_t k = first;
-    while (!(tris[k].flags & kTriLast)) ++k;
+    while (tris && !(tris[k].flags & kTriLast)) ++k;
     return k - first + 1;
   }
 
@@ -767,7 +767,7 @@ static cudaError_t make_quads(bvhc_mesh::QuadSet& q, bool with_boxes, const Pair
                               const std::vector<uint32_t>& roots) {
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&q.ray_pairs), std::max<size_t>(pairs.size(), 1) * sizeof(RayPair));
   if (e == cudaSuccess) e = launch_ray_pairs(nodes, pairs.size(), q.ray_pairs, nullptr);
-  QuadBuilder qb{pairs, tris};
+  QuadBuilder qb{pairs, tris.data()};
   std::vector<uint32_t> qroots;
   if (e == cudaSuccess && tris.size() < kRunFirst) try {
     qroots.resize(roots.size());
@@ -2030,14 +2030,13 @@ int bvhc_batch_mesh_count(const bvhc_mesh* m) { return m ? m->n_meshes : 0; }
 struct bvhc_scene {
   bvhc_mesh* batch = nullptr;
   int n_instances = 0;
+  void* d_arrays = nullptr;  // the next three
+  size_t arrays_cap = 0;
   InstanceDev* d_inst = nullptr;
-  size_t inst_cap = 0;
   PairNode* d_tlas = nullptr;
-  size_t tlas_cap = 0;
+  QuadNode* d_quads = nullptr;  // the same tree in four-child records
   uint32_t root = kEmptyLeaf;
-  QuadNode* d_quads = nullptr;  // the same tree in four-child records; has_quads: of these instances
-  size_t quads_cap = 0;
-  bool has_quads = false;
+  bool has_quads = false;       // its boxes nest
   uint32_t quad_root = 0;
   int quad_stack = 0;
   void* d_in = nullptr;
@@ -2122,32 +2121,6 @@ float round_up(double x) {
   return (double)f < x ? std::nextafter(f, INFINITY) : f;
 }
 
-// The instance tree in four-child records, for the phased raycastFirst.
-bvhc_status set_instance_quads(bvhc_scene* sc, const std::vector<PairNode>& nodes) {
-  sc->has_quads = false;
-  try {
-    TriRecord one{};
-    one.flags = kTriLast;  // a leaf's run: its instance
-    const std::vector<TriRecord> leaves(std::max(sc->n_instances, 1), one);
-    QuadBuilder qb{nodes, leaves};
-    sc->quad_root = qb.root(sc->root);
-    if (!qb.nested) return BVHC_OK;
-    std::vector<QuadNode> quads(qb.shape.size() / 4);
-    float box[6];
-    for (size_t k = 0; k < qb.shape.size(); ++k)
-      quads[k / 4].c[k % 4] = quad_child(qb.shape[k], nodes.data(), nullptr, box);
-    BVHC_CUDA_TRY(ensure(reinterpret_cast<void**>(&sc->d_quads), &sc->quads_cap, quads.size() * sizeof(QuadNode)));
-    BVHC_CUDA_TRY(cudaMemcpy(sc->d_quads, quads.data(), quads.size() * sizeof(QuadNode), cudaMemcpyHostToDevice));
-    sc->quad_stack = qb.stack;
-    sc->has_quads = true;
-  } catch (const Status& st) {
-    return st.code;
-  } catch (const std::bad_alloc&) {
-    return BVHC_ERR_OUT_OF_MEMORY;
-  }
-  return BVHC_OK;
-}
-
 bvhc_status set_instances(bvhc_scene* sc, int n, const uint32_t* geometry, const double* matrices,
                           const uint8_t* visible) {
   bvhc_mesh* m = sc->batch;
@@ -2230,18 +2203,47 @@ bvhc_status set_instances(bvhc_scene* sc, int n, const uint32_t* geometry, const
   std::vector<PairNode> nodes;
   uint32_t root = kEmptyLeaf;
   if (!boxes.empty()) root = build_tlas(boxes, 0, boxes.size(), nodes);
+  // the same tree in four-child records, for the phased raycastFirst; then all three arrays in one copy
+  QuadBuilder qb{nodes, nullptr};
+  uint32_t quad_root = 0;
+  std::vector<uint8_t> all;
+  size_t at_nodes = 0, at_inst = 0;
+  try {
+    quad_root = qb.root(root);
+    at_nodes = qb.shape.size() / 4 * sizeof(QuadNode);
+    at_inst = at_nodes + nodes.size() * sizeof(PairNode);
+    all.resize(at_inst + inst.size() * sizeof(InstanceDev));
+    float box[6];
+    for (size_t k = 0; k < qb.shape.size(); ++k) {
+      const QuadChild c = quad_child(qb.shape[k], nodes.data(), nullptr, box);
+      std::memcpy(&all[k * sizeof c], &c, sizeof c);
+    }
+    if (!nodes.empty()) std::memcpy(&all[at_nodes], nodes.data(), at_inst - at_nodes);
+    if (!inst.empty()) std::memcpy(&all[at_inst], inst.data(), inst.size() * sizeof(InstanceDev));
+  } catch (const Status& st) {
+    return st.code;
+  } catch (const std::bad_alloc&) {
+    return BVHC_ERR_OUT_OF_MEMORY;
+  }
   BVHC_CUDA_TRY(cudaSetDevice(m->device));
-  if (n > 0) {
-    BVHC_CUDA_TRY(ensure(reinterpret_cast<void**>(&sc->d_inst), &sc->inst_cap, inst.size() * sizeof(InstanceDev)));
-    BVHC_CUDA_TRY(cudaMemcpy(sc->d_inst, inst.data(), inst.size() * sizeof(InstanceDev), cudaMemcpyHostToDevice));
+  if (sc->arrays_cap < all.size()) {  // the old ones stay until there is room for the new
+    void* mem = nullptr;
+    BVHC_CUDA_TRY(cudaMalloc(&mem, all.size()));
+    cudaFree(sc->d_arrays);
+    sc->d_arrays = mem;
+    sc->arrays_cap = all.size();
   }
-  if (!nodes.empty()) {
-    BVHC_CUDA_TRY(ensure(reinterpret_cast<void**>(&sc->d_tlas), &sc->tlas_cap, nodes.size() * sizeof(PairNode)));
-    BVHC_CUDA_TRY(cudaMemcpy(sc->d_tlas, nodes.data(), nodes.size() * sizeof(PairNode), cudaMemcpyHostToDevice));
-  }
+  BVHC_CUDA_TRY(cudaMemcpy(sc->d_arrays, all.data(), all.size(), cudaMemcpyHostToDevice));
+  uint8_t* base = static_cast<uint8_t*>(sc->d_arrays);
+  sc->d_quads = reinterpret_cast<QuadNode*>(base);
+  sc->d_tlas = reinterpret_cast<PairNode*>(base + at_nodes);
+  sc->d_inst = reinterpret_cast<InstanceDev*>(base + at_inst);
+  sc->has_quads = qb.nested;
+  sc->quad_root = quad_root;
+  sc->quad_stack = qb.stack;
   sc->root = root;
   sc->n_instances = n;
-  return set_instance_quads(sc, nodes);
+  return BVHC_OK;
 }
 
 }  // namespace
@@ -2399,9 +2401,7 @@ bvhc_status bvhc_scene_raycast(bvhc_scene* sc, const float* rays, uint64_t n, in
 void bvhc_scene_destroy(bvhc_scene* sc) {
   if (!sc) return;
   if (sc->batch) cudaSetDevice(sc->batch->device);
-  cudaFree(sc->d_inst);
-  cudaFree(sc->d_tlas);
-  cudaFree(sc->d_quads);
+  cudaFree(sc->d_arrays);
   cudaFree(sc->d_in);
   cudaFree(sc->d_out);
   cudaFree(sc->d_ids);
