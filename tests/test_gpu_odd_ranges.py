@@ -33,7 +33,7 @@ def test_first_hits(pkg, cuda, mesh, near, far):
 
     g, opts = _mesh(pkg, mesh)
     bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH, **opts})
-    for n in (500, 30_000, 140_000):
+    for n in (500, 30_000, 200_000):
         rays = torch.from_numpy(_rays(pkg, n)).to(cuda)
         for leaf in (0, 4):
             bvh.set_leaf_size(leaf)

@@ -11,7 +11,9 @@ namespace dev {
 // 159 us with one lane per ray over child pairs, 50 us here; 80,000 triangles: 157 (one lane over the
 // same records) and 64 us.
 constexpr int kGroupBlocksPerSm = 8;    // 64 registers; 10 and 12 blocks spill more and measured slower
-constexpr unsigned kGroupChunk = 32;    // rays a warp takes from the work counter at once
+// Rays a warp takes from the work counter at once: so many warps are resident that with 32 a batch of 40,000 to
+// 150,000 rays left a third of them without any (40,000 camera rays 168 us, by 16 111, by 8 86).
+constexpr unsigned kGroupChunk = 8;
 constexpr int kGroupRefill = 2 * kGroup;  // idle lanes at which a warp takes new rays
 
 template <bool BATCHED, bool MATERIALS, bool RANGED>

@@ -496,11 +496,11 @@ static inline int group_stack(const MeshDev& m) {
 
 // Calls of up to kWideMaxRays rays take the whole warp for each ray, of up to kGroupMaxRays four lanes,
 // larger ones one lane.  With few rays the longest ray's chain of dependent steps is the time, and more
-// lanes make the chain shorter; with many, the chip is full and the lanes' own work counts.  Measured on
-// the 80,000-triangle knot, rays towards its box: 4,097 rays 24 us by warps (four lanes: 62, one lane 157),
-// 16,000 rays 65 (95), 32,000 rays 118 (110); 100,000 rays 188 by fours (one lane: 200), 250,000 rays 294
-// (254).  Incoherent rays, which mostly miss, cross later.
-constexpr uint64_t kWideMaxRays = 24576, kGroupMaxRays = 131072;
+// lanes make the chain shorter; with many, the chip is full and the lanes' own work counts.  Rays towards the
+// mesh's box, incoherent rays, a camera's, on the 80,000-triangle knot: 4,097 rays 24 us by warps (four lanes: 62,
+// one lane 157); 24,000 rays 102, 38, 97 us by warps (four lanes 110, 60, 77); 40,000 rays 158, 53, 148 (127, 70,
+// 86); 180,000 rays 227, 104, 176 by fours (one lane 254, 137, 180); 262,145 rays 307, 111, 219 (295, 130, 183).
+constexpr uint64_t kWideMaxRays = 24576, kGroupMaxRays = 196608;
 
 // Root-box pre-pass into `queue`, then (single mesh, sort requested) the ray-ordering sort
 // (kernels_first.cu).
