@@ -148,7 +148,7 @@ bvhc_status bvhc_mesh_get_info(const bvhc_mesh* mesh, bvhc_mesh_info* info);
 /* Traversal variant used by this mesh's raycastFirst calls (no reference counterpart: the
  * reference has one recursive traversal).  persistent = 1 walks four-child records (collapsed
  * from raycastFirst's child pairs, same leaves; children nearest first) with as many lanes per ray as
- * the batch leaves idle: a warp for up to 24,576 rays, four lanes for up to 131,072, else one, in
+ * the batch leaves idle: a warp for up to 24,576 rays, four lanes for up to 196,608, else one, in
  * resident warps that refill idle lanes from a work counter; a tree too deep for those records' stack
  * (or whose boxes do not nest) is walked over child pairs by resident warps that refill once `refill`
  * (1..32) lanes are idle.  0 runs one ray per

@@ -129,15 +129,16 @@ def tune_raycast_all(bvh, rays, cap: int = 64, reps: int = 3, candidates=tuple(r
 
 def tune_closest_point(bvh, points, min_t: float = 0.0, max_t: float = math.inf, reps: int = 3,
                        candidates=(0, 1, 2, 3, 4, 5, 6), tile_pitches=()) -> dict:
-    """Time closestPointToPoint's kernels (the `closest` field: per query; warp-cooperative in
-    input order and over Morton-sorted queries, with whole warps (1, 2), 16-lane (3, 4) or 8-lane
-    (5, 6) groups; and each input-order form reading the queries in tiled order for each row length
+    """Time closestPointToPoint's kernels (the `closest` field: a warp or four lanes per query (0),
+    warp-cooperative in input order (1; 3 and 5 are the same) and over Morton-sorted queries (2; 4 and
+    6 are the same); and the input-order form reading the queries in tiled order for each row length
     in `tile_pitches`, e.g. a grid's, with 2-, 4- and 8-row tiles) on `points` (torch CUDA tensor,
-    n x 3), keeping the mesh's other traversal fields, and install the fastest.
-    Returns {"best": name, "setting": fields, "timings_ms": ...}."""
+    n x 3), keeping the mesh's other traversal fields, and install the fastest.  Settings that are the
+    same kernel are timed once.  Returns {"best": name, "setting": fields, "timings_ms": ...}."""
     import torch
 
     cur = bvh.get_traversal()
+    candidates = [c for k, c in enumerate(candidates) if c == 0 or all(d == 0 or (d - c) % 2 for d in candidates[:k])]
     settings = {str(c): {"closest": c, "tile": 0, "tile_rows": 0} for c in candidates}
     for pitch in tile_pitches:
         for c in (c for c in candidates if c % 2 == 1):

@@ -7,7 +7,7 @@
 // each set's best warp-cooperative or persistent candidate on that layout: threads per block (64,
 // 128, 256; warp-cooperative form), the tile height of a tiled order (2, 4, 8 rows), the refill
 // threshold (8, 24; persistent form), and the 32-entry traversal stack (when the tree is shallow
-// enough).  Every variant returns the same hits (up to exact ties), so tuning changes speed only.
+// enough).  Candidates that differ in fields which the mesh's kernels do not read are timed once.  Every variant returns the same hits (up to exact ties), so tuning changes speed only.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "bvhcuda.h"
+#include "kernels.cuh"
 
 namespace {
 
@@ -62,6 +63,21 @@ std::vector<bvhc_traversal_config> stage1(const int32_t* tiles, int n_tiles) {
     for (int occ = 0; occ < 3; ++occ) c.push_back(make(2, 1, 16, occ, 0, 0, 1, tiles[k]));  // four-child records
   }
   return c;
+}
+
+// Whether the persistent form of this mesh reads the refill threshold: over four-child records it does not.
+bool reads_refill(const bvhc_mesh* mesh) {
+  bvhc::MeshDev v{};
+  bvhc::TraversalConfig cfg;
+  int device = 0;
+  return !bvhc::mesh_launch_info(mesh, &v, &cfg, &device) || !v.quads || v.quad_stack > bvhc::kMaxStack;
+}
+
+// Whether the persistent form launches the same for both: of its child order, register budget, record form and
+// stack it reads nothing.
+bool same_launch(const bvhc_traversal_config& a, const bvhc_traversal_config& b, bool refill) {
+  return a.persistent == 1 && b.persistent == 1 && a.compact == b.compact && a.sort == b.sort &&
+         (!refill || a.refill == b.refill);
 }
 
 // A tiled-order row pitch bvhc_mesh_set_traversal accepts: a multiple of 8 in [8, 2^24].
@@ -139,10 +155,17 @@ extern "C" bvhc_status bvhc_mesh_autotune(bvhc_mesh* mesh, int n_sets, const flo
   int best_leaf = -1;
   for (size_t li = 0; li < leaves.size() && st == BVHC_OK; ++li) {
     st = bvhc_mesh_set_leaf_size(mesh, leaves[li]);
+    const bool refill = reads_refill(mesh);
+    std::vector<bvhc_traversal_config> distinct;
+    for (const auto& c : cands) {
+      bool seen = false;
+      for (const auto& d : distinct) seen = seen || same_launch(c, d, refill);
+      if (!seen) distinct.push_back(c);
+    }
     float total = 0.0f;
     for (int k = 0; k < n_sets && st == BVHC_OK; ++k) {
       set_ms[k] = -1.0f;
-      for (const auto& c : cands) {
+      for (const auto& c : distinct) {
         float ms = 0.0f;
         st = time_variant(mesh, c, rays[k], counts[k], side, near_dist, far_dist, out, reps, s, t, &ms);
         if (st != BVHC_OK) break;
@@ -168,7 +191,7 @@ extern "C" bvhc_status bvhc_mesh_autotune(bvhc_mesh* mesh, int n_sets, const flo
     const bvhc_traversal_config base = chosen[k];
     if (base.persistent == 0 || (base.persistent == 2 && base.wide && !base.tile)) continue;
     std::vector<bvhc_traversal_config> more{base};
-    if (base.persistent == 1)
+    if (base.persistent == 1 && reads_refill(mesh))
       for (int refill : {8, 24})  // the refill thresholds between and below stage 1's 16 and 32
         if (refill != base.refill) {
           bvhc_traversal_config c = base;
@@ -201,7 +224,7 @@ extern "C" bvhc_status bvhc_mesh_autotune(bvhc_mesh* mesh, int n_sets, const flo
       }
     }
     if (st != BVHC_OK) break;
-    if (!chosen[k].wide) {  // the four-child kernels have one stack size
+    if (!chosen[k].wide && chosen[k].persistent == 2) {  // the other kernels have one stack size
       bvhc_traversal_config shallow = chosen[k];
       shallow.stack = 32;
       float ms = 0.0f;
