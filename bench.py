@@ -233,7 +233,7 @@ def traversal_kernel(cfg):
     p = 1 if cfg is None else cfg[0]
     if p == 2 and cfg is not None and len(cfg) > 7 and cfg[7]:
         return "raycast_first_packet4_kernel"
-    # the persistent form's kernel for batches of more than 131,072 rays
+    # the persistent form's kernel for batches of more than 196,608 rays
     return {0: "raycast_first_kernel", 1: "raycast_first_phased_kernel", 2: "raycast_first_packet_kernel"}[p]
 
 
@@ -504,7 +504,7 @@ def run_engine(args, ws, rank, local):
         k = max(range(len(sets)), key=lambda j: per_set_ms[j])
         achieved = bytes_per_launch[k] / (per_set_ms[k] / 1e3) / 1e9
         both = sum(bytes_per_launch) / (sum(per_set_ms) / 1e3) / 1e9
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        roof = {"bound": "issue", "of": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": profile_traffic(f"raycast_first_k2_{sets[k][0]}.md"), "peak_source": how,
                 "kernel": traversal_kernel(set_configs[k]), "ray_set": sets[k][0],
                 "both_sets": {"achieved": both, "frac": both / peak},
@@ -769,7 +769,7 @@ def run_closest(args, ws, rank, local):
         per_query = 12 + 20 + 32 * float(nn.mean()) + 36 * float(nt.mean())
         peak, how = measured_peak()
         achieved = n * per_query / (ms / 1e3) / 1e9
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        roof = {"bound": "issue", "of": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": how, "algorithmic_bytes_per_launch": n * per_query,
                 "reference_node_reads_per_query": float(nn.mean()),
                 "reference_triangle_tests_per_query": float(nt.mean()),
@@ -881,7 +881,7 @@ def run_all_hits(args, ws, rank, local):
         peak, how = measured_peak()
         k = max(range(len(sets)), key=lambda j: per_set_ms[j])
         achieved = bytes_per_set[k] / (per_set_ms[k] / 1e3) / 1e9
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        roof = {"bound": "issue", "of": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": how, "ray_set": sets[k][0],
                 "kernel": {0: "raycast_all_kernel", 1: "raycast_all_packet_kernel", "1t": "raycast_all_packet_kernel",
                            "1t2": "raycast_all_packet_kernel", "1t8": "raycast_all_packet_kernel",
@@ -1394,7 +1394,7 @@ def run_shapecast(args, ws, rank, local):
         cpu = {"value": m / dt / 1e6, "unit": "Mqueries/s", "cores": threads, "kind": "port",
                "sample": f"{m} evenly strided brush spheres, float64 oracle"}
         achieved = n_brush * per / (ms["sphere_triangles"] / 1e3) / 1e9
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        roof = {"bound": "issue", "of": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": None, "peak_source": how, "algorithmic_bytes_per_launch": n_brush * per,
                 "kernel": "sphere_triangles_kernel"}
     if rank == 0:
