@@ -1307,6 +1307,12 @@ bvhc_status bvhc_mesh_set_leaf_size(bvhc_mesh* m, int max_leaf) {
   std::vector<TriRecord> tris;
   std::vector<uint32_t> roots(m->h_roots.size());
   int depth = 0;
+  if (max_leaf > 0 && m->refit[0].leaves) {  // what a refit has made of the records
+    BVHC_CUDA_TRY(cudaSetDevice(m->device));
+    BVHC_CUDA_TRY(cudaDeviceSynchronize());
+    BVHC_CUDA_TRY(cudaMemcpy(m->h_pairs.data(), m->d_nodes, m->h_pairs.size() * sizeof(PairNode), cudaMemcpyDeviceToHost));
+    BVHC_CUDA_TRY(cudaMemcpy(m->h_tris.data(), m->d_tris, m->h_tris.size() * sizeof(TriRecord), cudaMemcpyDeviceToHost));
+  }
   if (max_leaf > 0) {
     LeafSplitter sp{m->h_pairs, m->h_tris, max_leaf};
     try {
