@@ -66,9 +66,10 @@ __device__ __forceinline__ Candidate candidate(float3 p, const Tri& t) {
   const float cpx = apx - acx, cpy = apy - acy, cpz = apz - acz;
   const float d5 = abx * cpx + aby * cpy + abz * cpz;
   const float d6 = acx * cpx + acy * cpy + acz * cpz;
-  // rounded product by product, so that it is zero where b = c (a segment, met on its edge a b)
-  const float vc = __fmul_rn(d1, d4) - __fmul_rn(d3, d2), vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
   const float e43 = d4 - d3, e56 = d5 - d6;
+  // both are zero where b = c, a segment, which is met on its edge a b: the products' fused difference is not
+  const float vc = e43 == 0.0f && e56 == 0.0f ? 0.0f : d1 * d4 - d3 * d2;
+  const float vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
   // the first region that holds wins, so they are taken last to first
   float nv = vb, nw = vc, den = va + vb + vc;
   const bool bc = va <= 0.0f && e43 >= 0.0f && e56 >= 0.0f;

@@ -262,7 +262,7 @@ __device__ __forceinline__ float closest_sq_f(float3 p, float3 a, float3 b, floa
   float cpx = apx - acx, cpy = apy - acy, cpz = apz - acz;
   float d5 = abx * cpx + aby * cpy + abz * cpz;
   float d6 = acx * cpx + acy * cpy + acz * cpz;
-  float vc = __fmul_rn(d1, d4) - __fmul_rn(d3, d2);  // zero where b = c
+  float vc = d4 == d3 && d5 == d6 ? 0.0f : d1 * d4 - d3 * d2;  // b = c: met on its edge a b
   float vb = d5 * d2 - d1 * d6;
   float va = d3 * d6 - d5 * d4;
   if (d1 <= 0.0f && d2 <= 0.0f) {
