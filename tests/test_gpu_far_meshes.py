@@ -96,10 +96,10 @@ def test_directions_far_from_unit_length(pkg, cuda, length):
     every = pkg.MeshBVH(g, {"strategy": pkg.SAH, "maxLeafSize": 2000})
     every.set_traversal(0, 1)
     bvh = pkg.MeshBVH(g, {"strategy": pkg.SAH})
-    r = _rays(g, 30_000, 7)
+    r = _rays(g, 200_000, 7)
     rng = np.random.default_rng(8)
-    r[:, 3:] = (r[:, 3:] + (rng.random((30_000, 3)) * 2 - 1) * 0.01) * length
-    for n in (1000, 30_000):
+    r[:, 3:] = (r[:, 3:] + (rng.random((200_000, 3)) * 2 - 1) * 0.01) * length
+    for n in (1000, 30_000, 200_000):
         rays = torch.from_numpy(r[:n].copy()).to(cuda)
         want = every.raycast_first_batch(rays, 2)[:, 1]
         bvh.set_traversal(0, 1)

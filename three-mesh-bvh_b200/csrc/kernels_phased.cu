@@ -68,7 +68,8 @@ __global__ void __launch_bounds__(kBlock, kPhasedBlocksPerSm) raycast_first_phas
       --sp;
       const uint2 e = sp < kPhasedTop ? s_top[sp][threadIdx.x] : rest[sp - kPhasedTop];
       link = e.x;
-      dead = !(__uint_as_float(e.y) <= (RANGED ? lim_hit : lim));
+      // (an infinite distance with a child's number in its low bits is no number, and not beyond)
+      dead = __uint_as_float(e.y) > (RANGED ? lim_hit : lim);
     } else {
       dead = false;
       walking = ++root < root_end;

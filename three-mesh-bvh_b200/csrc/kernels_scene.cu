@@ -430,7 +430,8 @@ __global__ void __launch_bounds__(kBlock, kSceneBlocksPerSm) scene_first_phased_
       --sp;
       const uint2 e = sp < kSceneTop ? s_top[sp][threadIdx.x] : rest[sp - kSceneTop];
       link = e.x;
-      dead = !(__uint_as_float(e.y) <= (RANGED ? lim_hit : lim));
+      // (an infinite distance with a child's number in its low bits is no number, and not beyond)
+      dead = __uint_as_float(e.y) > (RANGED ? lim_hit : lim);
     } else {
       dead = false;
       walking = inst != kNone && ++root < root_end;
