@@ -25,7 +25,7 @@ __device__ __forceinline__ RayF ray_from(float3 o, float3 d) {
   RayF r;
   r.o = o;
   r.d = d;
-  r.inv = ray_reciprocals(o, d);
+  r.inv = ray_reciprocals<false>(o, d);
   r.dk = kFilterK * (fabsf(d.x) + fabsf(d.y) + fabsf(d.z));
   return r;
 }
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kBlock, MINB) scene_raycast_first_kernel(MeshD
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const uint64_t i = queue ? queue[t] : t;
-  const RayF w = make_ray(rays, i);
+  const RayF w = make_ray<false>(rays, i);
   const float wlen = sqrtf(w.d.x * w.d.x + w.d.y * w.d.y + w.d.z * w.d.z);
   const SideTable no_sides{};
   // the best world record so far lives in the ray's output row (rewritten when a closer instance
@@ -381,7 +381,7 @@ __device__ __forceinline__ void offer_world(const MeshDev& m, const SceneDev& sc
 
 static __device__ __noinline__ void scene_record(const MeshDev& m, const SceneDev& sc, const float* __restrict__ rays,
                                                  uint64_t i, uint32_t inst, uint32_t rec, bvhc_hit* __restrict__ out) {
-  const RayF w = make_ray(rays, i);
+  const RayF w = make_ray<false>(rays, i);
   LocalRay L;
   local_ray(sc.inst[inst], w, 0.0f, kInf, L);
   bvhc_hit h;
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(kBlock, kSceneBlocksPerSm) scene_first_phased_
         alive = pending = true;
         dead = false;
         wb = world_none();
-        world(make_ray(rays, rid));
+        world(make_ray<false>(rays, rid));
         sp = 0;
         link = sc.quad_root;
       }
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kBlock, kSceneBlocksPerSm) scene_first_phased_
       if (__popc(nodes | leaves | switches) < keep) break;
       if (S >= kSceneSwitch || S >= N + L) {
         if (at_switch) {
-          const RayF w = make_ray(rays, rid);
+          const RayF w = make_ray<false>(rays, rid);
           if (inst != kNone) {
             if (best.rec != kNone) offer_world(m, sc, w, r, best, inst, vlen, wb);
             world(w);
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kBlock, 14) scene_raycast_all_kernel(MeshDev m
                                                                       uint32_t* __restrict__ inst_out) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const RayF w = make_ray(rays, i);
+  const RayF w = make_ray<false>(rays, i);
   const SideTable no_sides{};
   bvhc_hit* row = hits + i * (uint64_t)cap;
   uint32_t* irow = inst_out + i * (uint64_t)cap;
@@ -771,7 +771,7 @@ __global__ void __launch_bounds__(kBlock) scene_key_kernel(const float* __restri
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *qcount = (unsigned int)n;
   if (i >= n) return;
-  const RayF r = make_ray(rays, i);
+  const RayF r = make_ray<false>(rays, i);
   ids[i] = (uint32_t)i;
   if (kind != 4) {
     keys[i] = ray_key(kind, r.o, r.d, box);
