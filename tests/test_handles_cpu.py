@@ -17,8 +17,8 @@ def lib(pkg, tmp_path_factory):
     out = tmp_path_factory.mktemp("fake") / "libfake.so"
     csrc = os.path.join(ROOT, "three-mesh-bvh_b200", "csrc")
     cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-include", "cmath", "-I", csrc, "-I",
-                    os.path.join(ROOT, "include"), "-I", cuda, "-x", "c++", os.path.join(csrc, "api.cu"),
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-include", "cmath",
+                    "-I", csrc, "-I", os.path.join(ROOT, "include"), "-I", cuda, "-x", "c++", os.path.join(csrc, "api.cu"),
                     os.path.join(csrc, "builder.cpp"), os.path.join(ROOT, "tests", "native", "fake_cuda.cpp"),
                     "-o", str(out)], check=True)
     # lazily bound (ctypes itself binds at once): the launches that no test reaches are not there

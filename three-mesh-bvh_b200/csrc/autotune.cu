@@ -6,8 +6,10 @@
 // asked for; the layout with the smallest sum of the sets' best times is kept.  Stage 2 refines
 // each set's best warp-cooperative or persistent candidate on that layout: threads per block (64,
 // 128, 256; warp-cooperative form), the tile height of a tiled order (2, 4, 8 rows), the refill
-// threshold (8, 24; persistent form), and the 32-entry traversal stack (when the tree is shallow
-// enough).  Candidates that differ in fields which the mesh's kernels do not read are timed once.  Every variant returns the same hits (up to exact ties), so tuning changes speed only.
+// threshold (8, 24; persistent form over child pairs), and the 32-entry traversal stack
+// (warp-cooperative form, when the tree is shallow enough).  Candidates that differ in fields which
+// the mesh's kernels do not read are timed once.  Every variant returns the same hits (up to exact
+// ties), so tuning changes speed only.
 #include <cuda_runtime.h>
 
 #include <algorithm>

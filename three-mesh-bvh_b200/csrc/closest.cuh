@@ -361,8 +361,8 @@ cudaError_t launch_closest_wide(const MeshDev& m, const float* pts, uint32_t n, 
 
 // closestPointToPoint's traversals with minThreshold 0 (kernels_closest.cu): pending records of five words
 // (triangle record and vertex, or 0xFFFFFFFF; number of undecided candidates; those).  shared: the 32 queries of
-// a warp in one traversal of the child pairs (m.n_tris < kRunFirst), in the order of `queue` (nullable), or with pitch > 0 in
-// tiled order with 2^rows_log2 rows a tile; else over the four-child records (group_stack(m) > 0).
+// a warp in one traversal of the child pairs (m.n_tris < kRunFirst), in the order of `queue` (nullable), or with
+// pitch > 0 in tiled order with 2^rows_log2 rows a tile; else over the four-child records (group_stack(m) > 0).
 cudaError_t launch_closest_phased(const MeshDev& m, const float* pts, uint32_t n, float max_t, bvhc_closest* out,
                                   bool shared, const uint32_t* queue, uint32_t pitch, int rows_log2,
                                   cudaStream_t stream);
