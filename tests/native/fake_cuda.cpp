@@ -15,6 +15,8 @@ std::map<void*, size_t> held;
 int fail_in = 0;  // > 0: that many allocations from now, one fails
 int bad = 0;      // launches given records that do not belong together
 int packets = 0;
+int host_blocks = 0;  // page-locked allocations so far
+bool host_gone = false;  // their context is
 
 bool live(const void* p, size_t bytes) {
   auto it = held.find(const_cast<void*>(p));
@@ -29,6 +31,8 @@ int fake_fail_left() { return fail_in; }
 int64_t fake_held() { return (int64_t)held.size(); }
 int fake_bad() { return bad; }
 int fake_packets() { return packets; }
+int fake_host_blocks() { return host_blocks; }
+void fake_lose_host(int gone) { host_gone = gone != 0; }
 
 cudaError_t cudaMalloc(void** p, size_t n) {
   if (fail_in > 0 && --fail_in == 0) return cudaErrorMemoryAllocation;
@@ -46,7 +50,15 @@ cudaError_t cudaFree(void* p) {
   std::free(p);
   return cudaSuccess;
 }
-cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
+cudaError_t cudaMallocHost(void** p, size_t n) {
+  ++host_blocks;
+  return cudaMalloc(p, n);
+}
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+  a->type = host_gone ? cudaMemoryTypeUnregistered : cudaMemoryTypeHost;
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
   std::memcpy(d, s, n);

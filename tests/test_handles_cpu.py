@@ -81,3 +81,32 @@ def test_a_leaf_layout_that_cannot_be_made_changes_nothing(pkg, lib):
     cast()
     lib.bvhc_mesh_destroy(mesh)
     assert lib.fake_held() == start and lib.fake_bad() == 0
+
+
+def test_handles_made_for_one_pick_share_page_locked_memory(pkg, lib):
+    native = importlib.import_module(pkg.__name__ + "._native")
+    args, _, keep = _mesh(pkg, lib)
+    rays, hits = np.zeros((4, 6), np.float32), np.zeros((4, 8), np.float32)
+    cfg = native.BvhcTraversalConfig(2, 0, 16, 2)
+
+    def pick():
+        mesh = C.c_void_p()
+        assert lib.bvhc_mesh_create(*args, C.byref(mesh)) == OK
+        assert lib.bvhc_mesh_set_traversal(mesh, C.byref(cfg)) == OK
+        assert lib.bvhc_raycast_first(mesh, rays.ctypes.data, 4, 0, 0.0, 1e9, hits.ctypes.data, native.MEM_HOST, None) == OK
+        return mesh
+
+    before, held = lib.fake_host_blocks(), lib.fake_held()
+    for _ in range(5):
+        lib.bvhc_mesh_destroy(pick())
+    assert lib.fake_host_blocks() == before + 1
+    meshes = [pick() for _ in range(7)]                      # one block each while they live
+    assert lib.fake_host_blocks() == before + 7
+    for mesh in meshes:
+        lib.bvhc_mesh_destroy(mesh)
+    assert lib.fake_held() == held + 4                       # no more are kept than four
+    lib.fake_lose_host(1)                                    # nor used once their context is gone
+    mesh = pick()
+    lib.fake_lose_host(0)
+    lib.bvhc_mesh_destroy(mesh)
+    assert lib.fake_host_blocks() == before + 8 and lib.fake_bad() == 0

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstring>
 #include <exception>
+#include <mutex>
 #include <new>
 #include <stdexcept>
 #include <thread>
@@ -750,6 +751,42 @@ static void keep_serialized(bvhc_mesh* m, std::vector<std::vector<uint8_t>> root
   }
 }
 
+// The page-locked blocks of handles that are gone, for the next handles: the process's only such block takes the
+// driver 2.3 to 3 ms to make, as long as 100 picks save, and a program that makes a handle for one pick would pay
+// that each time.  At most four (29 KB each) are kept, until the process ends; those above are freed.  A block
+// belongs to one handle at a time, whatever its device or stream (page-locked memory is every device's).
+static std::mutex few_lock;
+static bvhc_mesh::Few* few_kept[4];
+static int n_few_kept = 0;
+
+static cudaError_t take_few(bvhc_mesh::Few** few) {
+  {
+    const std::lock_guard<std::mutex> hold(few_lock);
+    while (n_few_kept > 0) {
+      bvhc_mesh::Few* p = few_kept[--n_few_kept];
+      cudaPointerAttributes at;
+      if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost) {
+        *few = p;
+        return cudaSuccess;
+      }
+      cudaGetLastError();  // it went with its context (cudaDeviceReset)
+    }
+  }
+  return cudaMallocHost(reinterpret_cast<void**>(few), sizeof(bvhc_mesh::Few));
+}
+
+// No launch may still use it.
+static void give_few(bvhc_mesh::Few* few) {
+  {
+    const std::lock_guard<std::mutex> hold(few_lock);
+    if (n_few_kept < 4) {
+      few_kept[n_few_kept++] = few;
+      return;
+    }
+  }
+  cudaFreeHost(few);
+}
+
 static void free_quads(bvhc_mesh::QuadSet& q) {
   cudaFree(q.quads);
   cudaFree(q.boxes);
@@ -1130,7 +1167,8 @@ void bvhc_mesh_destroy(bvhc_mesh* m) {
   cudaFree(m->d_work);
   cudaFree(m->d_work_all);
   cudaFree(m->d_in);
-  if (m->few) cudaFreeHost(m->few);
+  if (m->few && cudaDeviceSynchronize() == cudaSuccess) give_few(m->few);  // after a call that failed half way
+  else cudaFreeHost(m->few);
   cudaFree(m->d_out);
   cudaFree(m->d_out2);
   for (int k = 0; k < bvhc_mesh::kPipes; ++k) {
@@ -1477,7 +1515,7 @@ static bvhc_status raycast_first_impl(bvhc_mesh* m, const float* rays, uint64_t 
     return from_cuda(dispatch_first(m, rays, n, side, tab, near_d, far_d, out, m->d_work, s));
   }
   if (n <= bvhc_mesh::kFewRays) {
-    if (!m->few) BVHC_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&m->few), sizeof(bvhc_mesh::Few)));
+    if (!m->few) BVHC_CUDA_TRY(take_few(&m->few));
     bvhc_mesh::Few& f = *m->few;
     std::memcpy(f.rays, rays, n * 24);
     BVHC_CUDA_TRY(dispatch_first(m, f.rays, n, side, tab, near_d, far_d, f.hits, m->d_work, s));
