@@ -114,8 +114,8 @@ struct bvhc_mesh {
   QuadSet quad_set[2];
 
   // Host-memory raycastFirst of a few rays (a pick): page-locked memory that the kernels read and write in
-  // place, made on first need, instead of three copies through pageable memory that are waited for one by
-  // one.  1 ray 48 -> 34 us, 256 rays 47 -> 36, 512 rays 48 -> 40; 1,024 rays 47 -> 48.
+  // place, taken on first need (take_few), instead of three copies through pageable memory that are waited for
+  // one by one.  1 ray 48 -> 34 us, 256 rays 47 -> 36, 512 rays 48 -> 40; 1,024 rays 47 -> 48.
   static constexpr uint64_t kFewRays = 512;
   struct Few {
     alignas(16) bvhc_hit hits[kFewRays];
