@@ -618,8 +618,8 @@ def measure_batched(args, ws, rank, local):
     from three_mesh_bvh_b200 import autotune
 
     # (the batched launch always runs the persistent form; ray ordering applies to single meshes),
-    # on each device leaf layout
-    cands = [c for c in autotune.candidates() if c[0] == 1 and c[5] == 0]
+    # on each device leaf layout; over four-child records it reads of the variants only the compaction
+    cands = [c for c in autotune.candidates() if (*c[:4], c[5], c[7]) == (1, 1, 16, 2, 0, 1)]
     timings = {}
     for leaf in (0, 2, 4):
         batch.set_leaf_size(leaf)
